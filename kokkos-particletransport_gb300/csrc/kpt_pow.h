@@ -53,6 +53,13 @@
 #define KPT_POW_FN static inline
 #endif
 
+/* The device build spends as few FP64 instructions as it can (they issue at
+ * a small fraction of the other pipes' rate): comparisons, exact scalings by
+ * powers of two and integer conversions act on the bits, quotients by one
+ * divisor share its rounded reciprocal, and exact two-operand sums whose
+ * larger operand is known take three operations (Dekker) instead of six.
+ * Each replacement is exact or rounds once to the same value, so host and
+ * device agree bit for bit. */
 #if defined(__CUDA_ARCH__)
 #define KPT_P_ADD(a, b) __dadd_rn((a), (b))
 #define KPT_P_SUB(a, b) __dsub_rn((a), (b))
@@ -86,6 +93,28 @@ KPT_POW_FN double kpt_pow_two(int k) {
     return kpt_pow_from_bits((uint64_t)(k + 1023) << 52);
 }
 
+/* (double)k for |k| < 2^31 */
+KPT_POW_FN double kpt_pow_int(int k) {
+#if defined(__CUDA_ARCH__)
+    const unsigned a = k < 0 ? 0u - (unsigned)k : (unsigned)k;
+    const int lz = __clz((int)a);
+    const unsigned m = lz >= 31 ? 0u : a << (lz + 1);
+    const unsigned hi = ((unsigned)(1023 + 31 - lz) << 20) | (m >> 12) | ((unsigned)k & 0x80000000u);
+    return a == 0u ? 0.0 : __hiloint2double((int)hi, (int)(m << 20));
+#else
+    return (double)k;
+#endif
+}
+
+#if defined(__CUDA_ARCH__)
+/* RN(a / b) for r = RN(1 / b) and operands far from the ends of the exponent
+ * range (Markstein 1990): one product, the exact remainder, one correction */
+KPT_POW_FN double kpt_pow_quotient(double a, double b, double r) {
+    const double q = __dmul_rn(a, r);
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+#endif
+
 /* ln(x) as hi + lo for finite x > 0 (subnormals included). */
 KPT_POW_FN void kpt_pow_log(double x, double* hi, double* lo) {
     /* ln 2 = LN2_HI + LN2_LO, LN2_HI with 42 significant bits */
@@ -99,21 +128,30 @@ KPT_POW_FN void kpt_pow_log(double x, double* hi, double* lo) {
         e = (int)((u >> 52) & 0x7ff) - 54;
     }
     e -= 1023;
-    double m = kpt_pow_from_bits((u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL);
-    if (m > SQRT2) {
-        m = KPT_P_MUL(m, 0.5);
+    uint64_t mb = (u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL;
+    if (mb > kpt_pow_bits(SQRT2)) { /* m > sqrt 2: halve */
+        mb -= 0x0010000000000000ULL;
         e += 1;
     }
+    const double m = kpt_pow_from_bits(mb);
     const double f = KPT_P_SUB(m, 1.0); /* exact (Sterbenz) */
-    /* d = m + 1 as a double-double (two-sum) */
+    /* d = m + 1 as a double-double (m < 2, so 1 is the larger exponent) */
     const double d_hi = KPT_P_ADD(m, 1.0);
-    const double bv = KPT_P_SUB(d_hi, m);
-    const double d_lo = KPT_P_ADD(KPT_P_SUB(m, KPT_P_SUB(d_hi, bv)), KPT_P_SUB(1.0, bv));
+    const double d_lo = KPT_P_SUB(m, KPT_P_SUB(d_hi, 1.0));
     /* s = f / d to double-double accuracy */
+#if defined(__CUDA_ARCH__)
+    const double rcp = __drcp_rn(d_hi);
+    const double s_hi = kpt_pow_quotient(f, d_hi, rcp);
+#else
     const double s_hi = KPT_P_DIV(f, d_hi);
+#endif
     double rem = KPT_P_FMA(-s_hi, d_hi, f); /* exact */
     rem = KPT_P_SUB(rem, KPT_P_MUL(s_hi, d_lo));
+#if defined(__CUDA_ARCH__)
+    const double s_lo = kpt_pow_quotient(rem, d_hi, rcp);
+#else
     const double s_lo = KPT_P_DIV(rem, d_hi);
+#endif
     /* P(z) = sum_{k=1..12} 2/(2k+1) z^(k-1), z = s^2 */
     const double z = KPT_P_MUL(s_hi, s_hi);
     double p = 0x1.47ae147ae147bp-4;       /* 2/25 */
@@ -131,15 +169,14 @@ KPT_POW_FN void kpt_pow_log(double x, double* hi, double* lo) {
     const double tail = KPT_P_MUL(KPT_P_MUL(s_hi, z), p);
     /* ln m = 2 s_hi + (2 s_lo + tail), |2 s_hi| >= |rest| */
     const double lm_hi0 = KPT_P_MUL(2.0, s_hi);
-    const double lm_rest = KPT_P_ADD(KPT_P_MUL(2.0, s_lo), tail);
+    const double lm_rest = KPT_P_FMA(2.0, s_lo, tail); /* the product is exact */
     const double lm_hi = KPT_P_ADD(lm_hi0, lm_rest);
     const double lm_lo = KPT_P_SUB(lm_rest, KPT_P_SUB(lm_hi, lm_hi0));
-    /* + e ln2 (e * LN2_HI exact) */
-    const double ed = (double)e;
+    /* + e ln2 (e * LN2_HI exact, and larger than lm_hi unless e = 0) */
+    const double ed = kpt_pow_int(e);
     const double a = KPT_P_MUL(ed, LN2_HI);
     const double sum = KPT_P_ADD(a, lm_hi);
-    const double bb = KPT_P_SUB(sum, a);
-    const double err = KPT_P_ADD(KPT_P_SUB(a, KPT_P_SUB(sum, bb)), KPT_P_SUB(lm_hi, bb));
+    const double err = KPT_P_SUB(lm_hi, KPT_P_SUB(sum, a));
     const double low = KPT_P_ADD(KPT_P_ADD(err, lm_lo), KPT_P_MUL(ed, LN2_LO));
     const double h = KPT_P_ADD(sum, low);
     *hi = h;
@@ -152,16 +189,19 @@ KPT_POW_FN double kpt_pow_exp(double hi, double lo) {
     const double LN2_LO = 0x1.ef35793c76730p-45;
     const double INV_LN2 = 0x1.71547652b82fep+0;
     const double SHIFTER = 0x1.8p52; /* round to nearest integer by addition */
-    if (hi > 709.8) {
+    /* hi > 709.8 and hi < -745.2 (hi is never NaN here) */
+    const uint64_t hb = kpt_pow_bits(hi);
+    if ((hb >> 63) == 0 && hb > kpt_pow_bits(709.8)) {
         return kpt_pow_from_bits(0x7ff0000000000000ULL);
     }
-    if (hi < -745.2) {
+    if (hb > kpt_pow_bits(-745.2)) {
         return 0.0;
     }
-    const double kd = KPT_P_SUB(KPT_P_ADD(KPT_P_MUL(hi, INV_LN2), SHIFTER), SHIFTER);
-    const int k = (int)kd;
-    /* r = hi - k ln2 + lo; the head subtraction is exact */
-    const double r_head = KPT_P_SUB(hi, KPT_P_MUL(kd, LN2_HI));
+    const double kr = KPT_P_ADD(KPT_P_MUL(hi, INV_LN2), SHIFTER);
+    const double kd = KPT_P_SUB(kr, SHIFTER);
+    const int k = (int)(uint32_t)kpt_pow_bits(kr); /* the shifted sum's low bits */
+    /* r = hi - k ln2 + lo; k LN2_HI and the head subtraction are exact */
+    const double r_head = KPT_P_FMA(-kd, LN2_HI, hi);
     const double r_tail = KPT_P_SUB(lo, KPT_P_MUL(kd, LN2_LO));
     const double r_hi = KPT_P_ADD(r_head, r_tail);
     const double bv = KPT_P_SUB(r_hi, r_head);
@@ -181,27 +221,24 @@ KPT_POW_FN double kpt_pow_exp(double hi, double lo) {
     q = KPT_P_FMA(q, r_hi, 0x1.1111111111111p-7);  /* 1/5! */
     q = KPT_P_FMA(q, r_hi, 0x1.5555555555555p-5);  /* 1/4! */
     q = KPT_P_FMA(q, r_hi, 0x1.5555555555555p-3);  /* 1/3! */
-    /* r^2 / 2 exactly (fma product error), scaled by 1/2 exactly */
+    /* r^2 exactly (fma product error); its halves enter as exact products */
     const double sq = KPT_P_MUL(r_hi, r_hi);
     const double sq_err = KPT_P_FMA(r_hi, r_hi, -sq);
-    const double half_sq = KPT_P_MUL(sq, 0.5);
-    const double half_sq_err = KPT_P_MUL(sq_err, 0.5);
     const double cube_q = KPT_P_MUL(KPT_P_MUL(sq, r_hi), q);
     /* 1 + r_hi (|1| >= |r_hi|), then + r^2/2 */
     const double a_hi = KPT_P_ADD(1.0, r_hi);
     const double a_lo = KPT_P_SUB(r_hi, KPT_P_SUB(a_hi, 1.0));
-    const double b_hi = KPT_P_ADD(a_hi, half_sq);
-    const double bb = KPT_P_SUB(b_hi, a_hi);
-    const double b_lo =
-        KPT_P_ADD(KPT_P_SUB(a_hi, KPT_P_SUB(b_hi, bb)), KPT_P_SUB(half_sq, bb));
+    const double b_hi = KPT_P_FMA(sq, 0.5, a_hi); /* a_hi is the larger */
+    const double b_lo = KPT_P_FMA(sq, 0.5, -KPT_P_SUB(b_hi, a_hi));
     /* the small terms; r_lo enters as exp(r_hi) r_lo ~ (1 + r_hi) r_lo */
     double low = KPT_P_ADD(a_lo, b_lo);
-    low = KPT_P_ADD(low, half_sq_err);
+    low = KPT_P_FMA(sq_err, 0.5, low);
     low = KPT_P_ADD(low, KPT_P_FMA(r_lo, r_hi, r_lo));
     low = KPT_P_ADD(low, cube_q);
     const double e = KPT_P_ADD(b_hi, low); /* the one rounding of the result */
     if (k >= -1021 && k <= 1023) {
-        return KPT_P_MUL(e, kpt_pow_two(k));
+        /* e in [0.7, 1.5): the scaled result is normal */
+        return kpt_pow_from_bits(kpt_pow_bits(e) + ((uint64_t)(int64_t)k << 52));
     }
     /* near the ends of the range: scale in two exact-or-final steps */
     const int k1 = k / 2;

@@ -25,9 +25,9 @@
 // on the lane, launch shape or work order.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <type_traits>
 
 #include "kpt_device.cuh"
 #include "kpt_internal.h"
@@ -58,25 +58,6 @@ constexpr double kSqrt3 = 1.7320508075688772935;
 
 template <typename T>
 struct Num;
-
-template <>
-struct Num<double> {
-#if KPT_PUSH_PART == 1
-    // the project pow (kpt_pow.h): rounds exactly as the host oracle does
-    static __device__ __forceinline__ double pow(double a, double b) { return kpt_pow(a, b); }
-#else
-    // the contracted FP64 push: CUDA's pow
-    static __device__ __forceinline__ double pow(double a, double b) { return ::pow(a, b); }
-#endif
-    static __device__ __forceinline__ double sqrt(double a) { return ::sqrt(a); }
-    static __device__ __forceinline__ double div(double a, double b) { return a / b; }
-    static __device__ __forceinline__ bool finite(double a) { return isfinite(a); }
-    static __device__ __forceinline__ double abs(double a) { return fabs(a); }
-    // uniform_sqrt3 (RandomManager.hpp:111-114) on draw (lo, hi).
-    static __device__ __forceinline__ double noise(uint32_t lo, uint32_t hi) {
-        return __dadd_rn(-kSqrt3, __dmul_rn(kSqrt3 + kSqrt3, u01_f64(lo, hi)));
-    }
-};
 
 template <>
 struct Num<float> {
@@ -685,6 +666,33 @@ __device__ __forceinline__ void increments(const Rates<T>& r, T dt, const uint4&
     }
 }
 
+// What the FP64 push precomputes per launch (make_f64_consts, make_pow_plan).
+struct F64AxisKeys {
+    long long lower, upper;  // integer keys of the axis bounds
+    long long floor_zero;    // coordinates in [lower, floor_zero) need no wrap
+    double rcp_step;         // RN(1 / step) of a uniform axis
+};
+struct F64Consts {
+    F64AxisKeys axis[2];
+    double rcp_mhd_dt, rcp_p0, rcp_3;  // rounded reciprocals (div_known)
+    double drift1_p0, drift2_p0_p0;    // drift_param1 p0, drift_param2 p0 p0
+    double inv_charge;                 // 1 / charge focused, 1 / (3 charge) Parker
+    double half_cell;                  // half the smaller mean cell width
+    double p_floor;
+    long long end_key;                 // interval end
+    int single_step;                   // dt_min == dt_max
+    unsigned lane_cap;                 // particles a warp holds
+    int simple;                        // schedule without refill
+};
+// Powers of a substep: out[e] = base[base[e]] ^ exponent[e].
+constexpr int kF64Powers = 6;
+struct PowPlan {
+    int powers;
+    int shared_logs;  // every exponent finite
+    int base[kF64Powers];
+    double exponent[kF64Powers];
+};
+
 struct PushParams {
     Grid grid;
     FixedGrid fixed;
@@ -705,113 +713,9 @@ struct PushParams {
     PushCounters* counters;
     SurrogateDevice sg;  // used by the surrogate instantiation only
     const float* records;  // cell records of (lower, upper); nullptr: point-major sampling
+    F64Consts f64;         // FP64 push
+    PowPlan pows;
 };
-
-// ------------------------------------------------------------- FP64 path
-struct StateF64 {
-    double x, y, p, t, diag_dt, mu;
-    int steps;
-    int status;
-    uint32_t index;
-};
-
-// The first part of an FP64 substep: count it, wrap the position and sample
-// the time-interpolated table at the shifted position.
-template <bool FOCUSED>
-__device__ __forceinline__ void sample_f64(StateF64& st, const PushParams& P,
-                                           double c[FOCUSED ? 21 : 16]) {
-    constexpr int C = FOCUSED ? 21 : 16;
-    constexpr int STRIDE = FOCUSED ? 22 : 16;
-    const DeviceSettings& s = P.s;
-    ++st.steps;
-    st.x = wrap_driver(st.x, s.x_lower, s.x_upper, s.x_width);
-    st.y = wrap_driver(st.y, s.y_lower, s.y_upper, s.y_width);
-    const double rt = __ddiv_rn(__dsub_rn(st.t, P.interval_start), s.mhd_dt);
-    sample_coefficients<double, C, STRIDE>(P.grid, static_cast<const double*>(P.lower),
-                                           static_cast<const double*>(P.upper),
-                                           __dadd_rn(st.x, s.shift_x), __dadd_rn(st.y, s.shift_y),
-                                           rt, s.time_interpolation, c);
-}
-
-// The rest of an FP64 substep from the sampled table values: physics (with
-// the served closure when SURR), step size, noise and the update.
-template <bool FOCUSED, bool SURR = false>
-__device__ __forceinline__ bool advance_f64(StateF64& st, const PushParams& P, const double* c,
-                                            const Served* served = nullptr) {
-    const DeviceSettings& s = P.s;
-    Rates<double> r;
-    if (!physics<double, FOCUSED, SURR>(c, st.p, st.mu, P.kd, r, served)) {
-        st.status = 2;
-        return false;
-    }
-    double dt = r.fixed_dt ? s.dt_min : r.dt;
-    if (dt < s.dt_min) dt = s.dt_min;
-    if (dt > s.dt_max) dt = s.dt_max;
-    st.diag_dt = dt;
-    const double remaining = __dsub_rn(P.interval_end, st.t);
-    if (dt > remaining) dt = remaining;
-    if (!isfinite(dt) || dt <= 0.0) {
-        st.status = 2;
-        return false;
-    }
-    const uint32_t block = 2u * static_cast<uint32_t>(st.steps - 1);
-    const uint4 r0 = philox4x32_10(make_uint4(block, st.index, P.frame, kTagPush), P.key);
-    const uint4 r1 = philox4x32_10(make_uint4(block + 1u, st.index, P.frame, kTagPush), P.key);
-    double dx, dy, mu;
-    increments<double, FOCUSED>(r, dt, r0, r1, P.kd, dx, dy, mu);
-    st.mu = mu;
-    st.x = __dadd_rn(st.x, dx);
-    st.y = __dadd_rn(st.y, dy);
-    st.p = __dadd_rn(st.p, r.dp_dt * dt);
-    st.t = __dadd_rn(st.t, dt);
-    const double pfloor = 0.25 * s.p0;
-    if (st.p < pfloor) st.p = pfloor;
-    if (!isfinite(st.x) || !isfinite(st.y) || !isfinite(st.p) || !isfinite(st.t)) {
-        st.status = 2;
-        return false;
-    }
-    return st.t < P.interval_end && st.steps < s.max_steps;
-}
-
-template <bool FOCUSED>
-__device__ __forceinline__ bool substep(StateF64& st, const PushParams& P) {
-    double c[FOCUSED ? 21 : 16];
-    sample_f64<FOCUSED>(st, P, c);
-    return advance_f64<FOCUSED>(st, P, c);
-}
-
-template <bool FOCUSED>
-__device__ __forceinline__ void load(StateF64& st, const PushParams& P, uint32_t index) {
-    const ParticleArrays& a = P.parts;
-    st.index = index;
-    st.x = a.x[index];
-    st.y = a.y[index];
-    st.p = a.p[index];
-    st.t = a.t[index];
-    st.diag_dt = a.step_dt[index];
-    st.mu = FOCUSED ? clamp_mu(a.mu[index], P.s.mu_max) : 0.0;
-    st.steps = 0;
-    st.status = 0;
-}
-
-template <bool FOCUSED>
-__device__ __forceinline__ void store(StateF64& st, const PushParams& P) {
-    const ParticleArrays& a = P.parts;
-    const DeviceSettings& s = P.s;
-    if (st.steps >= s.max_steps && st.t < P.interval_end) st.status = 2;
-    const uint32_t i = st.index;
-    a.x[i] = wrap_driver(st.x, s.x_lower, s.x_upper, s.x_width);
-    a.y[i] = wrap_driver(st.y, s.y_lower, s.y_upper, s.y_width);
-    a.p[i] = st.p;
-    a.t[i] = st.t;
-    a.step_dt[i] = st.diag_dt;
-    if (FOCUSED) a.mu[i] = st.mu;
-    a.status[i] = st.status;
-}
-
-__device__ __forceinline__ bool live(const StateF64& st, const PushParams& P) {
-    return st.t < P.interval_end && st.steps < P.s.max_steps;
-}
 
 // ------------------------------------------------------------ mixed path
 // No FP64 instruction runs inside the mixed substep loop:
@@ -1252,58 +1156,6 @@ __device__ __forceinline__ bool substep_surrogate(StateMixed& st, const PushPara
     return advance_mixed<true, true>(st, P, c, &served);
 }
 
-// The FP64 focused substep with the learned closure, warp-collective on the
-// mma.sync engine (as the mixed one above): the table is sampled and the
-// physics evaluated in FP64, the network serves D_mumu, dD_mumu/dmu and
-// kappa_parallel in place of the plain closure's powers.  The plain closure
-// answers outside the training box and below mu_cut, blends in over
-// [mu_cut, 2 mu_cut] and judges one substep in judge_period, in FP64.
-template <bool FP16, int H>
-__device__ __forceinline__ bool substep_surrogate(StateF64& st, const PushParams& P, bool have,
-                                                  const uint2* smem, JudgeTally& tally,
-                                                  float* /*xpose: FP64 tables have no records*/) {
-    const SurrogateDevice& sg = P.sg;
-    const SurrogateBox& box = sg.box;
-    double c[21];
-    float f[kMlpIn] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    bool use = false;
-    double mu = 0.0;
-    if (have) {
-        sample_f64<true>(st, P, c);
-        mu = clamp_mu(st.mu, P.kd.mu_max);
-        const float b = static_cast<float>(c[6]);
-        const float p = static_cast<float>(st.p);
-        const float amu = fabsf(static_cast<float>(mu));
-        if (sg.constants_in_box && amu >= box.mu_cut && b > 0.0f && p > 0.0f) {
-            const float lm = __logf(amu);
-            const float lp = __logf(p);
-            const float lb = __logf(b);
-            use = lm <= box.in_hi[0] && lp >= box.in_lo[1] && lp <= box.in_hi[1] &&
-                  lb >= box.in_lo[2] && lb <= box.in_hi[2];
-            if (use) {
-                f[0] = lm * box.in_scale[0] + box.in_offset[0];
-                f[1] = lp * box.in_scale[1] + box.in_offset[1];
-                f[2] = lb * box.in_scale[2] + box.in_offset[2];
-                f[3] = sg.f3;
-                f[4] = sg.f4;
-            }
-        }
-    }
-    float y[kMlpOut];
-    __syncwarp();
-    mlp_warp<FP16, H>(smem, f, y);
-    if (!have) {
-        return false;
-    }
-    // The served values are FP32 whichever closure gives them, so the lanes
-    // outside the training box (and the judged and blended ones) take the
-    // plain closure in FP32 too: a warp then never runs the FP64 closure's
-    // five powers for a few of its lanes.
-    const Served served = serve_closure(P, use, static_cast<float>(mu), static_cast<float>(c[6]),
-                                        static_cast<float>(st.p), st.steps, y, tally);
-    return advance_f64<true, true>(st, P, c, &served);
-}
-
 // Position <-> fixed-point phase (once per particle and push).
 __device__ __forceinline__ uint64_t to_phase(double x, double lower, double inv_width) {
     double f = (x - lower) * inv_width;
@@ -1418,12 +1270,8 @@ __device__ __forceinline__ void flush_judge(unsigned long long* judge, JudgeTall
 #ifndef KPT_MIXED_MIN_BLOCKS
 #define KPT_MIXED_MIN_BLOCKS 5
 #endif
-template <typename State, bool FOCUSED>
+template <bool FOCUSED>
 struct MinBlocks {
-    static constexpr int value = FOCUSED ? 2 : 4;
-};
-template <>
-struct MinBlocks<StateMixed, false> {
     static constexpr int value = KPT_MIXED_MIN_BLOCKS;
 };
 // Focused mixed push with the plain closure: 5 blocks (96 registers, a few
@@ -1432,7 +1280,7 @@ struct MinBlocks<StateMixed, false> {
 #define KPT_MIXED_FOCUSED_MIN_BLOCKS 5
 #endif
 template <>
-struct MinBlocks<StateMixed, true> {
+struct MinBlocks<true> {
     static constexpr int value = KPT_MIXED_FOCUSED_MIN_BLOCKS;
 };
 
@@ -1447,12 +1295,10 @@ struct MinBlocks<StateMixed, true> {
 #endif
 __host__ __device__ constexpr bool surr_fp16(int surr) { return surr == 2 || surr == 4; }
 __host__ __device__ constexpr int surr_hidden(int surr) { return surr <= 2 ? 64 : 32; }
-template <typename State, bool FOCUSED, int SURR = 0>
-__global__ void __launch_bounds__(128, !std::is_same<State, StateMixed>::value
-                                           ? MinBlocks<State, FOCUSED>::value
-                                       : SURR >= 3 ? KPT_SURROGATE32_MIN_BLOCKS
-                                       : SURR      ? KPT_SURROGATE_MIN_BLOCKS
-                                                   : MinBlocks<State, FOCUSED>::value)
+template <bool FOCUSED, int SURR = 0>
+__global__ void __launch_bounds__(128, SURR >= 3 ? KPT_SURROGATE32_MIN_BLOCKS
+                                       : SURR    ? KPT_SURROGATE_MIN_BLOCKS
+                                                 : MinBlocks<FOCUSED>::value)
     push_refill_kernel(const PushParams P) {
     const unsigned full = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
@@ -1464,12 +1310,12 @@ __global__ void __launch_bounds__(128, !std::is_same<State, StateMixed>::value
     }
     // the warp's rows for the record sampler, after the network's block
     float* xpose = nullptr;
-    if (std::is_same<State, StateMixed>::value && P.records != nullptr) {
+    if (P.records != nullptr) {
         xpose = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(surrogate_smem) +
                                          (SURR ? mlp_smem_bytes(surr_hidden(SURR)) : 0)) +
                 (threadIdx.x >> 5) * 32 * record_xpose_stride(FOCUSED);
     }
-    State st;
+    StateMixed st;
     bool have = false;
     bool exhausted = false;
     unsigned long long my_steps = 0, my_pushed = 0, my_failed = 0;
@@ -1515,11 +1361,9 @@ __global__ void __launch_bounds__(128, !std::is_same<State, StateMixed>::value
         if constexpr (SURR) {
             more = substep_surrogate<surr_fp16(SURR), surr_hidden(SURR)>(
                 st, P, have, surrogate_smem, tally, xpose);
-        } else if constexpr (std::is_same<State, StateMixed>::value) {
+        } else {
             more = xpose != nullptr ? substep_records<FOCUSED>(st, P, have, xpose)
                                     : have && substep<FOCUSED>(st, P);
-        } else {
-            more = have && substep<FOCUSED>(st, P);
         }
         if (have && !more) {
             store<FOCUSED>(st, P);
@@ -1633,7 +1477,7 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
 }
 
 // One particle per thread, no refill (schedule alternative for the tuner).
-template <typename State, bool FOCUSED>
+template <bool FOCUSED>
 __global__ void __launch_bounds__(128) push_simple_kernel(const PushParams P) {
     unsigned long long my_steps = 0, my_pushed = 0, my_failed = 0;
     unsigned int my_max = 0;
@@ -1644,7 +1488,7 @@ __global__ void __launch_bounds__(128) push_simple_kernel(const PushParams P) {
         if (P.parts.status[idx] != 0) {
             continue;
         }
-        State st;
+        StateMixed st;
         load<FOCUSED>(st, P, idx);
         ++my_pushed;
         if (live(st, P)) {
@@ -1658,6 +1502,9 @@ __global__ void __launch_bounds__(128) push_simple_kernel(const PushParams P) {
     }
     flush_counters(P.counters, my_steps, my_pushed, my_failed, my_max);
 }
+
+F64Consts make_f64_consts(const PushLaunch& L);
+PowPlan make_pow_plan(const PushLaunch& L);
 
 PushParams make_push_params(const PushLaunch& L) {
     PushParams P;
@@ -1683,8 +1530,22 @@ PushParams make_push_params(const PushLaunch& L) {
         P.sg = *L.surrogate;
     }
     P.records = L.precision == kPrecisionMixed ? L.records : nullptr;
+    P.f64 = F64Consts{};
+    P.pows = PowPlan{};
+    if (L.precision == kPrecisionF64) {
+        P.f64 = make_f64_consts(L);
+        P.pows = make_pow_plan(L);
+    }
     return P;
 }
+
+}  // namespace
+}  // namespace kpt
+
+#include "kpt_push_f64.cuh"
+
+namespace kpt {
+namespace {
 
 // Persistent grid of the tcgen05 push: as many blocks per SM as both the
 // TMEM (TcMlp<H>::Cols of the SM's 512 columns each) and the registers
@@ -1728,11 +1589,11 @@ cudaError_t launch_push_tc(const PushParams& P, const PushLaunch& L, cudaStream_
     return cudaGetLastError();
 }
 
-template <typename State, bool FOCUSED, int SURR = 0>
+template <bool FOCUSED, int SURR = 0>
 cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
     const PushParams P = make_push_params(L);
     const int threads = 128;
-    if constexpr (SURR != 0 && std::is_same<State, StateMixed>::value) {
+    if constexpr (SURR != 0) {
         if (L.surrogate->engine == kEngineTcgen05) {
             return launch_push_tc<surr_fp16(SURR), surr_hidden(SURR)>(P, L, stream);
         }
@@ -1743,18 +1604,18 @@ cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
         const uint64_t want = (L.count + threads - 1) / threads;
         const int blocks =
             static_cast<int>(want < 1 ? 1 : (want > 65535u * 8u ? 65535u * 8u : want));
-        push_simple_kernel<State, FOCUSED><<<blocks, threads, 0, stream>>>(P);
+        push_simple_kernel<FOCUSED><<<blocks, threads, 0, stream>>>(P);
     } else {
         // Persistent grid: as many resident blocks per SM as the kernel's
         // registers allow (or fewer on request).
         int resident = 0;
         cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &resident, push_refill_kernel<State, FOCUSED, SURR>, threads, smem);
+            &resident, push_refill_kernel<FOCUSED, SURR>, threads, smem);
         if (err != cudaSuccess) return err;
         resident = resident < 1 ? 1 : resident;
         const int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm
                                                                             : resident;
-        push_refill_kernel<State, FOCUSED, SURR>
+        push_refill_kernel<FOCUSED, SURR>
             <<<L.sm_count * per_sm, threads, smem, stream>>>(P);
     }
     return cudaGetLastError();
@@ -1826,7 +1687,7 @@ __device__ __forceinline__ bool substep_batch_records(StateMixed& st, const Push
 // the particles a lane carries (each carries its own state).
 template <bool FOCUSED, int THREADS, int PPL>
 struct BatchMinBlocks {
-    static constexpr int threads_per_sm = MinBlocks<StateMixed, FOCUSED>::value * 128 / PPL;
+    static constexpr int threads_per_sm = MinBlocks<FOCUSED>::value * 128 / PPL;
     static constexpr int value = threads_per_sm / THREADS > 0 ? threads_per_sm / THREADS : 1;
 };
 
@@ -1972,8 +1833,8 @@ __global__ void sample_kernel(const SampleLaunch L) {
 #if KPT_PUSH_PART == 1
 
 cudaError_t launch_push_interval_f64(const PushLaunch& launch, cudaStream_t stream) {
-    return launch.focused ? launch_push<StateF64, true>(launch, stream)
-                          : launch_push<StateF64, false>(launch, stream);
+    return launch.focused ? launch_push_f64<true>(launch, stream)
+                          : launch_push_f64<false>(launch, stream);
 }
 
 cudaError_t launch_sample_f64(const SampleLaunch& L, int blocks, cudaStream_t stream) {
@@ -2044,8 +1905,8 @@ cudaError_t launch_batch_focused(const BatchLaunch& B, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_push_interval_f64_contracted(const PushLaunch& launch, cudaStream_t stream) {
-    return launch.focused ? launch_push<StateF64, true>(launch, stream)
-                          : launch_push<StateF64, false>(launch, stream);
+    return launch.focused ? launch_push_f64<true>(launch, stream)
+                          : launch_push_f64<false>(launch, stream);
 }
 
 bool batch_shape_supported(int threads, int particles_per_lane) {
@@ -2076,11 +1937,11 @@ cudaError_t launch_push_interval(const PushLaunch& launch, cudaStream_t stream) 
             // with the contracted FP64 arithmetic
             const SurrogateBox& box = launch.surrogate->box;
             if (box.hidden == 64) {
-                return box.fp16 ? launch_push<StateF64, true, 2>(launch, stream)
-                                : launch_push<StateF64, true, 1>(launch, stream);
+                return box.fp16 ? launch_push_f64<true, 2>(launch, stream)
+                                : launch_push_f64<true, 1>(launch, stream);
             }
-            return box.fp16 ? launch_push<StateF64, true, 4>(launch, stream)
-                            : launch_push<StateF64, true, 3>(launch, stream);
+            return box.fp16 ? launch_push_f64<true, 4>(launch, stream)
+                            : launch_push_f64<true, 3>(launch, stream);
         }
         return launch.fp64_contracted ? launch_push_interval_f64_contracted(launch, stream)
                                       : launch_push_interval_f64(launch, stream);
@@ -2088,14 +1949,14 @@ cudaError_t launch_push_interval(const PushLaunch& launch, cudaStream_t stream) 
     if (launch.surrogate != nullptr) {
         const SurrogateBox& box = launch.surrogate->box;
         if (box.hidden == 64) {
-            return box.fp16 ? launch_push<StateMixed, true, 2>(launch, stream)
-                            : launch_push<StateMixed, true, 1>(launch, stream);
+            return box.fp16 ? launch_push<true, 2>(launch, stream)
+                            : launch_push<true, 1>(launch, stream);
         }
-        return box.fp16 ? launch_push<StateMixed, true, 4>(launch, stream)
-                        : launch_push<StateMixed, true, 3>(launch, stream);
+        return box.fp16 ? launch_push<true, 4>(launch, stream)
+                        : launch_push<true, 3>(launch, stream);
     }
-    return launch.focused ? launch_push<StateMixed, true>(launch, stream)
-                          : launch_push<StateMixed, false>(launch, stream);
+    return launch.focused ? launch_push<true>(launch, stream)
+                          : launch_push<false>(launch, stream);
 }
 
 #endif  // KPT_PUSH_PART
