@@ -95,6 +95,9 @@ struct ScopedBuffer : DeviceBuffer {
     ~ScopedBuffer() { release(); }
 };
 
+// Floats of an array rounded up to whole 16-byte chunks.
+size_t aligned_floats(size_t n) { return (n + 3) & ~static_cast<size_t>(3); }
+
 }  // namespace
 
 struct kpt_context {
@@ -1654,8 +1657,13 @@ int kpt_surrogate_train(kpt_context* ctx, const kpt_settings* settings,
     const size_t b = static_cast<size_t>(c.batch);
     const size_t pcount = static_cast<size_t>(kpt::mlp_params(hidden));
     const size_t chunks = (b + kpt::kGradChunk - 1) / kpt::kGradChunk;
-    const size_t floats = 4 * pcount + b * (kpt::kMlpIn + 4 * hidden + kpt::kMlpOut) +
-                          static_cast<size_t>(c.steps) + chunks * pcount;
+    // rows of activations and deltas are read four floats at a time: every
+    // array starts on a 16-byte boundary
+    const size_t pfloats = aligned_floats(pcount);
+    const size_t hfloats = b * static_cast<size_t>(hidden);
+    const size_t floats = 4 * pfloats + aligned_floats(b * kpt::kMlpIn) + 4 * hfloats +
+                          aligned_floats(b * kpt::kMlpOut) +
+                          aligned_floats(static_cast<size_t>(c.steps)) + chunks * pcount;
     KPT_CUDA(work.reserve(floats * sizeof(float)));
     KPT_CUDA(cudaMemsetAsync(work.ptr, 0, floats * sizeof(float), st));
     kpt::SurrogateTrainLaunch L{};
@@ -1667,17 +1675,17 @@ int kpt_surrogate_train(kpt_context* ctx, const kpt_settings* settings,
     L.batch = c.batch;
     L.box = box;
     L.params = w;
-    L.grad = w + pcount;
-    L.m = w + 2 * pcount;
-    L.v = w + 3 * pcount;
-    L.xb = w + 4 * pcount;
-    L.h1 = L.xb + b * kpt::kMlpIn;
-    L.h2 = L.h1 + b * hidden;
-    L.g1 = L.h2 + b * hidden;
-    L.g2 = L.g1 + b * hidden;
-    L.gy = L.g2 + b * hidden;
-    L.loss = L.gy + b * kpt::kMlpOut;
-    L.partial = L.loss + c.steps;
+    L.grad = w + pfloats;
+    L.m = w + 2 * pfloats;
+    L.v = w + 3 * pfloats;
+    L.xb = w + 4 * pfloats;
+    L.h1 = L.xb + aligned_floats(b * kpt::kMlpIn);
+    L.h2 = L.h1 + hfloats;
+    L.g1 = L.h2 + hfloats;
+    L.g2 = L.g1 + hfloats;
+    L.gy = L.g2 + hfloats;
+    L.loss = L.gy + aligned_floats(b * kpt::kMlpOut);
+    L.partial = L.loss + aligned_floats(static_cast<size_t>(c.steps));
     L.beta1 = 0.9f;
     L.beta2 = 0.999f;
     // quantization-aware fine-tuning: the last quarter of the steps sees the
@@ -1687,6 +1695,7 @@ int kpt_surrogate_train(kpt_context* ctx, const kpt_settings* settings,
     KPT_CUDA(cudaMemcpyAsync(L.params, sg->params.data(), pcount * sizeof(float),
                              cudaMemcpyHostToDevice, st));
     const double pi = 3.141592653589793238462643383279502884;
+    KPT_CUDA(kpt::surrogate_prepare_training(hidden));
     for (int step = 0; step < c.steps; ++step) {
         const double phase = static_cast<double>(step) / static_cast<double>(c.steps);
         L.lr = static_cast<float>(c.learning_rate * (0.01 + 0.99 * 0.5 * (1.0 + std::cos(pi * phase))));
@@ -1861,15 +1870,17 @@ int kpt_surrogate_gradient(kpt_context* ctx, int32_t hidden_width, const float* 
     if (int rc = activate(ctx)) return rc;
     const size_t pcount = static_cast<size_t>(kpt::mlp_params(hidden));
     const size_t chunks = (n + kpt::kGradChunk - 1) / kpt::kGradChunk;
-    const size_t floats =
-        n * (5 + 3) + 2 * pcount + n * (5 + 4 * hidden + 3) + 1 + chunks * pcount;
+    const size_t pfloats = aligned_floats(pcount);
+    const size_t hfloats = n * static_cast<size_t>(hidden);
+    const size_t floats = 2 * aligned_floats(n * 5) + 2 * aligned_floats(n * 3) + 2 * pfloats +
+                          4 * hfloats + aligned_floats(1) + chunks * pcount;
     ScopedBuffer buf;
     KPT_CUDA(buf.reserve(floats * sizeof(float)));
     KPT_CUDA(cudaMemsetAsync(buf.ptr, 0, floats * sizeof(float), ctx->stream));
     float* w = buf.as<float>();
     kpt::SurrogateTrainLaunch L{};
     float* x = w;
-    float* t = x + n * 5;
+    float* t = x + aligned_floats(n * 5);
     L.x = x;
     L.t = t;
     L.n = static_cast<int>(n);
@@ -1884,17 +1895,17 @@ int kpt_surrogate_gradient(kpt_context* ctx, int32_t hidden_width, const float* 
         L.box.out_offset[k] = 0.0f;
         L.box.out_scale[k] = 1.0f;
     }
-    L.params = t + n * 3;
-    L.grad = L.params + pcount;
-    L.xb = L.grad + pcount;
+    L.params = t + aligned_floats(n * 3);
+    L.grad = L.params + pfloats;
+    L.xb = L.grad + pfloats;
     L.box.hidden = hidden;
-    L.h1 = L.xb + n * 5;
-    L.h2 = L.h1 + n * hidden;
-    L.g1 = L.h2 + n * hidden;
-    L.g2 = L.g1 + n * hidden;
-    L.gy = L.g2 + n * hidden;
-    L.loss = L.gy + n * 3;
-    L.partial = L.loss + 1;
+    L.h1 = L.xb + aligned_floats(n * 5);
+    L.h2 = L.h1 + hfloats;
+    L.g1 = L.h2 + hfloats;
+    L.g2 = L.g1 + hfloats;
+    L.gy = L.g2 + hfloats;
+    L.loss = L.gy + aligned_floats(n * 3);
+    L.partial = L.loss + aligned_floats(1);
     cudaStream_t st = ctx->stream;
     KPT_CUDA(cudaMemcpyAsync(x, inputs, n * 5 * sizeof(float), cudaMemcpyHostToDevice, st));
     KPT_CUDA(cudaMemcpyAsync(t, targets, n * 3 * sizeof(float), cudaMemcpyHostToDevice, st));

@@ -230,7 +230,7 @@ struct SurrogateTrainLaunch {
     float* m;
     float* v;
     float* xb;        // batch x 5 normalised inputs
-    float* h1;        // batch x 64
+    float* h1;        // batch x hidden width; h1, h2, g1, g2 on 16-byte boundaries
     float* h2;
     float* g1;
     float* g2;
@@ -244,6 +244,8 @@ struct SurrogateTrainLaunch {
 constexpr int kGradChunk = 256;
 cudaError_t surrogate_make_samples(uint64_t seed, int n, const SurrogateBox& box, float* x,
                                    float* t, cudaStream_t stream);
+// Once before the steps of a training: kernel attributes of the width.
+cudaError_t surrogate_prepare_training(int hidden);
 cudaError_t surrogate_train_step(const SurrogateTrainLaunch& launch, int step,
                                  cudaStream_t stream);
 // Gradient of the loss over the first `batch` samples in order (step < 0).

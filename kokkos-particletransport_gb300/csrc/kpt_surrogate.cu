@@ -110,162 +110,516 @@ __device__ __forceinline__ float normalise_input(const SurrogateBox& box, int k,
     return v * box.in_scale[k] + box.in_offset[k];
 }
 
-// Forward and backward of one minibatch, one thread per sample.  Stores
-// H1, H2 (activations) and G1, G2, GY (deltas) for the gradient reductions.
+// ---- one optimisation step ------------------------------------------------------
+// Three kernels: forward + backward (train_pass_kernel), the weight gradients
+// of every chunk of kGradChunk samples (train_grad_kernel), the chunk sums and
+// Adam (train_update_kernel).  Every sum runs over the same terms in the same
+// order as one thread per sample (passes) or per parameter (gradients) would
+// take them, each term one FMA: weights of a row in input order, samples of a
+// chunk in sample order, chunks in chunk order, so the trained weights do not
+// depend on the tiling.
+//
+// What bounds a step (batch 8192, width 64): 0.2 GFLOP of FP32 FMA is 1.4 us
+// of the chip; the step is launch and latency bound, so the tiles are chosen
+// to fill the SMs (256 pass blocks of 32 samples, 192 gradient blocks) rather
+// than to reuse operands further, operands arrive by asynchronous copies that
+// a block waits for once, and each kernel starts while the previous one
+// drains.  A step takes 26 us; 115 us when a thread ran a whole sample with
+// its activations in local memory and a gradient thread one column over 256
+// samples from global memory.  Width 32: 61 -> 22 us.
+
+constexpr int kPassSamples = 32;   // samples of a pass block
+constexpr int kPassThreads = 256;
+constexpr int kGradThreads = 256;
+
+// Rows of H floats padded by four: 128-bit reads at a fixed column offset hit
+// distinct banks for eight consecutive rows.
 template <int H>
-__global__ void __launch_bounds__(128) fwd_bwd_kernel(const float* __restrict__ x,
-                                                      const float* __restrict__ t, int n,
-                                                      uint64_t seed, int step, int batch,
-                                                      SurrogateBox box,
-                                                      const float* __restrict__ params,
-                                                      float* xb, float* h1, float* h2, float* g1,
-                                                      float* g2, float* gy, float* loss,
-                                                      int quant) {
+struct PassSmem {
+    static constexpr int LD = H + 4;
+    alignas(16) float w1[H * kMlpIn];
+    alignas(16) float b1[H];
+    alignas(16) float b2[H];
+    alignas(16) float w3[kMlpOut * H];
+    float b3[4];
+    float in[kPassSamples * kMlpIn];
+    float target[kPassSamples * 4];
+    float dy[kPassSamples * 4];
+    alignas(16) float w2[H * LD];
+    alignas(16) float a1[kPassSamples * LD];
+    alignas(16) float a2[kPassSamples * LD];  // activations, then deltas
+};
+
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    v[0] = f.x;
+    v[1] = f.y;
+    v[2] = f.z;
+    v[3] = f.w;
+}
+
+// 16 bytes from global to shared memory without a register: a block's whole
+// operand set is in flight before it waits once.
+__device__ __forceinline__ void copy16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" : : "r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_done() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// The kernels of consecutive steps are launched with programmatic dependence:
+// a kernel's blocks may start while the previous kernel drains, and read or
+// write nothing an earlier kernel touches before previous_done (which returns
+// once the previous kernel, and so everything before it, has completed).
+__device__ __forceinline__ void previous_done() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void next_may_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <int J>
+__device__ __forceinline__ void load_row(const float* p, float (&v)[J]) {
+    static_assert(J == 4 || J == 2, "H / 16 columns");
+    if constexpr (J == 4) {
+        load4(p, v);
+    } else {
+        const float2 f = *reinterpret_cast<const float2*>(p);
+        v[0] = f.x;
+        v[1] = f.y;
+    }
+}
+
+// Forward and backward of 32 samples per block.  The two H x H products give
+// each thread two samples (sg, sg + 16) times H / 16 columns; operands
+// come four along the summed dimension per 128-bit read, from the weights'
+// own row order in both directions.  Stores H1, H2 (activations) and G1, G2,
+// GY (deltas) for the gradients.
+template <int H>
+__global__ void __launch_bounds__(kPassThreads)
+    train_pass_kernel(const float* __restrict__ x, const float* __restrict__ t, int n,
+                      uint64_t seed, int step, int batch, const SurrogateBox box,
+                      const float* __restrict__ params, float* __restrict__ xb,
+                      float* __restrict__ h1, float* __restrict__ h2, float* __restrict__ g1,
+                      float* __restrict__ g2, float* __restrict__ gy, float* loss, int quant) {
     // quant != 0: the forward sees the served network's rounding (weights,
     // inputs and activations in the 16-bit type, FP16 pre-activations too;
     // biases and accumulation FP32) and the backward passes straight
     // through it
     using M = Mlp<H>;
-    __shared__ float w[M::Params];
-    for (int k = threadIdx.x; k < M::Params; k += blockDim.x) {
-        const bool bias = (k >= M::B1 && k < M::W2) || (k >= M::B2 && k < M::W3) || k >= M::B3;
-        w[k] = bias ? params[k] : quantize(params[k], quant);
+    using S = PassSmem<H>;
+    constexpr int LD = S::LD;
+    constexpr int J = H / 16;                             // columns of a thread
+    constexpr int I = kPassSamples * 16 / kPassThreads;   // samples of a thread
+    constexpr int SG = kPassSamples / I;                  // sample groups
+    extern __shared__ __align__(16) unsigned char pass_smem[];
+    S& sm = *reinterpret_cast<S*>(pass_smem);
+    const int tid = threadIdx.x;
+    const int b0 = blockIdx.x * kPassSamples;
+    const int here = batch - b0 < kPassSamples ? batch - b0 : kPassSamples;
+    next_may_start();
+    // The block's samples are drawn and gathered from the fixed training set
+    // before the previous step's update has to be complete.
+    float in[kMlpIn] = {};
+    if (tid < kPassSamples) {
+        float target[kMlpOut] = {};
+        if (tid < here) {
+            const int b = b0 + tid;
+            int i = b % n;
+            if (step >= 0) {
+                const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(b),
+                                                         static_cast<uint32_t>(step), 0u, 9u),
+                                              seed_key(seed));
+                i = static_cast<int>(u01_f64(r.x, r.y) * n) % n;
+            }
+            for (int k = 0; k < kMlpIn; ++k) {
+                in[k] = quantize(normalise_input(box, k, x[static_cast<size_t>(i) * kMlpIn + k]),
+                                 quant);
+            }
+            for (int o = 0; o < kMlpOut; ++o) {
+                target[o] = (t[static_cast<size_t>(i) * kMlpOut + o] - box.out_offset[o]) /
+                            box.out_scale[o];
+            }
+        }
+        for (int k = 0; k < kMlpIn; ++k) sm.in[tid * kMlpIn + k] = in[k];
+        for (int o = 0; o < kMlpOut; ++o) sm.target[tid * 4 + o] = target[o];
+    }
+    previous_done();
+    for (int k = tid; k < H * H / 4; k += kPassThreads) {
+        copy16(sm.w2 + (4 * k / H) * LD + 4 * k % H, params + M::W2 + 4 * k);
+    }
+    for (int k = tid; k < H * kMlpIn / 4; k += kPassThreads) {
+        copy16(sm.w1 + 4 * k, params + M::W1 + 4 * k);
+    }
+    if (tid < H / 4) {
+        copy16(sm.b1 + 4 * tid, params + M::B1 + 4 * tid);
+        copy16(sm.b2 + 4 * tid, params + M::B2 + 4 * tid);
+    }
+    if (tid < kMlpOut * H / 4) copy16(sm.w3 + 4 * tid, params + M::W3 + 4 * tid);
+    if (tid < kMlpOut) sm.b3[tid] = params[M::B3 + tid];
+    if (tid < here) {
+        for (int k = 0; k < kMlpIn; ++k) xb[static_cast<size_t>(b0 + tid) * kMlpIn + k] = in[k];
+    }
+    copies_done();
+    __syncthreads();
+    if (quant != 0) {
+        for (int k = tid; k < H * H; k += kPassThreads) {
+            float& w = sm.w2[(k / H) * LD + k % H];
+            w = quantize(w, quant);
+        }
+        for (int k = tid; k < H * kMlpIn; k += kPassThreads) sm.w1[k] = quantize(sm.w1[k], quant);
+        for (int k = tid; k < kMlpOut * H; k += kPassThreads) {
+            sm.w3[k] = quantize(sm.w3[k], quant);
+        }
+        __syncthreads();
+    }
+    // layer 1: sample s, columns c0, c0 + 4, ...
+    {
+        const int s = tid & (kPassSamples - 1);
+        for (int j = tid / kPassSamples; j < H; j += kPassThreads / kPassSamples) {
+            float z = sm.b1[j];
+#pragma unroll
+            for (int k = 0; k < kMlpIn; ++k) {
+                z = fmaf(sm.w1[j * kMlpIn + k], sm.in[s * kMlpIn + k], z);
+            }
+            sm.a1[s * LD + j] = quantize(tanhf(quant == 2 ? quantize(z, quant) : z), quant);
+        }
     }
     __syncthreads();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int sg = tid % SG;
+    const int cg = tid / SG;  // 16 column groups
+    // layer 2: columns j = cg + 16 m
+    {
+        float acc[I][J];
+#pragma unroll
+        for (int m = 0; m < J; ++m) {
+#pragma unroll
+            for (int i = 0; i < I; ++i) acc[i][m] = sm.b2[cg + 16 * m];
+        }
+#pragma unroll 4
+        for (int k = 0; k < H; k += 4) {
+            float a[I][4], w[J][4];
+#pragma unroll
+            for (int i = 0; i < I; ++i) load4(sm.a1 + (sg + SG * i) * LD + k, a[i]);
+#pragma unroll
+            for (int m = 0; m < J; ++m) load4(sm.w2 + (cg + 16 * m) * LD + k, w[m]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+#pragma unroll
+                for (int i = 0; i < I; ++i) {
+#pragma unroll
+                    for (int m = 0; m < J; ++m) acc[i][m] = fmaf(w[m][e], a[i][e], acc[i][m]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+#pragma unroll
+            for (int m = 0; m < J; ++m) {
+                const float z = acc[i][m];
+                sm.a2[(sg + SG * i) * LD + cg + 16 * m] =
+                    quantize(tanhf(quant == 2 ? quantize(z, quant) : z), quant);
+            }
+        }
+    }
+    __syncthreads();
+    // layer 3 and the loss: one thread per (sample, output); a warp per output
     float sq = 0.0f;
-    if (b < batch) {
-        int i = b % n;
-        if (step >= 0) {
-            const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(b),
-                                                     static_cast<uint32_t>(step), 0u, 9u),
-                                          seed_key(seed));
-            i = static_cast<int>(u01_f64(r.x, r.y) * n) % n;
+    if (tid < kMlpOut * kPassSamples) {
+        const int s = tid & (kPassSamples - 1);
+        const int o = tid / kPassSamples;
+        float y = sm.b3[o];
+#pragma unroll 4
+        for (int j = 0; j < H; j += 4) {
+            float a[4], w[4];
+            load4(sm.a2 + s * LD + j, a);
+            load4(sm.w3 + o * H + j, w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y = fmaf(w[e], a[e], y);
         }
-        float in[kMlpIn];
-        for (int k = 0; k < kMlpIn; ++k) {
-            in[k] = quantize(normalise_input(box, k, x[static_cast<size_t>(i) * kMlpIn + k]),
-                             quant);
-            xb[static_cast<size_t>(b) * kMlpIn + k] = in[k];
+        float dy = 0.0f;
+        if (s < here) {
+            const float e = y - sm.target[s * 4 + o];
+            sq = e * e;
+            dy = 2.0f * e / static_cast<float>(batch * kMlpOut);
+            gy[static_cast<size_t>(b0 + s) * kMlpOut + o] = dy;
         }
-        float a1[H];
-        for (int j = 0; j < H; ++j) {
-            float z = w[M::B1 + j];
-            for (int k = 0; k < kMlpIn; ++k) z += w[M::W1 + j * kMlpIn + k] * in[k];
-            a1[j] = quantize(tanhf(quant == 2 ? quantize(z, quant) : z), quant);
-            h1[static_cast<size_t>(b) * H + j] = a1[j];
-        }
-        float y[kMlpOut];
-        for (int o = 0; o < kMlpOut; ++o) y[o] = w[M::B3 + o];
-        for (int j = 0; j < H; ++j) {
-            float z = w[M::B2 + j];
-            for (int k = 0; k < H; ++k) z += w[M::W2 + j * H + k] * a1[k];
-            const float a2 = quantize(tanhf(quant == 2 ? quantize(z, quant) : z), quant);
-            h2[static_cast<size_t>(b) * H + j] = a2;
-            for (int o = 0; o < kMlpOut; ++o) y[o] += w[M::W3 + o * H + j] * a2;
-        }
-        float dy[kMlpOut];
-        for (int o = 0; o < kMlpOut; ++o) {
-            const float target = (t[static_cast<size_t>(i) * kMlpOut + o] - box.out_offset[o]) /
-                                 box.out_scale[o];
-            const float e = y[o] - target;
-            sq += e * e;
-            dy[o] = 2.0f * e / static_cast<float>(batch * kMlpOut);
-            gy[static_cast<size_t>(b) * kMlpOut + o] = dy[o];
-        }
-        float d1[H];
-        for (int k = 0; k < H; ++k) d1[k] = 0.0f;
-        for (int j = 0; j < H; ++j) {
-            const float a2 = h2[static_cast<size_t>(b) * H + j];
-            float dh = 0.0f;
-            for (int o = 0; o < kMlpOut; ++o) dh += w[M::W3 + o * H + j] * dy[o];
-            const float dz = dh * (1.0f - a2 * a2);
-            g2[static_cast<size_t>(b) * H + j] = dz;
-            for (int k = 0; k < H; ++k) d1[k] += w[M::W2 + j * H + k] * dz;
-        }
-        for (int k = 0; k < H; ++k) {
-            g1[static_cast<size_t>(b) * H + k] = d1[k] * (1.0f - a1[k] * a1[k]);
-        }
+        sm.dy[s * 4 + o] = dy;
     }
     // batch loss (mean squared error in normalised units)
     for (int off = 16; off > 0; off >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, off);
-    if ((threadIdx.x & 31u) == 0u && sq != 0.0f) {
+    if ((tid & 31) == 0 && sq != 0.0f) {
         atomicAdd(loss, sq / static_cast<float>(batch * kMlpOut));
     }
+    __syncthreads();
+    // stores of the activations, deltas of layer 2 (whole rows, coalesced)
+    for (int k = tid; k < kPassSamples * H; k += kPassThreads) {
+        const int s = k / H;
+        const int j = k % H;
+        const float a2 = sm.a2[s * LD + j];
+        float dh = 0.0f;
+#pragma unroll
+        for (int o = 0; o < kMlpOut; ++o) dh = fmaf(sm.w3[o * H + j], sm.dy[s * 4 + o], dh);
+        const float dz = dh * fmaf(-a2, a2, 1.0f);
+        if (s < here) {
+            const size_t at = static_cast<size_t>(b0) * H + k;
+            h1[at] = sm.a1[s * LD + j];
+            h2[at] = a2;
+            g2[at] = dz;
+        }
+        sm.a2[s * LD + j] = dz;
+    }
+    __syncthreads();
+    // deltas of layer 1: columns k = J cg .. J cg + J - 1, summed over j
+    {
+        float acc[I][J] = {};
+#pragma unroll 4
+        for (int j = 0; j < H; j += 4) {
+            float d[I][4], w[4][J];
+#pragma unroll
+            for (int i = 0; i < I; ++i) load4(sm.a2 + (sg + SG * i) * LD + j, d[i]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) load_row<J>(sm.w2 + (j + e) * LD + J * cg, w[e]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+#pragma unroll
+                for (int i = 0; i < I; ++i) {
+#pragma unroll
+                    for (int m = 0; m < J; ++m) acc[i][m] = fmaf(w[e][m], d[i][e], acc[i][m]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+            const int s = sg + SG * i;
+            if (s < here) {
+#pragma unroll
+                for (int m = 0; m < J; ++m) {
+                    const float a = sm.a1[s * LD + J * cg + m];
+                    g1[static_cast<size_t>(b0 + s) * H + J * cg + m] =
+                        acc[i][m] * fmaf(-a, a, 1.0f);
+                }
+            }
+        }
+    }
 }
 
-// Weight and bias gradients, deterministic two-level reduction: block
-// (row, chunk) sums its chunk of kGradChunk samples for one parameter row,
-// threads over the row's columns; grad_sum_kernel then adds the chunk
-// partials in chunk order.  Row r of:
-//   W1 (H rows x 5):  sum_b G1[b][r] X[b][c];   b1[r] = sum_b G1[b][r]
-//   W2 (H rows x H):  sum_b G2[b][r] H1[b][c];  b2[r] = sum_b G2[b][r]
-//   W3 (3 rows x H):  sum_b GY[b][r] H2[b][c];  b3[r] = sum_b GY[b][r]
+// Weight and bias gradients of one chunk of samples:
+//   W1 (H x 5):  sum_b G1[b][r] X[b][c];   b1[r] = sum_b G1[b][r]
+//   W2 (H x H):  sum_b G2[b][r] H1[b][c];  b2[r] = sum_b G2[b][r]
+//   W3 (3 x H):  sum_b GY[b][r] H2[b][c];  b3[r] = sum_b GY[b][r]
+// blockIdx.y = chunk; blockIdx.x < (H / 32)^2: a 32 x 32 tile of W2 (and, in
+// the first tile column, its part of b2 by a warp of its own), each thread 4
+// rows x 1 column; then one block for W1 and b1 and one for W3 and b3.  The chunk's operands are
+// staged in shared memory as a whole, so a block waits for memory once.
 template <int H>
-__global__ void __launch_bounds__(64) grad_partial_kernel(int batch, const float* xb,
-                                                          const float* h1, const float* h2,
-                                                          const float* g1, const float* g2,
-                                                          const float* gy, float* partial) {
+__host__ __device__ constexpr int grad_tiles() {
+    return (H / 32) * (H / 32);
+}
+template <int H>
+constexpr size_t grad_smem_bytes() {
+    const size_t tile = 2u * kGradChunk * 32u;
+    const size_t rest = kGradChunk * (H + kMlpIn);
+    return (tile > rest ? tile : rest) * sizeof(float);
+}
+template <int H>
+__global__ void __launch_bounds__(kGradThreads + 32)
+    train_grad_kernel(int batch, const float* __restrict__ xb, const float* __restrict__ h1,
+                      const float* __restrict__ h2, const float* __restrict__ g1,
+                      const float* __restrict__ g2, const float* __restrict__ gy,
+                      float* __restrict__ partial) {
     using M = Mlp<H>;
-    const int row = blockIdx.x;
-    const int chunk = blockIdx.y;
-    const int c = threadIdx.x;
-    const float* delta;
-    const float* input;
-    int dstride, istride, cols, wbase, bbase, r;
-    if (row < H) {
-        r = row; delta = g1; dstride = H; input = xb; istride = kMlpIn; cols = kMlpIn;
-        wbase = M::W1; bbase = M::B1;
-    } else if (row < 2 * H) {
-        r = row - H; delta = g2; dstride = H; input = h1; istride = H;
-        cols = H; wbase = M::W2; bbase = M::B2;
+    extern __shared__ __align__(16) float grad_smem[];
+    const int tid = threadIdx.x;
+    const int part = static_cast<int>(blockIdx.x);
+    const int b0 = blockIdx.y * kGradChunk;
+    const int count = batch - b0 < kGradChunk ? batch - b0 : kGradChunk;
+    float* out = partial + static_cast<size_t>(blockIdx.y) * M::Params;
+    next_may_start();
+    previous_done();
+    if (part < grad_tiles<H>()) {
+        const int r0 = part / (H / 32) * 32;
+        const int c0 = part % (H / 32) * 32;
+        float* d = grad_smem;
+        float* in = grad_smem + kGradChunk * 32;
+        for (int k = tid; k < count * 8; k += blockDim.x) {
+            const int b = k >> 3;
+            const int q = (k & 7) * 4;
+            const size_t row = static_cast<size_t>(b0 + b) * H;
+            copy16(d + b * 32 + q, g2 + row + r0 + q);
+            copy16(in + b * 32 + q, h1 + row + c0 + q);
+        }
+        copies_done();
+        __syncthreads();
+        if (tid >= kGradThreads) {  // the last warp: the bias of row r0 + lane
+            if (c0 == 0) {
+                const int r = tid - kGradThreads;
+                float bacc = 0.0f;
+#pragma unroll 8
+                for (int b = 0; b < count; ++b) bacc += d[b * 32 + r];
+                out[M::B2 + r0 + r] = bacc;
+            }
+            return;
+        }
+        const int r = (tid >> 5) * 4;
+        const int c = tid & 31;
+        float acc[4] = {};
+#pragma unroll 8
+        for (int b = 0; b < count; ++b) {
+            float dv[4];
+            load4(d + b * 32 + r, dv);
+            const float iv = in[b * 32 + c];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) acc[m] = fmaf(dv[m], iv, acc[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) out[M::W2 + (r0 + r + m) * H + c0 + c] = acc[m];
+        return;
+    }
+    // thread: hidden unit r and columns (W1) or rows (W3) g, g + G, ...
+    const bool first_layer = part == grad_tiles<H>();
+    constexpr int G = kGradThreads / H;
+    const int r = tid & (H - 1);
+    const int g = tid / H;
+    float* units = grad_smem;                 // G1 or H2
+    float* other = units + kGradChunk * H;    // X or GY
+    const float* src = first_layer ? g1 : h2;
+    for (int k = tid; k < count * H / 4; k += blockDim.x) {
+        copy16(units + 4 * k, src + static_cast<size_t>(b0) * H + 4 * k);
+    }
+    const int width = first_layer ? kMlpIn : kMlpOut;
+    const float* src2 = (first_layer ? xb : gy) + static_cast<size_t>(b0) * width;
+    // a chunk's rows start on a 16-byte boundary (256 samples); the last
+    // floats of a ragged chunk go one by one
+    const int whole = count * width / 4;
+    for (int k = tid; k < whole; k += blockDim.x) copy16(other + 4 * k, src2 + 4 * k);
+    if (tid < count * width - 4 * whole) other[4 * whole + tid] = src2[4 * whole + tid];
+    copies_done();
+    __syncthreads();
+    if (tid >= kGradThreads) {  // the last warp: b3
+        const int o = tid - kGradThreads;
+        if (!first_layer && o < kMlpOut) {
+            float bacc = 0.0f;
+#pragma unroll 8
+            for (int b = 0; b < count; ++b) bacc += other[b * kMlpOut + o];
+            out[M::B3 + o] = bacc;
+        }
+        return;
+    }
+    if (first_layer) {
+        constexpr int N = (kMlpIn + 1 + G - 1) / G;  // column 5: the bias
+        float acc[N] = {};
+#pragma unroll 8
+        for (int b = 0; b < count; ++b) {
+            const float d = units[b * H + r];
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                const int c = g + m * G;
+                const float v = c < kMlpIn ? other[b * kMlpIn + c] : 1.0f;
+                acc[m] = fmaf(d, v, acc[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const int c = g + m * G;
+            if (c < kMlpIn) out[M::W1 + r * kMlpIn + c] = acc[m];
+            if (c == kMlpIn) out[M::B1 + r] = acc[m];
+        }
     } else {
-        r = row - 2 * H; delta = gy; dstride = kMlpOut; input = h2;
-        istride = H; cols = H; wbase = M::W3; bbase = M::B3;
+        constexpr int N = (kMlpOut + G - 1) / G;
+        float acc[N] = {};
+#pragma unroll 8
+        for (int b = 0; b < count; ++b) {
+            const float a = units[b * H + r];
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                const int o = g + m * G < kMlpOut ? g + m * G : 0;
+                acc[m] = fmaf(other[b * kMlpOut + o], a, acc[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const int o = g + m * G;
+            if (o < kMlpOut) out[M::W3 + o * H + r] = acc[m];
+        }
     }
-    const int b0 = chunk * kGradChunk;
-    const int b1 = b0 + kGradChunk < batch ? b0 + kGradChunk : batch;
-    float acc = 0.0f, bacc = 0.0f;
-    for (int b = b0; b < b1; ++b) {
-        const float d = delta[static_cast<size_t>(b) * dstride + r];
-        if (c < cols) acc += d * input[static_cast<size_t>(b) * istride + c];
-        bacc += d;
-    }
-    float* out = partial + static_cast<size_t>(chunk) * M::Params;
-    if (c < cols) out[wbase + r * cols + c] = acc;
-    if (c == 0) out[bbase + r] = bacc;
 }
 
-__global__ void grad_sum_kernel(const float* partial, int chunks, int params, float* grad) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= params) return;
+// The chunk partials of one parameter in chunk order.
+__device__ __forceinline__ float chunk_sum(const float* __restrict__ partial, int chunks,
+                                           int params, int k) {
     float sum = 0.0f;
+#pragma unroll 16
     for (int ch = 0; ch < chunks; ++ch) sum += partial[static_cast<size_t>(ch) * params + k];
-    grad[k] = sum;
+    return sum;
 }
 
-template <int H>
-cudaError_t launch_gradients(const SurrogateTrainLaunch& L, cudaStream_t stream) {
-    using M = Mlp<H>;
-    const int chunks = (L.batch + kGradChunk - 1) / kGradChunk;
-    grad_partial_kernel<H><<<dim3(2 * H + kMlpOut, chunks), 64, 0, stream>>>(
-        L.batch, L.xb, L.h1, L.h2, L.g1, L.g2, L.gy, L.partial);
-    grad_sum_kernel<<<(M::Params + 255) / 256, 256, 0, stream>>>(L.partial, chunks, M::Params,
-                                                                 L.grad);
-    return cudaGetLastError();
+__global__ void grad_sum_kernel(const float* __restrict__ partial, int chunks, int params,
+                                float* __restrict__ grad) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < params) grad[k] = chunk_sum(partial, chunks, params, k);
 }
 
-__global__ void adam_kernel(float* params, const float* grad, float* m, float* v, int count,
-                            float lr, float beta1, float beta2, float eps, float bias1,
-                            float bias2) {
+// Chunk sums and Adam, one thread per parameter.
+__global__ void train_update_kernel(const float* __restrict__ partial, int chunks, float* params,
+                                    float* m, float* v, int count, float lr, float beta1,
+                                    float beta2, float eps, float bias1, float bias2) {
+    next_may_start();
+    previous_done();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
-    const float g = grad[k];
+    const float g = chunk_sum(partial, chunks, count, k);
     const float mk = beta1 * m[k] + (1.0f - beta1) * g;
     const float vk = beta2 * v[k] + (1.0f - beta2) * g * g;
     m[k] = mk;
     v[k] = vk;
     params[k] -= lr * (mk / bias1) / (sqrtf(vk / bias2) + eps);
+}
+
+// A launch that may overlap the end of the stream's previous kernel (the first
+// kernel after a copy is ordered behind it as a whole: overlap = false).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(bool overlap, void (*kernel)(Params...), dim3 grid, int threads,
+                             size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// The pass and the chunk gradients of one batch (step < 0: its first samples
+// in order).
+template <int H>
+cudaError_t launch_gradients(const SurrogateTrainLaunch& L, int step, float* loss, int quant,
+                             cudaStream_t stream) {
+    const int chunks = (L.batch + kGradChunk - 1) / kGradChunk;
+    const cudaError_t err = launch_dependent(
+        step > 0, train_pass_kernel<H>, dim3((L.batch + kPassSamples - 1) / kPassSamples), kPassThreads,
+        sizeof(PassSmem<H>), stream, L.x, L.t, L.n, L.seed, step, L.batch, L.box, L.params, L.xb,
+        L.h1, L.h2, L.g1, L.g2, L.gy, loss, quant);
+    if (err != cudaSuccess) return err;
+    return launch_dependent(true, train_grad_kernel<H>, dim3(grad_tiles<H>() + 2, chunks),
+                            kGradThreads + 32, grad_smem_bytes<H>(), stream, L.batch, L.xb, L.h1,
+                            L.h2, L.g1, L.g2, L.gy, L.partial);
+}
+
+// Shared memory beyond 48 KB has to be asked for once per kernel.
+template <int H>
+cudaError_t prepare_training() {
+    cudaError_t err = cudaFuncSetAttribute(train_pass_kernel<H>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>(sizeof(PassSmem<H>)));
+    if (err != cudaSuccess) return err;
+    return cudaFuncSetAttribute(train_grad_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(grad_smem_bytes<H>()));
 }
 
 // FP32 SIMT forward of normalised features -> normalised outputs.
@@ -468,24 +822,27 @@ namespace {
 
 template <int H>
 cudaError_t train_step(const SurrogateTrainLaunch& L, int step, cudaStream_t stream) {
-    fwd_bwd_kernel<H><<<(L.batch + 127) / 128, 128, 0, stream>>>(
-        L.x, L.t, L.n, L.seed, step, L.batch, L.box, L.params, L.xb, L.h1, L.h2, L.g1, L.g2, L.gy,
-        L.loss + step, step >= L.quant_from ? L.quant : 0);
-    launch_gradients<H>(L, stream);
+    const cudaError_t err = launch_gradients<H>(L, step, L.loss + step,
+                                                step >= L.quant_from ? L.quant : 0, stream);
+    if (err != cudaSuccess) return err;
     const float t1 = static_cast<float>(step + 1);
     const float bias1 = 1.0f - powf(L.beta1, t1);
     const float bias2 = 1.0f - powf(L.beta2, t1);
-    adam_kernel<<<(Mlp<H>::Params + 255) / 256, 256, 0, stream>>>(
-        L.params, L.grad, L.m, L.v, Mlp<H>::Params, L.lr, L.beta1, L.beta2, 1e-8f, bias1, bias2);
-    return cudaGetLastError();
+    const int chunks = (L.batch + kGradChunk - 1) / kGradChunk;
+    return launch_dependent(true, train_update_kernel, dim3((Mlp<H>::Params + 63) / 64), 64, 0, stream,
+                            L.partial, chunks, L.params, L.m, L.v, Mlp<H>::Params, L.lr, L.beta1,
+                            L.beta2, 1e-8f, bias1, bias2);
 }
 
 template <int H>
 cudaError_t gradient(const SurrogateTrainLaunch& L, cudaStream_t stream) {
-    fwd_bwd_kernel<H><<<(L.batch + 127) / 128, 128, 0, stream>>>(
-        L.x, L.t, L.n, L.seed, -1, L.batch, L.box, L.params, L.xb, L.h1, L.h2, L.g1, L.g2, L.gy,
-        L.loss, 0);
-    return launch_gradients<H>(L, stream);
+    cudaError_t err = prepare_training<H>();
+    if (err == cudaSuccess) err = launch_gradients<H>(L, -1, L.loss, 0, stream);
+    if (err != cudaSuccess) return err;
+    const int chunks = (L.batch + kGradChunk - 1) / kGradChunk;
+    grad_sum_kernel<<<(Mlp<H>::Params + 63) / 64, 64, 0, stream>>>(L.partial, chunks,
+                                                                   Mlp<H>::Params, L.grad);
+    return cudaGetLastError();
 }
 
 template <int H>
@@ -523,6 +880,10 @@ cudaError_t eval(int n, const double* inputs, const SurrogateBox& box, const Sur
 }
 
 }  // namespace
+
+cudaError_t surrogate_prepare_training(int hidden) {
+    return hidden == 64 ? prepare_training<64>() : prepare_training<32>();
+}
 
 cudaError_t surrogate_train_step(const SurrogateTrainLaunch& L, int step, cudaStream_t stream) {
     return L.box.hidden == 64 ? train_step<64>(L, step, stream) : train_step<32>(L, step, stream);
