@@ -171,13 +171,11 @@ __global__ void build_table_kernel(const TableLaunch L) {
     }
 }
 
-// One thread per (cell, sector): sector s of line m holds frame m % 2 of
-// component pair 4 (m / 2) + s at the cell's four corners (zeros past the
-// last component).  Cells on the last ghosted column or row have no
-// upper-right corner and no record; no particle's stencil starts there.
+// One thread per (cell, sector).  Cells on the last ghosted column or row
+// have no upper-right corner and no record; no particle's stencil starts
+// there.
 template <bool FOCUSED>
 __global__ void build_records_kernel(const RecordLaunch L) {
-    constexpr int C = FOCUSED ? 21 : 16;
     constexpr int S = record_sectors(FOCUSED);
     const uint64_t total = L.points * S;
     const size_t ex = static_cast<size_t>(L.ex);
@@ -187,19 +185,15 @@ __global__ void build_records_kernel(const RecordLaunch L) {
         const int sector = static_cast<int>(q % S);
         const size_t i = p % ex, j = p / ex;
         if (i + 1 >= ex || j + 2 > static_cast<size_t>(L.ey)) continue;
-        const int line = sector / 4;
-        const float* table = (line & 1) ? L.upper : L.lower;
-        const int first = 2 * (4 * (line / 2) + sector % 4);
+        const float* table = record_frame(FOCUSED, sector) != 0 ? L.upper : L.lower;
+        const int first = record_component(FOCUSED, record_pair(FOCUSED, sector));
         const size_t corner[4] = {p, p + 1, p + ex, p + ex + 1};
         float v[8];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            v[2 * k] = first < C ? __ldg(table + table_f32_offset(FOCUSED, L.points, corner[k],
-                                                                  first))
-                                 : 0.0f;
-            v[2 * k + 1] = first + 1 < C ? __ldg(table + table_f32_offset(FOCUSED, L.points,
-                                                                          corner[k], first + 1))
-                                         : 0.0f;
+            v[2 * k] = __ldg(table + table_f32_offset(FOCUSED, L.points, corner[k], first));
+            v[2 * k + 1] =
+                __ldg(table + table_f32_offset(FOCUSED, L.points, corner[k], first + 1));
         }
         float4* out =
             reinterpret_cast<float4*>(L.records + p * record_floats(FOCUSED) + 8 * sector);

@@ -41,17 +41,33 @@ __host__ __device__ inline size_t table_f32_offset(bool focused, size_t points, 
 // Cell records of a pair of FP32 tables (the frames at the interval's two
 // ends), for the mixed pushes.  The record of a cell is indexed by its
 // lower-left ghosted point p and is made of 128-byte lines of four 32-byte
-// sectors.  Line m holds frame m % 2 (lower, upper) of the component pairs
-// 4 (m / 2) .. 4 (m / 2) + 3; the sector of pair k holds components 2k and
-// 2k + 1 at the cell's corners p, p + 1, p + ex, p + ex + 1, pair by pair --
-// the operands of the packed-pair interpolation, in the order the
-// point-major sampler accumulates them.  Four lanes then read one line of a
-// particle's record per request (four lines for the point-major rows), and
-// a lane interpolates a component pair from its own two sectors.
-// Components past the last are zero padding.
-__host__ __device__ constexpr int record_sectors(bool focused) { return focused ? 24 : 16; }
+// sectors.  A sector holds one component pair of one frame at the cell's
+// corners p, p + 1, p + ex, p + ex + 1, pair by pair -- the operands of the
+// packed-pair interpolation, in the order the point-major sampler accumulates
+// them.  The pairs are those of the components the push reads: all 16
+// (Parker), or the 20 other than Vz (focused; Vz enters no rate, and leaving
+// it out makes five lines of six).  Lines 2i and 2i + 1 hold pairs 4i .. 4i + 3
+// of the lower and of the upper frame; two pairs left over share one line,
+// lower frame first.  Four lanes then read one line of a particle's record
+// per request (four lines for the point-major rows).
+__host__ __device__ constexpr int record_pairs(bool focused) { return focused ? 10 : 8; }
+__host__ __device__ constexpr int record_sectors(bool focused) {
+    return 2 * record_pairs(focused);
+}
 __host__ __device__ constexpr int record_floats(bool focused) {
     return 8 * record_sectors(focused);
+}
+// Frame and pair of a record's sector, first component of a pair (its second
+// is the next one).
+__host__ __device__ constexpr int record_frame(bool focused, int sector) {
+    return sector < 16 ? (sector / 4) % 2 : (sector - 16) / (record_pairs(focused) - 8);
+}
+__host__ __device__ constexpr int record_pair(bool focused, int sector) {
+    return sector < 16 ? 4 * (sector / 8) + sector % 4
+                       : 8 + (sector - 16) % (record_pairs(focused) - 8);
+}
+__host__ __device__ constexpr int record_component(bool focused, int pair) {
+    return 2 * pair + (focused && pair > 0 ? 1 : 0);
 }
 
 struct RecordLaunch {

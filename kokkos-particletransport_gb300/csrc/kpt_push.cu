@@ -843,9 +843,9 @@ __device__ __forceinline__ void sample_mixed(const StateMixed& st, const PushPar
                                     rt, P.s.time_interpolation, c);
 }
 
-// Per-warp shared memory of the record sampler: 32 rows of the components
-// rounded up to whole pairs (row strides of 22 and 18 floats keep its 64-bit
-// stores and loads free of bank conflicts).
+// Per-warp shared memory of the record sampler: 32 rows of the sampled
+// pairs (row strides of 22 and 18 floats keep its 64-bit stores and loads
+// free of bank conflicts).
 __host__ __device__ constexpr int record_xpose_stride(bool focused) {
     return focused ? 22 : 18;
 }
@@ -857,12 +857,17 @@ __host__ __device__ constexpr size_t record_xpose_bytes(bool focused, int warps)
 // converged; rec = the lane's cell record, any valid record for a lane
 // without a particle).  Lanes 4g..4g+3 form a group: for each of the
 // group's four particles in turn, lane 4g+s reads the sectors of component
-// pairs s, s+4, s+8 of that particle's record -- one 128-byte line per
+// pairs s and s+4 of that particle's record -- one 128-byte line per
 // request for the group -- and interpolates each pair from its own sectors
 // with the eight corner weights, in the operations and the order of
 // sample_stencil_pairs, so the values equal the point-major sampler's bit
-// for bit.  The pairs then reach their particle's lane through the warp's
-// rows of shared memory.
+// for bit.  The focused record's last line holds two pairs of both frames:
+// lanes 0 and 1 interpolate their lower frame and hand the sums to lanes 2
+// and 3, which add the upper one.  The pairs then reach their particle's lane
+// through the warp's rows of shared memory.  c[2] (Vz) is not sampled by the
+// focused push, which does not read it: five lines a particle instead of six,
+// 8.44 -> 7.61 ms for two 100-step intervals of 777 777 particles (512 x
+// 1024, slab QLT), 58.8 -> 55.6 ms for the 4 Mi-particle learned closure.
 // Particles of a group whose requests the sampler unrolls together (4: all
 // of the group's loads may be in flight at once, register pressure allowing).
 #ifndef KPT_RECORD_Q_UNROLL
@@ -872,8 +877,8 @@ constexpr int kRecordQUnroll = KPT_RECORD_Q_UNROLL;
 template <bool FOCUSED, bool USE_TIME>
 __device__ __forceinline__ void sample_records(const float* rec, float w0, float w1, float rt,
                                                float (&c)[FOCUSED ? 21 : 16], float* xpose) {
-    constexpr int C = FOCUSED ? 21 : 16;
-    constexpr int GROUPS = record_sectors(FOCUSED) / 8;  // line pairs (frames 0 and 1)
+    constexpr int PAIRS = record_pairs(FOCUSED);
+    static_assert(PAIRS == 8 || PAIRS == 10, "two line pairs, and a shared line for two pairs");
     constexpr int XS = record_xpose_stride(FOCUSED);
     const unsigned full = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
@@ -900,7 +905,7 @@ __device__ __forceinline__ void sample_records(const float* rec, float w0, float
         const float* sector = reinterpret_cast<const float*>(qrec) + 8 * s;
         float* row = xpose + (group + q) * XS;
 #pragma unroll
-        for (int m = 0; m < GROUPS; ++m) {
+        for (int m = 0; m < 2; ++m) {
             unsigned long long v[4];
             load4_pairs(sector + 64 * m, v);
             unsigned long long acc = f2_mul(w_lo[0], v[0]);
@@ -911,21 +916,32 @@ __device__ __forceinline__ void sample_records(const float* rec, float w0, float
 #pragma unroll
                 for (int k = 0; k < 4; ++k) acc = f2_fma(w_hi[k], v[k], acc);
             }
-            const int first = 2 * (4 * m + s);
-            if (8 * m + 7 < C || first < C) {
-                *reinterpret_cast<unsigned long long*>(row + first) = acc;
+            *reinterpret_cast<unsigned long long*>(row + 2 * (4 * m + s)) = acc;
+        }
+        if (PAIRS > 8) {  // the shared last line
+            unsigned long long v[4];
+            load4_pairs(sector + 128, v);
+            unsigned long long acc = f2_mul(w_lo[0], v[0]);
+#pragma unroll
+            for (int k = 1; k < 4; ++k) acc = f2_fma(w_lo[k], v[k], acc);
+            if (USE_TIME) {
+                acc = __shfl_up_sync(full, acc, 2, 4);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc = f2_fma(w_hi[k], v[k], acc);
+            }
+            if ((s >= 2) == USE_TIME) {
+                *reinterpret_cast<unsigned long long*>(row + 2 * (8 + (s & 1))) = acc;
             }
         }
     }
     __syncwarp();
     const unsigned long long* mine = reinterpret_cast<const unsigned long long*>(xpose + lane * XS);
 #pragma unroll
-    for (int k = 0; k < (C + 1) / 2; ++k) {
-        float lo, hi;
-        f2_split(mine[k], lo, hi);
-        c[2 * k] = lo;
-        if (2 * k + 1 < C) c[2 * k + 1] = hi;
+    for (int k = 0; k < PAIRS; ++k) {
+        const int first = record_component(FOCUSED, k);
+        f2_split(mine[k], c[first], c[first + 1]);
     }
+    if (FOCUSED) c[2] = 0.0f;
     __syncwarp();
 }
 
