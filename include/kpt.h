@@ -241,10 +241,11 @@ int kpt_context_set_fp64_arithmetic(kpt_context* ctx, int mode);
  * keeps one record per cell with each component's eight corner values of
  * both frames in one 32-byte sector, so four lanes of a warp read a
  * particle's cell one 128-byte line at a time.  KPT_RECORDS_AUTO (default)
- * builds them (record_floats x 4 bytes per table point: 768 focused, 512
+ * builds them (record_floats x 4 bytes per table point: 640 focused, 512
  * Parker; rebuilt when the table pair changes) for a refill-scheduled
  * mixed push of at least a quarter as many particles as the table has
- * points; KPT_RECORDS_OFF never, KPT_RECORDS_ON for every refill-scheduled
+ * points, or of fewer that fill the GPU for enough substeps to repay the
+ * build; KPT_RECORDS_OFF never, KPT_RECORDS_ON for every refill-scheduled
  * mixed push.  Results are bit-identical either way.  The records are built
  * on the context's stream; a later push on another stream waits for them. */
 enum kpt_records_mode { KPT_RECORDS_AUTO = 0, KPT_RECORDS_OFF = 1, KPT_RECORDS_ON = 2 };

@@ -79,7 +79,7 @@ struct Num<float> {
     static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
     static __device__ __forceinline__ bool finite(float a) { return isfinite(a); }
     static __device__ __forceinline__ float abs(float a) { return fabsf(a); }
-    static __device__ __forceinline__ float noise(uint32_t, uint32_t hi) {
+    static __device__ __forceinline__ float noise(uint32_t hi) {
         return -static_cast<float>(kSqrt3) + static_cast<float>(2.0 * kSqrt3) * u01_f32(hi);
     }
 };
@@ -628,18 +628,25 @@ __device__ __forceinline__ bool physics(const T* c, T p, T pitch_mu, const Const
     return true;
 }
 
+// The words of a substep's draws that the mixed push uses: the high words of
+// draws 0 and 1 and of draw 2 (Parker, along the field) or 3 (focused, pitch
+// angle).
+struct Draws {
+    uint32_t first, second, third;
+};
+
 // Displacements and the new pitch cosine from the four draws of a substep
 // (src/main.cpp:1280-1291 Parker, :1660-1702 focused).
 template <typename T, bool FOCUSED>
-__device__ __forceinline__ void increments(const Rates<T>& r, T dt, const uint4& r0,
-                                           const uint4& r1, const Consts<T>& s, T& delta_x,
-                                           T& delta_y, T& new_mu) {
+__device__ __forceinline__ void increments(const Rates<T>& r, T dt, const Draws& d,
+                                           const Consts<T>& s, T& delta_x, T& delta_y,
+                                           T& new_mu) {
     using N = Num<T>;
     const T sdt = N::sqrt(dt);
     if (FOCUSED) {
-        const T ran1 = N::noise(r0.x, r0.y);
-        const T ran2 = N::noise(r0.z, r0.w);
-        const T pitch_random = N::noise(r1.z, r1.w);
+        const T ran1 = N::noise(d.first);
+        const T ran2 = N::noise(d.second);
+        const T pitch_random = N::noise(d.third);
         const T bxn = r.bx * r.ib;
         const T byn = r.by * r.ib;
         const T bzn = r.bz * r.ib;
@@ -657,9 +664,9 @@ __device__ __forceinline__ void increments(const Rates<T>& r, T dt, const uint4&
         new_mu = clamp_mu(r.pitch_mu + r.dmu_dt * dt + pitch_random * N::sqrt(T(2) * r.duu) * sdt,
                           s.mu_max);
     } else {
-        const T ran1 = N::noise(r0.x, r0.y);
-        const T ran2 = N::noise(r0.z, r0.w);
-        const T ran3 = N::noise(r1.x, r1.y);
+        const T ran1 = N::noise(d.first);
+        const T ran2 = N::noise(d.second);
+        const T ran3 = N::noise(d.third);
         delta_x = r.dx_dt * dt + ran1 * r.skperp * sdt + ran3 * r.skpara_perp * sdt * r.bx * r.ib;
         delta_y = r.dy_dt * dt + ran2 * r.skperp * sdt + ran3 * r.skpara_perp * sdt * r.by * r.ib;
         new_mu = r.pitch_mu;
@@ -715,6 +722,7 @@ struct PushParams {
     const float* records;  // cell records of (lower, upper); nullptr: point-major sampling
     F64Consts f64;         // FP64 push
     PowPlan pows;
+    unsigned lane_cap;     // particles a warp holds (kPushFew)
 };
 
 // ------------------------------------------------------------ mixed path
@@ -967,7 +975,18 @@ __device__ __forceinline__ void sample_mixed_warp(const StateMixed& st, const Pu
     }
 }
 
-// Physics, step size, noise and the state update of one substep.
+// The draws of the substep st.steps (counted from 1).  (Drawn ahead of the
+// sampling, in the shadow of its loads, the substep is slower: three more
+// registers live across it cost loads in flight, Parker 50.7 -> 55.8 ms.)
+template <bool FOCUSED>
+__device__ __forceinline__ Draws draw_mixed(const StateMixed& st, const PushParams& P) {
+    const uint32_t block = 2u * static_cast<uint32_t>(st.steps - 1);
+    const uint4 r0 = philox4x32_10(make_uint4(block, st.index, P.frame, kTagPush), P.key);
+    const uint4 r1 = philox4x32_10(make_uint4(block + 1u, st.index, P.frame, kTagPush), P.key);
+    return Draws{r0.y, r0.w, FOCUSED ? r1.w : r1.y};
+}
+
+// Physics, step size and the state update of one substep.
 template <bool FOCUSED, bool SURR = false>
 __device__ __forceinline__ bool advance_mixed(StateMixed& st, const PushParams& P,
                                               const float (&c)[FOCUSED ? 21 : 16],
@@ -993,11 +1012,8 @@ __device__ __forceinline__ bool advance_mixed(StateMixed& st, const PushParams& 
         st.status = 2;
         return false;
     }
-    const uint32_t block = 2u * static_cast<uint32_t>(st.steps - 1);
-    const uint4 r0 = philox4x32_10(make_uint4(block, st.index, P.frame, kTagPush), P.key);
-    const uint4 r1 = philox4x32_10(make_uint4(block + 1u, st.index, P.frame, kTagPush), P.key);
     float dx, dy, mu;
-    increments<float, FOCUSED>(r, dtf, r0, r1, P.kf, dx, dy, mu);
+    increments<float, FOCUSED>(r, dtf, draw_mixed<FOCUSED>(st, P), P.kf, dx, dy, mu);
     const float dp = r.dp_dt * dtf;
     if (!isfinite(dx) || !isfinite(dy) || !isfinite(dp)) {
         st.status = 2;
@@ -1034,11 +1050,57 @@ __device__ __forceinline__ bool substep_records(StateMixed& st, const PushParams
     return have && advance_mixed<FOCUSED>(st, P, c);
 }
 
-// Per-lane tallies of the surrogate judge.
-struct JudgeTally {
-    unsigned long long evaluations, judged, fallbacks;
-    float max_error;
+// Counters of one block, in shared memory: they change when a particle
+// finishes, is judged or falls back, so keeping them out of the registers
+// costs nothing per substep and leaves 7 (14 with the network's) registers to
+// the warps.
+struct BlockTally {
+    unsigned steps[2], fallbacks[2];  // low and high words
+    unsigned pushed, failed, max_steps, judged;
+    unsigned max_error;  // float bits (non-negative floats order like them)
 };
+
+__device__ __forceinline__ void tally_init(BlockTally& b) {
+    if (threadIdx.x == 0) b = BlockTally{};
+    __syncthreads();
+}
+
+__device__ __forceinline__ void tally_add(unsigned (&word)[2], unsigned v) {
+    const unsigned old = atomicAdd(&word[0], v);
+    if (old + v < old) atomicAdd(&word[1], 1u);
+}
+
+// A particle the block loaded has reached its last substep.
+__device__ __forceinline__ void tally_finish(BlockTally& b, int steps, int status) {
+    tally_add(b.steps, static_cast<unsigned>(steps));
+    atomicAdd(&b.pushed, 1u);
+    if (status != 0) atomicAdd(&b.failed, 1u);
+    atomicMax(&b.max_steps, static_cast<unsigned>(steps));
+}
+
+__device__ __forceinline__ unsigned long long tally_word(const unsigned (&word)[2]) {
+    return (static_cast<unsigned long long>(word[1]) << 32) | word[0];
+}
+
+// The block's counters to the launch's (every thread calls it, at the end).
+__device__ __forceinline__ void tally_flush(const BlockTally& b, PushCounters* counters,
+                                            unsigned long long* judge) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const unsigned long long steps = tally_word(b.steps);
+    if (steps) atomicAdd(&counters->particle_steps, steps);
+    if (b.pushed) atomicAdd(&counters->pushed, static_cast<unsigned long long>(b.pushed));
+    if (b.failed) atomicAdd(&counters->failed, static_cast<unsigned long long>(b.failed));
+    if (b.max_steps) atomicMax(&counters->max_steps, b.max_steps);
+    if (judge != nullptr) {
+        // every substep of a particle is served by the network or falls back
+        const unsigned long long fallbacks = tally_word(b.fallbacks);
+        if (steps != fallbacks) atomicAdd(judge + 0, steps - fallbacks);
+        if (b.judged) atomicAdd(judge + 1, static_cast<unsigned long long>(b.judged));
+        if (fallbacks) atomicAdd(judge + 2, fallbacks);
+        atomicMax(judge + 3, static_cast<unsigned long long>(b.max_error));
+    }
+}
 
 // The closure values of one lane, in FP32: the network's normalised outputs
 // y mapped back to D_mumu, dD_mumu/dmu and kappa_parallel (use = inside the
@@ -1051,7 +1113,7 @@ struct JudgeTally {
 // plain closure in its own precision.
 __device__ __forceinline__ Served serve_closure(const PushParams& P, bool use, float mu,
                                                 float b, float p, int steps,
-                                                const float (&y)[kMlpOut], JudgeTally& tally) {
+                                                const float (&y)[kMlpOut], BlockTally& tally) {
     const SurrogateBox& box = P.sg.box;
     Served served;
     served.use = use;
@@ -1066,9 +1128,8 @@ __device__ __forceinline__ Served serve_closure(const PushParams& P, bool use, f
         served.duu_du = served.duu * (__fdividef(sign * y1, amu + P.kf.qlt_h0) -
                                       __fdividef(2.0f * mu, one_minus_mu2));
         served.kpara = __expf(y2);
-        ++tally.evaluations;
     } else {
-        ++tally.fallbacks;
+        tally_add(tally.fallbacks, 1u);
     }
     const bool blend = use && amu < 2.0f * box.mu_cut;
     const bool judge = use && (steps & (P.sg.judge_period - 1)) == 0;
@@ -1087,8 +1148,8 @@ __device__ __forceinline__ Served serve_closure(const PushParams& P, bool use, f
             const float e_d = fabsf(served.duu - duu) / duu;
             const float e_k = fabsf(served.kpara - kpara) / kpara;
             const float e = fmaxf(e_d, e_k);
-            tally.max_error = isfinite(e) ? fmaxf(tally.max_error, e) : INFINITY;
-            ++tally.judged;
+            atomicMax(&tally.max_error, __float_as_uint(isfinite(e) ? e : INFINITY));
+            atomicAdd(&tally.judged, 1u);
         }
         if (blend) {
             // continuous hand-over to the plain closure below mu_cut: a
@@ -1123,7 +1184,7 @@ __device__ __forceinline__ Served serve_closure(const PushParams& P, bool use, f
 // block, when a completion wait timed out (the substep is abandoned).
 template <bool FP16, int H, bool TC = false>
 __device__ __forceinline__ bool substep_surrogate(StateMixed& st, const PushParams& P, bool have,
-                                                  const uint2* smem, JudgeTally& tally,
+                                                  const uint2* smem, BlockTally& tally,
                                                   float* xpose, TcNet* net = nullptr,
                                                   bool* fail = nullptr, bool* stop = nullptr) {
     const SurrogateDevice& sg = P.sg;
@@ -1240,64 +1301,48 @@ __device__ __forceinline__ bool live(const StateMixed& st, const PushParams& P) 
 }
 
 // ---------------------------------------------------------------- drivers
-__device__ __forceinline__ void flush_counters(PushCounters* counters, unsigned long long steps,
-                                               unsigned long long pushed,
-                                               unsigned long long failed, unsigned int max_steps) {
-    const unsigned full = 0xffffffffu;
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-        steps += __shfl_down_sync(full, steps, offset);
-        pushed += __shfl_down_sync(full, pushed, offset);
-        failed += __shfl_down_sync(full, failed, offset);
-        max_steps = max(max_steps, __shfl_down_sync(full, max_steps, offset));
-    }
-    if ((threadIdx.x & 31u) == 0u) {
-        if (steps) atomicAdd(&counters->particle_steps, steps);
-        if (pushed) atomicAdd(&counters->pushed, pushed);
-        if (failed) atomicAdd(&counters->failed, failed);
-        if (max_steps) atomicMax(&counters->max_steps, max_steps);
-    }
-}
-
-__device__ __forceinline__ void flush_judge(unsigned long long* judge, JudgeTally t) {
-    const unsigned full = 0xffffffffu;
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-        t.evaluations += __shfl_down_sync(full, t.evaluations, offset);
-        t.judged += __shfl_down_sync(full, t.judged, offset);
-        t.fallbacks += __shfl_down_sync(full, t.fallbacks, offset);
-        t.max_error = fmaxf(t.max_error, __shfl_down_sync(full, t.max_error, offset));
-    }
-    if ((threadIdx.x & 31u) == 0u) {
-        if (t.evaluations) atomicAdd(judge + 0, t.evaluations);
-        if (t.judged) atomicAdd(judge + 1, t.judged);
-        if (t.fallbacks) atomicAdd(judge + 2, t.fallbacks);
-        // non-negative floats order like their bit patterns
-        atomicMax(judge + 3, static_cast<unsigned long long>(__float_as_uint(t.max_error)));
-    }
-}
-
 // Persistent warps with lane refill.  A warp claims particles from the
 // cursor in batches of (idle lanes); each trip advances every busy lane by
 // one substep.  Every trip either advances a particle (bounded by the step
 // guard) or moves the cursor, so the loop always terminates.
+//
+// Three builds, one register budget and one schedule of the loads each:
+//  * kPushDense: large populations, on cell records (warp-collective), or on
+//    the point-major tables when a launch asks for more than three blocks per
+//    SM.  (Without that choice in the loop the record path compiles to a
+//    schedule that is 4 % slower: 51.1 against 49.0 ms, 1 Mi Parker.)
+//  * kPushPoints: the point-major tables, each lane on its own, for
+//    populations too thin for records: loads in flight count for more than
+//    warps.  5 / 4 / 3 / 2 blocks per SM: 12.4 / 11.3 / 9.9 / 10.0 ms (50 000
+//    Parker particles, adaptive), 2.40 / 2.40 / 2.16 / 2.35 ms (100 000
+//    focused, 2 x 100 steps).
+//  * kPushFew: the point-major tables for populations that fit in eight warps
+//    per SM.  Nothing hides a substep's latency there, so it is what counts:
+//    up to 255 registers let all loads of a substep be in flight at once, and
+//    the particles are spread over all warps (lane_cap each, placed by
+//    position, warps of different SMs first), since a gather of 32 lanes
+//    occupies the L1 pipe for 32 cycles and one of three lanes for three.
+//    3 000 Parker particles, adaptive: 6.73 -> 5.31 ms; 2 000 focused, 2 x 100
+//    steps: 1.44 -> 0.71 ms; 30 000: 1.51 -> 0.93 ms.
+enum PushKind : int { kPushDense = 0, kPushPoints = 1, kPushFew = 2 };
+
 // Resident blocks of 128 threads per SM the register budget targets: the
-// mixed kernels are latency-bound gathers and want more warps in flight.
+// mixed kernels are latency-bound gathers that want both warps and loads in
+// flight.  Plain closures on records: 5 blocks (96 registers) 50.7 ms Parker,
+// 7.37 ms focused; 4 blocks 52.1 / 7.40; 6 blocks 53.0 / 7.81; 3 blocks 55.6 /
+// 8.38.
 #ifndef KPT_MIXED_MIN_BLOCKS
 #define KPT_MIXED_MIN_BLOCKS 5
 #endif
-template <bool FOCUSED>
-struct MinBlocks {
-    static constexpr int value = KPT_MIXED_MIN_BLOCKS;
-};
-// Focused mixed push with the plain closure: 5 blocks (96 registers, a few
-// spilled bytes) measured 2.9 % faster than 4 blocks at 128 registers.
 #ifndef KPT_MIXED_FOCUSED_MIN_BLOCKS
 #define KPT_MIXED_FOCUSED_MIN_BLOCKS 5
 #endif
-template <>
-struct MinBlocks<true> {
-    static constexpr int value = KPT_MIXED_FOCUSED_MIN_BLOCKS;
+constexpr int kPointsBlocks = 3;
+constexpr int kFewBlocks = 2;
+template <bool FOCUSED>
+struct MinBlocks {
+    static constexpr int value =
+        FOCUSED ? KPT_MIXED_FOCUSED_MIN_BLOCKS : KPT_MIXED_MIN_BLOCKS;
 };
 
 // The surrogate instantiations keep the MLP fragments live beside the
@@ -1311,22 +1356,29 @@ struct MinBlocks<true> {
 #endif
 __host__ __device__ constexpr bool surr_fp16(int surr) { return surr == 2 || surr == 4; }
 __host__ __device__ constexpr int surr_hidden(int surr) { return surr <= 2 ? 64 : 32; }
-template <bool FOCUSED, int SURR = 0>
-__global__ void __launch_bounds__(128, SURR >= 3 ? KPT_SURROGATE32_MIN_BLOCKS
-                                       : SURR    ? KPT_SURROGATE_MIN_BLOCKS
-                                                 : MinBlocks<FOCUSED>::value)
+template <bool FOCUSED, int SURR, int KIND>
+constexpr int push_blocks() {
+    return KIND == kPushFew ? kFewBlocks
+           : KIND == kPushPoints && SURR == 0 ? kPointsBlocks
+           : SURR >= 3      ? KPT_SURROGATE32_MIN_BLOCKS
+           : SURR           ? KPT_SURROGATE_MIN_BLOCKS
+                            : MinBlocks<FOCUSED>::value;
+}
+template <bool FOCUSED, int SURR, int KIND>
+__global__ void __launch_bounds__(128, (push_blocks<FOCUSED, SURR, KIND>()))
     push_refill_kernel(const PushParams P) {
     const unsigned full = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lanes_below = (1u << lane) - 1u;
     extern __shared__ uint2 surrogate_smem[];
-    JudgeTally tally{0ull, 0ull, 0ull, 0.0f};
+    __shared__ BlockTally tally;
+    tally_init(tally);
     if (SURR) {
         load_surrogate_block<surr_hidden(SURR)>(P.sg.block, surrogate_smem);
     }
     // the warp's rows for the record sampler, after the network's block
     float* xpose = nullptr;
-    if (P.records != nullptr) {
+    if (KIND == kPushDense && P.records != nullptr) {
         xpose = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(surrogate_smem) +
                                          (SURR ? mlp_smem_bytes(surr_hidden(SURR)) : 0)) +
                 (threadIdx.x >> 5) * 32 * record_xpose_stride(FOCUSED);
@@ -1334,33 +1386,39 @@ __global__ void __launch_bounds__(128, SURR >= 3 ? KPT_SURROGATE32_MIN_BLOCKS
     StateMixed st;
     bool have = false;
     bool exhausted = false;
-    unsigned long long my_steps = 0, my_pushed = 0, my_failed = 0;
-    unsigned int my_max = 0;
     for (;;) {
         const unsigned idle = __ballot_sync(full, !have);
         if (idle != 0u && !exhausted) {
-            const unsigned n_idle = __popc(idle);
-            const int leader = __ffs(idle) - 1;
             unsigned base = 0;
-            if (static_cast<int>(lane) == leader) {
-                base = atomicAdd(&P.counters->next_particle, n_idle);
-            }
-            base = __shfl_sync(full, base, leader);
-            if (static_cast<uint64_t>(base) + n_idle >= P.count) {
+            unsigned place = __popc(idle & lanes_below);
+            bool claim = !have;
+            if (KIND == kPushFew) {
+                // every particle has its place: one claim, no cursor
+                base = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * P.lane_cap;
+                claim = place < P.lane_cap;
                 exhausted = true;
+            } else {
+                const unsigned n_idle = __popc(idle);
+                const int leader = __ffs(idle) - 1;
+                if (static_cast<int>(lane) == leader) {
+                    base = atomicAdd(&P.counters->next_particle, n_idle);
+                }
+                base = __shfl_sync(full, base, leader);
+                if (static_cast<uint64_t>(base) + n_idle >= P.count) {
+                    exhausted = true;
+                }
             }
-            if (!have) {
-                const uint64_t slot = static_cast<uint64_t>(base) + __popc(idle & lanes_below);
+            if (claim) {
+                const uint64_t slot = static_cast<uint64_t>(base) + place;
                 if (slot < P.count) {
                     const uint32_t idx = P.order != nullptr ? __ldg(P.order + slot)
                                                             : static_cast<uint32_t>(slot);
                     if (P.parts.status[idx] == 0) {
                         load<FOCUSED>(st, P, idx);
-                        ++my_pushed;
                         have = true;
                         if (!live(st, P)) {
                             store<FOCUSED>(st, P);
-                            my_failed += st.status != 0 ? 1 : 0;
+                            tally_finish(tally, st.steps, st.status);
                             have = false;
                         }
                     }
@@ -1383,16 +1441,11 @@ __global__ void __launch_bounds__(128, SURR >= 3 ? KPT_SURROGATE32_MIN_BLOCKS
         }
         if (have && !more) {
             store<FOCUSED>(st, P);
-            my_steps += static_cast<unsigned long long>(st.steps);
-            my_max = max(my_max, static_cast<unsigned int>(st.steps));
-            my_failed += st.status != 0 ? 1 : 0;
+            tally_finish(tally, st.steps, st.status);
             have = false;
         }
     }
-    flush_counters(P.counters, my_steps, my_pushed, my_failed, my_max);
-    if (SURR) {
-        flush_judge(P.sg.judge, tally);
-    }
+    tally_flush(tally, P.counters, SURR ? P.sg.judge : nullptr);
 }
 
 // The learned-closure push with the network on the tcgen05 tensor cores.
@@ -1423,13 +1476,12 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
                        ? nullptr
                        : reinterpret_cast<float*>(tc_smem + tc_xpose_offset<H>()) +
                              (threadIdx.x >> 5) * 32 * record_xpose_stride(true);
-    JudgeTally tally{0ull, 0ull, 0ull, 0.0f};
+    __shared__ BlockTally tally;
+    tally_init(tally);
     StateMixed st;
     bool have = false;
     bool exhausted = false;
     bool fail = false;
-    unsigned long long my_steps = 0, my_pushed = 0, my_failed = 0;
-    unsigned int my_max = 0;
     for (;;) {
         const unsigned idle = __ballot_sync(full, !have);
         if (idle != 0u && !exhausted) {
@@ -1450,11 +1502,10 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
                                                             : static_cast<uint32_t>(slot);
                     if (P.parts.status[idx] == 0) {
                         load<true>(st, P, idx);
-                        ++my_pushed;
                         have = true;
                         if (!live(st, P)) {
                             store<true>(st, P);
-                            my_failed += st.status != 0 ? 1 : 0;
+                            tally_finish(tally, st.steps, st.status);
                             have = false;
                         }
                     }
@@ -1475,9 +1526,7 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
         }
         if (have && !more) {
             store<true>(st, P);
-            my_steps += static_cast<unsigned long long>(st.steps);
-            my_max = max(my_max, static_cast<unsigned int>(st.steps));
-            my_failed += st.status != 0 ? 1 : 0;
+            tally_finish(tally, st.steps, st.status);
             have = false;
         }
     }
@@ -1488,15 +1537,14 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
     if (!tc_teardown<H>(net, fail) && threadIdx.x == 0) {
         atomicAdd(&P.counters->teardown_incomplete, 1u);
     }
-    flush_counters(P.counters, my_steps, my_pushed, my_failed, my_max);
-    flush_judge(P.sg.judge, tally);
+    tally_flush(tally, P.counters, P.sg.judge);
 }
 
 // One particle per thread, no refill (schedule alternative for the tuner).
 template <bool FOCUSED>
 __global__ void __launch_bounds__(128) push_simple_kernel(const PushParams P) {
-    unsigned long long my_steps = 0, my_pushed = 0, my_failed = 0;
-    unsigned int my_max = 0;
+    __shared__ BlockTally tally;
+    tally_init(tally);
     for (uint64_t slot = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
          slot < P.count; slot += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t idx =
@@ -1506,17 +1554,14 @@ __global__ void __launch_bounds__(128) push_simple_kernel(const PushParams P) {
         }
         StateMixed st;
         load<FOCUSED>(st, P, idx);
-        ++my_pushed;
         if (live(st, P)) {
             while (substep<FOCUSED>(st, P)) {
             }
         }
         store<FOCUSED>(st, P);
-        my_steps += static_cast<unsigned long long>(st.steps);
-        my_max = max(my_max, static_cast<unsigned int>(st.steps));
-        my_failed += st.status != 0 ? 1 : 0;
+        tally_finish(tally, st.steps, st.status);
     }
-    flush_counters(P.counters, my_steps, my_pushed, my_failed, my_max);
+    tally_flush(tally, P.counters, nullptr);
 }
 
 F64Consts make_f64_consts(const PushLaunch& L);
@@ -1548,6 +1593,7 @@ PushParams make_push_params(const PushLaunch& L) {
     P.records = L.precision == kPrecisionMixed ? L.records : nullptr;
     P.f64 = F64Consts{};
     P.pows = PowPlan{};
+    P.lane_cap = 32;
     if (L.precision == kPrecisionF64) {
         P.f64 = make_f64_consts(L);
         P.pows = make_pow_plan(L);
@@ -1562,6 +1608,51 @@ PushParams make_push_params(const PushLaunch& L) {
 
 namespace kpt {
 namespace {
+
+// Ask for no more of an SM's 256 KB as shared memory than `blocks` blocks use;
+// the rest caches the gathers.  Left alone the driver set 132 KB aside for the
+// 61 KB of five blocks: 50.7 -> 49.2 ms (1 Mi Parker particles), 7.38 -> 7.22
+// ms (777 777 focused), 54.6 -> 54.0 ms (4 Mi, learned closure).  The
+// occupancy queries see the share too, so it is set before them.
+template <typename Kernel>
+cudaError_t keep_l1(Kernel kernel, int blocks, size_t block_smem) {
+    int device = 0, per_sm = 0, reserved = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    err = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    if (err != cudaSuccess) return err;
+    err = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
+    if (err != cudaSuccess) return err;
+    const size_t block = (block_smem + static_cast<size_t>(reserved) + 1023) / 1024 * 1024;
+    const size_t percent = (100 * blocks * block + per_sm - 1) / per_sm;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                percent < 100 ? static_cast<int>(percent) : 100);
+}
+
+// Persistent grid: as many resident blocks per SM as the kernel's registers
+// allow (or fewer on request).
+template <bool FOCUSED, int SURR, int KIND>
+cudaError_t launch_push_kind(const PushParams& P, const PushLaunch& L, cudaStream_t stream) {
+    const int threads = 128;
+    const size_t network = SURR ? mlp_smem_bytes(surr_hidden(SURR)) : 0;
+    const size_t rows = KIND == kPushDense ? record_xpose_bytes(FOCUSED, threads / 32) : 0;
+    const size_t smem = network + (P.records != nullptr ? rows : 0);
+    const auto kernel = push_refill_kernel<FOCUSED, SURR, KIND>;
+    cudaError_t err = cudaSuccess;
+    if (KIND == kPushDense) {
+        err = keep_l1(kernel, push_blocks<FOCUSED, SURR, KIND>(),
+                      network + rows + sizeof(BlockTally));
+        if (err != cudaSuccess) return err;
+    }
+    int resident = 0;
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
+    if (err != cudaSuccess) return err;
+    resident = resident < 1 ? 1 : resident;
+    int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm : resident;
+    if (KIND == kPushFew) per_sm = kFewBlocks;  // the places lane_cap was computed for
+    kernel<<<L.sm_count * per_sm, threads, smem, stream>>>(P);
+    return cudaGetLastError();
+}
 
 // Persistent grid of the tcgen05 push: as many blocks per SM as both the
 // TMEM (TcMlp<H>::Cols of the SM's 512 columns each) and the registers
@@ -1607,34 +1698,30 @@ cudaError_t launch_push_tc(const PushParams& P, const PushLaunch& L, cudaStream_
 
 template <bool FOCUSED, int SURR = 0>
 cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
-    const PushParams P = make_push_params(L);
+    PushParams P = make_push_params(L);
     const int threads = 128;
     if constexpr (SURR != 0) {
         if (L.surrogate->engine == kEngineTcgen05) {
             return launch_push_tc<surr_fp16(SURR), surr_hidden(SURR)>(P, L, stream);
         }
     }
-    const size_t smem = (SURR ? mlp_smem_bytes(surr_hidden(SURR)) : 0) +
-                        (P.records != nullptr ? record_xpose_bytes(FOCUSED, threads / 32) : 0);
     if (L.schedule == kScheduleSimple && !SURR) {
         const uint64_t want = (L.count + threads - 1) / threads;
         const int blocks =
             static_cast<int>(want < 1 ? 1 : (want > 65535u * 8u ? 65535u * 8u : want));
         push_simple_kernel<FOCUSED><<<blocks, threads, 0, stream>>>(P);
-    } else {
-        // Persistent grid: as many resident blocks per SM as the kernel's
-        // registers allow (or fewer on request).
-        int resident = 0;
-        cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &resident, push_refill_kernel<FOCUSED, SURR>, threads, smem);
-        if (err != cudaSuccess) return err;
-        resident = resident < 1 ? 1 : resident;
-        const int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm
-                                                                            : resident;
-        push_refill_kernel<FOCUSED, SURR>
-            <<<L.sm_count * per_sm, threads, smem, stream>>>(P);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    if (P.records != nullptr || L.blocks_per_sm > kPointsBlocks) {
+        return launch_push_kind<FOCUSED, SURR, kPushDense>(P, L, stream);
+    }
+    const uint64_t few = static_cast<uint64_t>(L.sm_count) * kFewBlocks * threads;
+    if (L.count <= few && L.blocks_per_sm == 0) {
+        const uint64_t warps = few / 32;
+        P.lane_cap = static_cast<unsigned>((L.count + warps - 1) / warps);
+        return launch_push_kind<FOCUSED, SURR, kPushFew>(P, L, stream);
+    }
+    return launch_push_kind<FOCUSED, SURR, kPushPoints>(P, L, stream);
 }
 
 #if KPT_PUSH_PART == 0
@@ -1646,6 +1733,13 @@ cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
 // global memory.  Lanes of one warp may belong to different runs.  Each
 // finished particle adds its counters to its run's counters.
 constexpr int kBatchMaxRuns = 1024;
+__host__ __device__ constexpr size_t batch_offset_bytes(int runs) {
+    return (static_cast<size_t>(runs + 1) * sizeof(uint64_t) + 15) / 16 * 16;
+}
+// Without records the tables' rows are shared through L1, and three blocks of
+// 128 threads reuse them better than five: 16 Parker runs, 50 steps, 3.60 ->
+// 3.31 ms.
+constexpr int kBatchPointThreads = 3 * 128;
 
 __device__ __forceinline__ int batch_run_of(const uint64_t* offsets, int runs, uint64_t slot) {
     int lo = 0;
@@ -1714,8 +1808,10 @@ struct BatchMinBlocks {
 template <bool FOCUSED, int THREADS, int PPL>
 __global__ void __launch_bounds__(THREADS, (BatchMinBlocks<FOCUSED, THREADS, PPL>::value))
     push_batch_kernel(const BatchLaunch B) {
-    __shared__ uint64_t offsets[kBatchMaxRuns + 1];
-    extern __shared__ float batch_xpose[];
+    // the runs' offsets (runs + 1), then the warps' rows of the record sampler
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    uint64_t* offsets = reinterpret_cast<uint64_t*>(batch_smem);
+    float* batch_xpose = reinterpret_cast<float*>(batch_smem + batch_offset_bytes(B.runs));
     for (int k = threadIdx.x; k <= B.runs; k += blockDim.x) offsets[k] = B.offsets[k];
     __syncthreads();
     const PushParams* runs = static_cast<const PushParams*>(B.params);
@@ -1893,14 +1989,25 @@ namespace {
 
 template <bool FOCUSED, int THREADS, int PPL>
 cudaError_t launch_batch_shape(const BatchLaunch& B, cudaStream_t stream) {
-    const size_t smem = B.records != 0 ? record_xpose_bytes(FOCUSED, THREADS / 32) : 0;
+    const size_t smem = batch_offset_bytes(B.runs) +
+                        (B.records != 0 ? record_xpose_bytes(FOCUSED, THREADS / 32) : 0);
+    cudaError_t err =
+        B.records != 0
+            ? keep_l1(push_batch_kernel<FOCUSED, THREADS, PPL>,
+                      BatchMinBlocks<FOCUSED, THREADS, PPL>::value, smem)
+            : cudaFuncSetAttribute(push_batch_kernel<FOCUSED, THREADS, PPL>,
+                                   cudaFuncAttributePreferredSharedMemoryCarveout,
+                                   cudaSharedmemCarveoutDefault);
+    if (err != cudaSuccess) return err;
     int resident = 0;
-    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &resident, push_batch_kernel<FOCUSED, THREADS, PPL>, THREADS, smem);
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
-    const int per_sm = B.blocks_per_sm > 0 && B.blocks_per_sm < resident ? B.blocks_per_sm
-                                                                        : resident;
+    int per_sm = B.blocks_per_sm > 0 && B.blocks_per_sm < resident ? B.blocks_per_sm : resident;
+    if (B.blocks_per_sm == 0 && B.records == 0 && per_sm * THREADS > kBatchPointThreads) {
+        per_sm = kBatchPointThreads / THREADS > 0 ? kBatchPointThreads / THREADS : 1;
+    }
     push_batch_kernel<FOCUSED, THREADS, PPL><<<B.sm_count * per_sm, THREADS, smem, stream>>>(B);
     return cudaGetLastError();
 }

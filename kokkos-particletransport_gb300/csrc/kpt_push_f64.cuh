@@ -815,7 +815,7 @@ __device__ __forceinline__ bool advance_f64(StateF64& st, const PushParams& P, c
 // plain closure in FP32 too.
 template <bool FP16, int H>
 __device__ __forceinline__ Served serve_f64(const StateF64& st, const PushParams& P, bool have,
-                                            double b64, const uint2* smem, JudgeTally& tally) {
+                                            double b64, const uint2* smem, BlockTally& tally) {
     const SurrogateDevice& sg = P.sg;
     const SurrogateBox& box = sg.box;
     float f[kMlpIn] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -871,7 +871,8 @@ __global__ void __launch_bounds__(128, kF64Blocks) push_f64_kernel(const PushPar
     const unsigned lanes_below = (1u << lane) - 1u;
     extern __shared__ __align__(16) unsigned char f64_smem[];
     const uint2* network = reinterpret_cast<const uint2*>(f64_smem);
-    JudgeTally tally{0ull, 0ull, 0ull, 0.0f};
+    __shared__ BlockTally tally;
+    tally_init(tally);
     if (SURR) {
         load_surrogate_block<surr_hidden(SURR)>(P.sg.block, reinterpret_cast<uint2*>(f64_smem));
     }
@@ -887,8 +888,6 @@ __global__ void __launch_bounds__(128, kF64Blocks) push_f64_kernel(const PushPar
     StateF64 st{};
     bool have = false;
     bool exhausted = false;
-    unsigned long long my_steps = 0;
-    unsigned int my_pushed = 0, my_failed = 0, my_max = 0;
     for (;;) {
         const unsigned idle = __ballot_sync(full, !have);
         const unsigned held = 32u - __popc(idle);
@@ -915,11 +914,10 @@ __global__ void __launch_bounds__(128, kF64Blocks) push_f64_kernel(const PushPar
                                                             : static_cast<uint32_t>(slot);
                     if (P.parts.status[idx] == 0) {
                         load<FOCUSED>(st, P, idx);
-                        ++my_pushed;
                         have = true;
                         if (!live(st, P)) {
                             store<FOCUSED>(st, P);
-                            my_failed += st.status != 0 ? 1 : 0;
+                            tally_finish(tally, st.steps, st.status);
                             have = false;
                         }
                     }
@@ -951,16 +949,11 @@ __global__ void __launch_bounds__(128, kF64Blocks) push_f64_kernel(const PushPar
         }
         if (have && !more) {
             store<FOCUSED>(st, P);
-            my_steps += static_cast<unsigned long long>(st.steps);
-            my_max = max(my_max, static_cast<unsigned int>(st.steps));
-            my_failed += st.status != 0 ? 1 : 0;
+            tally_finish(tally, st.steps, st.status);
             have = false;
         }
     }
-    flush_counters(P.counters, my_steps, my_pushed, my_failed, my_max);
-    if (SURR) {
-        flush_judge(P.sg.judge, tally);
-    }
+    tally_flush(tally, P.counters, SURR ? P.sg.judge : nullptr);
 }
 
 // Reciprocals, keys and the plan of powers of one launch.
