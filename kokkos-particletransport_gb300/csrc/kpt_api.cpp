@@ -2225,6 +2225,25 @@ int validate_properties(const kpt_particle_properties* p) {
 
 }  // namespace
 
+namespace {
+
+// The integer keys of an axis' bounds (signed order of the bits; -0 sorts
+// below +0, so a zero bound takes -0's key).  Below key_inside the wrap count
+// floor((x - lower) / width) is surely 0.
+void set_axis_keys(kpt::LibAxis& a) {
+    auto key = [](double v) {
+        long long bits;
+        std::memcpy(&bits, &v, sizeof(bits));
+        return v == 0.0 ? -1ll : bits ^ ((bits >> 63) & 0x7fffffffffffffffll);
+    };
+    a.key_lower = key(a.lower);
+    a.key_upper = key(a.upper);
+    const double safe = a.lower + (1.0 - 9.094947017729282e-13) * a.width;
+    a.key_inside = safe < a.upper ? key(safe) : a.key_lower;
+}
+
+}  // namespace
+
 extern "C" {
 
 int kpt_grid_create(kpt_context* ctx, int nx, int ny, const double* x_edges,
@@ -2263,6 +2282,7 @@ int kpt_grid_create(kpt_context* ctx, int nx, int ny, const double* x_edges,
         a.ghost_upper = a.x0 + static_cast<double>(n + 2) * a.dx;
         a.width = a.upper - a.lower;
         a.inv_width = a.width != 0.0 ? 1.0 / a.width : 0.0;
+        set_axis_keys(a);
     }
     g->g.ex = nx + 4;
     *out = g.release();
@@ -2347,6 +2367,7 @@ int kpt_grid_create_stored(kpt_context* ctx, int nx, int ny, const double* x_fac
         a.ghost_upper = f[n + 4];
         a.width = a.upper - a.lower;
         a.inv_width = a.width != 0.0 ? 1.0 / a.width : 0.0;
+        set_axis_keys(a);
     }
     g->g.ex = nx + 4;
     *out = g.release();
@@ -2695,6 +2716,8 @@ int parker_launch(kpt_context* ctx, kpt_parker_solver* s, kpt_system* sys, int a
     L.charge = sys->props.charge;
     L.speed_of_light = sys->props.speed_of_light;
     L.mc = sys->props.rest_mass * sys->props.speed_of_light;
+    L.inv_mc = 1.0 / L.mc;
+    L.drift = L.speed_of_light / (3.0 * L.charge);
     L.courant = s->courant;
     L.terms = s->terms.as<double>();
     char* sc = static_cast<char*>(s->scalars.ptr);

@@ -302,6 +302,9 @@ struct LibAxis {
     int stored;
     const double* faces;
     const double* cells;
+    // integer keys (f64_key) of the bounds; a coordinate in [key_lower,
+    // key_inside) of a periodic axis is its own wrap
+    long long key_lower, key_upper, key_inside;
 };
 struct LibGrid {
     LibAxis axis[2];
@@ -331,6 +334,7 @@ struct LibParkerLaunch {
     SystemArrays sys;
     uint64_t count, capacity;
     double rest_mass, charge, speed_of_light, mc;
+    double inv_mc, drift;     // 1 / mc, speed_of_light / (3 charge)
     double courant;
     double* terms;                  // count x kLibTermCount
     unsigned long long* min_bits;   // global minimum of the local dt bounds
