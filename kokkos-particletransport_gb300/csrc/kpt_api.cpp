@@ -2018,7 +2018,12 @@ int kpt_host_alloc(uint64_t bytes, void** out) {
     KPT_REQUIRE(out != nullptr, "kpt_host_alloc: NULL argument");
     *out = nullptr;
     if (bytes == 0) return KPT_OK;
-    KPT_CUDA(cudaHostAlloc(out, bytes, cudaHostAllocPortable));
+    const cudaError_t err = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+    if (err != cudaSuccess) {
+        cudaGetLastError();  // the caller may go on without page-locked memory
+        *out = nullptr;
+        KPT_CUDA(err);
+    }
     return KPT_OK;
 }
 
