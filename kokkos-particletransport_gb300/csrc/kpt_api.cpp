@@ -2185,7 +2185,8 @@ struct kpt_parker_solver {
     DeviceBuffer basis_f32;        // the mixed step's FP32 copy of the basis
     bool basis_f32_valid = false;  // cleared whenever the FP64 basis changes
     DeviceBuffer terms;
-    // min bits (u64), dt (f64), error (i32 + pad), error index (u64)
+    // min bits (u64), dt (f64), error (i32 + pad), error index (u64), arrivals
+    // (u32): 64 bytes, cleared before a step or a sequence of steps
     DeviceBuffer scalars;
     DeviceBuffer dt_history;
 };
@@ -2245,7 +2246,13 @@ void set_axis_keys(kpt::LibAxis& a) {
     a.key_upper = key(a.upper);
     const double safe = a.lower + (1.0 - 9.094947017729282e-13) * a.width;
     a.key_inside = safe < a.upper ? key(safe) : a.key_lower;
+    a.inv_dx32 = static_cast<float>(a.inv_dx);
+    a.dx32 = static_cast<float>(a.dx);
 }
+
+// Values from one row of per-particle terms to the next: rows start on whole
+// lines in either precision.
+uint64_t term_stride(uint64_t count) { return (std::max<uint64_t>(count, 1) + 31) / 32 * 32; }
 
 }  // namespace
 
@@ -2696,8 +2703,8 @@ int parker_validate(const kpt_parker_solver* s, const kpt_system* sys) {
 int parker_launch(kpt_context* ctx, kpt_parker_solver* s, kpt_system* sys, int advance,
                   int stochastic, uint64_t seed, uint32_t step, double* dt_history,
                   kpt::LibParkerLaunch* out) {
-    KPT_CUDA(s->terms.reserve(std::max<uint64_t>(sys->count, 1) * kpt::kLibTermCount *
-                              sizeof(double)));
+    const uint64_t stride = term_stride(sys->count);
+    KPT_CUDA(s->terms.reserve(stride * kpt::kLibTermCount * sizeof(double)));
     kpt::LibParkerLaunch& L = *out;
     L = kpt::LibParkerLaunch{};
     L.grid = s->grid;
@@ -2723,13 +2730,19 @@ int parker_launch(kpt_context* ctx, kpt_parker_solver* s, kpt_system* sys, int a
     L.mc = sys->props.rest_mass * sys->props.speed_of_light;
     L.inv_mc = 1.0 / L.mc;
     L.drift = L.speed_of_light / (3.0 * L.charge);
+    L.mc32 = static_cast<float>(L.mc);
+    L.rest_mass32 = static_cast<float>(L.rest_mass);
+    L.speed_of_light32 = static_cast<float>(L.speed_of_light);
+    L.charge32 = static_cast<float>(L.charge);
     L.courant = s->courant;
     L.terms = s->terms.as<double>();
+    L.term_stride = stride;
     char* sc = static_cast<char*>(s->scalars.ptr);
     L.min_bits = reinterpret_cast<unsigned long long*>(sc);
     L.dt_device_out = reinterpret_cast<double*>(sc + 8);
     L.error = reinterpret_cast<int*>(sc + 16);
     L.error_index = reinterpret_cast<unsigned long long*>(sc + 24);
+    L.arrivals = reinterpret_cast<unsigned int*>(sc + 32);
     L.dt_history = dt_history;
     L.apply_boundary = advance;
     L.advance = advance;
@@ -2785,7 +2798,7 @@ int parker_step(kpt_context* ctx, kpt_parker_solver* s, kpt_system* sys, int adv
     }
     ScopedBuffer noise;
     if (int rc = upload_noise(ctx, normals, sys->count, noise, &L.noise)) return rc;
-    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 32, ctx->stream));
+    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 64, ctx->stream));
     KPT_CUDA(kpt::lib_parker_step(L, ctx->stream));
     return step_finish(ctx, s->scalars.ptr, dt_out, stochastic != 0, false);
 }
@@ -2821,7 +2834,7 @@ int kpt_parker_advance_stochastic_steps(kpt_context* ctx, kpt_parker_solver* s,
     if (int rc = parker_validate(s, sys)) return rc;
     if (int rc = activate(ctx)) return rc;
     KPT_CUDA(s->dt_history.reserve(static_cast<size_t>(steps) * sizeof(double)));
-    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 32, ctx->stream));
+    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 64, ctx->stream));
     std::vector<kpt::LibParkerLaunch> launches(steps);
     for (uint32_t k = 0; k < steps; ++k) {
         if (int rc = parker_launch(ctx, s, sys, 1, 1, seed, first_step + k,
@@ -2890,8 +2903,8 @@ int focus_validate(const kpt_focus_solver* s, const kpt_system* sys) {
 
 int focus_launch(kpt_focus_solver* s, kpt_system* sys, int advance, int stochastic,
                  uint64_t seed, uint32_t step, double* dt_history, kpt::LibFocusLaunch* out) {
-    KPT_CUDA(s->terms.reserve(std::max<uint64_t>(sys->count, 1) * kpt::kFocusTermCount *
-                              sizeof(double)));
+    const uint64_t stride = term_stride(sys->count);
+    KPT_CUDA(s->terms.reserve(stride * kpt::kFocusTermCount * sizeof(double)));
     kpt::LibFocusLaunch& L = *out;
     L = kpt::LibFocusLaunch{};
     L.grid = s->grid;
@@ -2912,30 +2925,39 @@ int focus_launch(kpt_focus_solver* s, kpt_system* sys, int advance, int stochast
     L.sys = sys->a;
     L.count = sys->count;
     L.capacity = sys->capacity;
-    L.rest_mass = sys->props.rest_mass;
-    L.charge = sys->props.charge;
-    L.abs_charge = std::fabs(sys->props.charge);
-    L.speed_of_light = sys->props.speed_of_light;
-    L.mc = sys->props.rest_mass * sys->props.speed_of_light;
+    kpt::LibFocusConsts<double>& C = L.c64;
+    C.rest_mass = sys->props.rest_mass;
+    C.charge = sys->props.charge;
+    C.abs_charge = std::fabs(sys->props.charge);
+    C.speed_of_light = sys->props.speed_of_light;
+    C.mc = sys->props.rest_mass * sys->props.speed_of_light;
     const kpt_scattering_parameters& sc = s->scattering;
-    L.gk = sc.spectral_index;
-    L.h0 = sc.h0;
+    C.gk = sc.spectral_index;
+    C.h0 = sc.h0;
     // pitch_angle_spectrum_normalization (LegencyModel.hpp:539-552)
-    L.qlt_norm = sc.spectral_index * std::sin(3.141592653589793238462643383279502884 /
+    C.qlt_norm = sc.spectral_index * std::sin(3.141592653589793238462643383279502884 /
                                               sc.spectral_index) /
                  3.141592653589793238462643383279502884;
-    L.min_b = sc.minimum_magnetic_field_magnitude;
-    L.min_sigma2 = sc.minimum_sigma2;
-    L.min_lc = sc.minimum_correlation_length;
-    L.min_speed = sc.minimum_speed;
-    L.max_mu = s->max_mu;
+    C.min_b = sc.minimum_magnetic_field_magnitude;
+    C.min_sigma2 = sc.minimum_sigma2;
+    C.min_lc = sc.minimum_correlation_length;
+    C.min_speed = sc.minimum_speed;
+    C.max_mu = s->max_mu;
+    L.c32 = {static_cast<float>(C.rest_mass), static_cast<float>(C.charge),
+             static_cast<float>(C.abs_charge), static_cast<float>(C.speed_of_light),
+             static_cast<float>(C.mc), static_cast<float>(C.gk), static_cast<float>(C.h0),
+             static_cast<float>(C.qlt_norm), static_cast<float>(C.min_b),
+             static_cast<float>(C.min_sigma2), static_cast<float>(C.min_lc),
+             static_cast<float>(C.min_speed), static_cast<float>(C.max_mu)};
     L.courant = s->courant;
     L.terms = s->terms.as<double>();
+    L.term_stride = stride;
     char* scp = static_cast<char*>(s->scalars.ptr);
     L.min_bits = reinterpret_cast<unsigned long long*>(scp);
     L.dt_device_out = reinterpret_cast<double*>(scp + 8);
     L.error = reinterpret_cast<int*>(scp + 16);
     L.error_index = reinterpret_cast<unsigned long long*>(scp + 24);
+    L.arrivals = reinterpret_cast<unsigned int*>(scp + 32);
     L.dt_history = dt_history;
     L.apply_boundary = advance;
     L.advance = advance;
@@ -2956,7 +2978,7 @@ int focus_step(kpt_context* ctx, kpt_focus_solver* s, kpt_system* sys, int advan
     if (int rc = focus_launch(s, sys, advance, stochastic, seed, step, nullptr, &L)) return rc;
     ScopedBuffer noise;
     if (int rc = upload_noise(ctx, normals, sys->count, noise, &L.noise)) return rc;
-    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 32, ctx->stream));
+    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 64, ctx->stream));
     KPT_CUDA(kpt::lib_focus_step(L, ctx->stream));
     return step_finish(ctx, s->scalars.ptr, dt_out, stochastic != 0, true);
 }
@@ -3090,7 +3112,7 @@ int kpt_focus_advance_stochastic_steps(kpt_context* ctx, kpt_focus_solver* s, kp
     if (int rc = focus_validate(s, sys)) return rc;
     if (int rc = activate(ctx)) return rc;
     KPT_CUDA(s->dt_history.reserve(static_cast<size_t>(steps) * sizeof(double)));
-    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 32, ctx->stream));
+    KPT_CUDA(cudaMemsetAsync(s->scalars.ptr, 0, 64, ctx->stream));
     std::vector<kpt::LibFocusLaunch> launches(steps);
     for (uint32_t k = 0; k < steps; ++k) {
         if (int rc = focus_launch(s, sys, 1, 1, seed, first_step + k,

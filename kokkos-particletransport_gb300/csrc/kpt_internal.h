@@ -305,6 +305,7 @@ struct LibAxis {
     // integer keys (f64_key) of the bounds; a coordinate in [key_lower,
     // key_inside) of a periodic axis is its own wrap
     long long key_lower, key_upper, key_inside;
+    float inv_dx32, dx32;  // rounded, for the mixed step
 };
 struct LibGrid {
     LibAxis axis[2];
@@ -335,9 +336,12 @@ struct LibParkerLaunch {
     uint64_t count, capacity;
     double rest_mass, charge, speed_of_light, mc;
     double inv_mc, drift;     // 1 / mc, speed_of_light / (3 charge)
+    float mc32, rest_mass32, speed_of_light32, charge32;  // rounded, for the mixed step
     double courant;
-    double* terms;                  // count x kLibTermCount
-    unsigned long long* min_bits;   // global minimum of the local dt bounds
+    double* terms;                  // kLibTermCount rows of term_stride values
+    uint64_t term_stride;
+    unsigned long long* min_bits;   // global minimum of the local dt bounds (0: none yet)
+    unsigned int* arrivals;         // terms blocks done (0 between steps)
     double* dt_device_out;          // courant * min (device)
     double* dt_history;             // optional per-step record (device)
     const double* dt_device;        // advance: dt read from the device
@@ -366,6 +370,14 @@ constexpr int kFocusBasisStride = 28;
 constexpr int kFocusBasisStrideF32 = 28;  // FP32 copy: rows of seven 16-byte chunks
 constexpr int kFocusTermCount = 18;
 
+// The step's constants in its arithmetic's type (a conversion in the kernel
+// is one more FP64-pipe instruction).
+template <typename T>
+struct LibFocusConsts {
+    T rest_mass, charge, abs_charge, speed_of_light, mc;
+    T gk, h0, qlt_norm, min_b, min_sigma2, min_lc, min_speed, max_mu;
+};
+
 struct LibFocusLaunch {
     LibGrid grid;
     const double* basis;      // ghosted points x kFocusBasisStride
@@ -374,11 +386,13 @@ struct LibFocusLaunch {
     int constant_ratio;
     SystemArrays sys;
     uint64_t count, capacity;
-    double rest_mass, charge, abs_charge, speed_of_light, mc;
-    double gk, h0, qlt_norm, min_b, min_sigma2, min_lc, min_speed, max_mu;
+    LibFocusConsts<double> c64;
+    LibFocusConsts<float> c32;  // c64 rounded
     double courant;
-    double* terms;  // count x kFocusTermCount
+    double* terms;  // kFocusTermCount rows of term_stride values
+    uint64_t term_stride;
     unsigned long long* min_bits;
+    unsigned int* arrivals;
     double* dt_device_out;
     double* dt_history;
     const double* dt_device;

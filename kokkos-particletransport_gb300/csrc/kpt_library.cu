@@ -10,8 +10,8 @@
 // samples the packed coefficient basis once per particle, keeps the terms the
 // update needs (coordinate rates, momentum rate, kappa_par, kappa_perp, the
 // field direction, |p|) and folds the local stable time step into a global
-// minimum (an atomic min on the bit pattern of a positive double, exact and
-// order independent).  The second rotates the previous positions, draws the
+// minimum (an atomic on the bit pattern of a positive double, exact and order
+// independent), from which its last block forms the step's dt.  The second rotates the previous positions, draws the
 // noise, updates every active particle from the kept terms and applies the
 // boundary conditions again.  The reference evaluates the same terms twice
 // (once for dt, once for the update) from the same positions; keeping them
@@ -158,7 +158,7 @@ __device__ __forceinline__ void lib_stencil_mixed(const LibAxis& a, double x, in
         return;
     }
     const float logical =
-        fmaf(static_cast<float>(x - a.x0), static_cast<float>(a.inv_dx), -0.5f);
+        fmaf(static_cast<float>(x - a.x0), a.inv_dx32, -0.5f);
     const int lower_bound = -2;
     const int upper_bound = a.n + 1;
     if (logical <= static_cast<float>(lower_bound)) {
@@ -283,6 +283,10 @@ struct LibMath<double> {
     static __device__ __forceinline__ double cbrt(double v) { return ::cbrt(v); }
     static __device__ __forceinline__ double pow(double a, double b) { return ::pow(a, b); }
     static __device__ __forceinline__ double abs(double v) { return fabs(v); }
+    static __device__ __forceinline__ double product(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double fused(double a, double b, double c) {
+        return fma(a, b, c);
+    }
 };
 template <>
 struct LibMath<float> {
@@ -290,6 +294,10 @@ struct LibMath<float> {
     static __device__ __forceinline__ float cbrt(float v) { return cbrtf(v); }
     static __device__ __forceinline__ float pow(float a, float b) { return powf(a, b); }
     static __device__ __forceinline__ float abs(float v) { return fabsf(v); }
+    static __device__ __forceinline__ float product(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float fused(float a, float b, float c) {
+        return fmaf(a, b, c);
+    }
 };
 
 // The momentum scalings gamma^(1/3) and gamma^(1/9) of the diffusion
@@ -341,12 +349,20 @@ __device__ __forceinline__ bool lib_boundary(const LibGrid& g, const SystemArray
     return !escaped;
 }
 
+// A coordinate that lies inside the axis and is its own wrap (integer
+// compares only).
+__device__ __forceinline__ bool lib_inside(const LibAxis& a, double x) {
+    const long long key = f64_key(f64_bits(x));
+    return key >= a.key_lower && key < a.key_inside;
+}
+
 // The mixed step's boundary pass: a coordinate already inside [lower, upper)
 // of a periodic axis is its own wrap, so only coordinates outside take the
-// reference's floor formula (two FP64 compares for most particles instead of
+// reference's floor formula (integer compares for most particles instead of
 // the full wrap; GB300's FP64 pipe is the scarce one).
 __device__ __forceinline__ bool lib_boundary_mixed(const LibGrid& g, const SystemArrays& s,
                                                    size_t i) {
+    if (lib_inside(g.axis[0], s.x[i]) && lib_inside(g.axis[1], s.y[i])) return true;
     bool escaped = false;
 #pragma unroll
     for (int dim = 0; dim < 2; ++dim) {
@@ -374,13 +390,6 @@ __device__ __forceinline__ bool lib_boundary_mixed(const LibGrid& g, const Syste
     return !escaped;
 }
 
-// A coordinate that lies inside the axis and is its own wrap (integer
-// compares only).
-__device__ __forceinline__ bool lib_inside(const LibAxis& a, double x) {
-    const long long key = f64_key(f64_bits(x));
-    return key >= a.key_lower && key < a.key_inside;
-}
-
 // lib_boundary for the FP64 step: a particle inside both axes keeps its
 // positions and their histories (its shift is 0).
 __device__ __forceinline__ bool lib_boundary_f64(const LibGrid& g, const SystemArrays& s,
@@ -399,7 +408,9 @@ __device__ __forceinline__ bool lib_boundary_t(const LibGrid& g, const SystemArr
     }
 }
 
-// Kept per-particle terms (one row per particle, kLibTermCount doubles).
+// Kept per-particle terms: kLibTermCount rows of one value per particle, so
+// that a warp's stores and loads are whole lines (a row per particle spread
+// each of them over 32 sectors).
 enum TermSlot {
     kRateX = 0, kRateY, kMomentumRate, kKappaPar, kKappaPerp, kDirX, kDirY, kDirZ, kMomentum
 };
@@ -421,9 +432,8 @@ __device__ float lib_parker_terms_mixed(const LibParkerLaunch& L, size_t i, floa
 #pragma unroll
     for (int dim = 0; dim < 2; ++dim) {
         const LibAxis& a = g.axis[dim];
-        if (!(pos[dim] >= a.lower && pos[dim] < a.upper)) {
-            pos[dim] = lib_wrap(a, pos[dim]);
-        }
+        if (lib_inside(a, pos[dim])) continue;
+        pos[dim] = lib_wrap(a, pos[dim]);
         if (!lib_contains(a.lower, a.upper, pos[dim])) {
             // the reference's empty terms: zero rates, zero time step
             for (int k = 0; k < kLibTermCount; ++k) terms[k] = T(0);
@@ -436,9 +446,9 @@ __device__ float lib_parker_terms_mixed(const LibParkerLaunch& L, size_t i, floa
 
     const T p_in = static_cast<T>(s.p[i]);
     const T p = p_in >= T(0) ? p_in : -p_in;
-    const T normalized = p / static_cast<T>(L.mc);
+    const T normalized = p / L.mc32;
     const T gamma = M::sqrt(T(1) + normalized * normalized);
-    const T speed = p / (gamma * static_cast<T>(L.rest_mass));
+    const T speed = p / (gamma * L.rest_mass32);
     T b2 = T(0);
 #pragma unroll
     for (int c = 0; c < 3; ++c) b2 += v[c] * v[c];
@@ -475,8 +485,7 @@ __device__ float lib_parker_terms_mixed(const LibParkerLaunch& L, size_t i, floa
         }
     }
     const T divv = v[17];
-    const T prefactor = p * speed * static_cast<T>(L.speed_of_light) /
-                        (T(3) * static_cast<T>(L.charge));
+    const T prefactor = p * speed * L.speed_of_light32 / (T(3) * L.charge32);
     T total[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) total[c] = v[3 + c] + prefactor * v[6 + c] + diff[c];
@@ -500,7 +509,7 @@ __device__ float lib_parker_terms_mixed(const LibParkerLaunch& L, size_t i, floa
         const LibAxis& a = g.axis[dim];
         T dx;
         if (!a.stored) {
-            dx = static_cast<T>(a.dx);
+            dx = a.dx32;
         } else {
             const double x = pos[dim];
             if (!lib_contains(a.lower, a.upper, x)) {
@@ -659,12 +668,16 @@ __device__ double lib_parker_terms_f64(const LibParkerLaunch& L, size_t i, doubl
     return dt < kLargeTimeStep ? dt : kLargeTimeStep;
 }
 
-// The block's minimum of the local dt bounds to the global minimum: one
-// atomic per block on the bit pattern of a positive double (exact and order
-// independent); an FP32 bound of +inf (no limiter) is the reference's large
-// step.
-template <typename T>
-__device__ __forceinline__ void block_min_to_global(T local, unsigned long long* min_bits) {
+// The end of a terms kernel: the block's minimum of the local dt bounds joins
+// the global one (an atomic on bit patterns, exact and order independent), and
+// the last block to arrive turns it into the step's dt = courant x minimum (0
+// when no particle bounded it; the host reports that as an error), clears the
+// minimum and the arrival count for the next step, and notes the step.  The
+// word holds bits(large) - bits(minimum), so that cleared memory means "no
+// bound".  A step is two launches this way; a kernel before and one between
+// for the same two words took a third of a small system's step.
+template <typename T, typename Launch>
+__device__ __forceinline__ void finish_terms(T local, const Launch& L) {
     for (int off = 16; off > 0; off >>= 1) {
         const T o = __shfl_down_sync(0xffffffffu, local, off);
         local = o < local ? o : local;
@@ -672,12 +685,28 @@ __device__ __forceinline__ void block_min_to_global(T local, unsigned long long*
     __shared__ T warp_min[8];
     if ((threadIdx.x & 31u) == 0u) warp_min[threadIdx.x >> 5] = local;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        T m = warp_min[0];
-        for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) m = warp_min[k] < m ? warp_min[k] : m;
-        const double md = isinf(m) ? kLargeTimeStep : static_cast<double>(m);
-        // positive doubles order like their bit patterns
-        atomicMin(min_bits, static_cast<unsigned long long>(__double_as_longlong(md)));
+    if (threadIdx.x != 0) return;
+    T m = warp_min[0];
+    for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) m = warp_min[k] < m ? warp_min[k] : m;
+    const unsigned long long large =
+        static_cast<unsigned long long>(__double_as_longlong(kLargeTimeStep));
+    // an FP32 bound of +inf (no limiter) is the reference's large step
+    const double md = isinf(m) ? kLargeTimeStep : static_cast<double>(m);
+    const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(md));
+    if (bits < large) atomicMax(L.min_bits, large - bits);
+    __threadfence();
+    if (atomicAdd(L.arrivals, 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    const double least = __longlong_as_double(
+        static_cast<long long>(large - atomicExch(L.min_bits, 0ull)));
+    *L.arrivals = 0u;
+    const double dt = (!isfinite(least) || least >= 0.5 * kLargeTimeStep) ? 0.0
+                                                                          : L.courant * least;
+    const int error = *static_cast<volatile int*>(L.error);
+    *L.dt_device_out = dt;
+    if (L.dt_history != nullptr) *L.dt_history = error != 0 ? 0.0 : dt;
+    if (L.advance && !(isfinite(dt) && dt > 0.0) && error == 0) {
+        *L.error = 6;  // "adaptive time step is not positive and finite"
     }
 }
 
@@ -703,19 +732,22 @@ __global__ void __launch_bounds__(256) lib_parker_terms_kernel(const LibParkerLa
             continue;
         }
         T dt;
+        T row[kLibTermCount];
         if constexpr (sizeof(T) == 8) {
-            dt = lib_parker_terms_f64(L, i, terms + i * kLibTermCount);
+            dt = lib_parker_terms_f64(L, i, row);
         } else {
-            dt = lib_parker_terms_mixed(L, i, terms + i * kLibTermCount);
+            dt = lib_parker_terms_mixed(L, i, row);
         }
         if (dt < T(0)) {
             record_error(L.error, static_cast<int>(-dt), static_cast<uint32_t>(i),
                          L.error_index);
             continue;
         }
+#pragma unroll
+        for (int k = 0; k < kLibTermCount; ++k) terms[k * L.term_stride + i] = row[k];
         local = dt < local ? dt : local;
     }
-    block_min_to_global(local, L.min_bits);
+    finish_terms(local, L);
 }
 
 // Box-Muller pair from two stream draws (u1 = 1 - draw, u2 = draw): normals
@@ -792,7 +824,7 @@ __global__ void __launch_bounds__(256) lib_parker_advance_kernel(const LibParker
     const double dt = L.dt_device != nullptr ? *L.dt_device : L.dt;
     // a failed step (no positive dt, or an abort condition) changes nothing
     // beyond the boundary pass, as the reference throws before its update
-    if (!(isfinite(dt) && dt > 0.0) || *L.error != 0) {
+    if (!(f64_finite(dt) && f64_positive(dt)) || *L.error != 0) {
         return;
     }
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
@@ -807,7 +839,11 @@ __global__ void __launch_bounds__(256) lib_parker_advance_kernel(const LibParker
         if (i >= L.count || s.status[i] != 0) {
             continue;
         }
-        const T* t = reinterpret_cast<const T*>(L.terms) + i * kLibTermCount;
+        T t[kLibTermCount];
+#pragma unroll
+        for (int k = 0; k < kLibTermCount; ++k) {
+            t[k] = reinterpret_cast<const T*>(L.terms)[k * L.term_stride + i];
+        }
         if constexpr (sizeof(T) == 8) {
             double inc[2] = {0.0, 0.0};
             if (L.stochastic) {
@@ -863,39 +899,33 @@ __global__ void __launch_bounds__(256) lib_parker_advance_kernel(const LibParker
             s.x[i] += static_cast<double>(inc[0]);
             s.y[i] += static_cast<double>(inc[1]);
             // the momentum base is the FP64 state, as the terms pass read it
-            const double base = s.p[i] >= 0.0 ? s.p[i] : -s.p[i];
-            const double updated = base + static_cast<double>(tdt * t[kMomentumRate]);
-            s.p[i] = updated > 0.0 ? updated : 0.0;
+            const double updated = fabs(s.p[i]) + static_cast<double>(tdt * t[kMomentumRate]);
+            s.p[i] = f64_positive(updated) && !f64_nan(updated) ? updated : 0.0;
         }
         lib_boundary_t<T>(L.grid, s, i);
     }
 }
 
-// dt = courant * min over the active particles, on the device (0 when no
-// particle bounded it; the host reports that as an error).
-__global__ void lib_finish_dt_kernel(const unsigned long long* min_bits, double courant,
-                                     double* dt_out, double* dt_history, int* error,
-                                     int require_positive) {
-    const double m = __longlong_as_double(static_cast<long long>(*min_bits));
-    const double dt = (!isfinite(m) || m >= 0.5 * kLargeTimeStep) ? 0.0 : courant * m;
-    *dt_out = dt;
-    if (dt_history != nullptr) *dt_history = *error != 0 ? 0.0 : dt;
-    if (require_positive && !(isfinite(dt) && dt > 0.0) && *error == 0) {
-        *error = 6;  // "adaptive time step is not positive and finite"
-    }
-}
-
-__global__ void lib_reset_min_kernel(unsigned long long* min_bits) {
-    *min_bits = static_cast<unsigned long long>(__double_as_longlong(kLargeTimeStep));
-}
-
 // ---- FocusTransportSolver ----------------------------------------------------
 
+// Kept per-particle terms, a row each (as the Parker step's): the update's
+// rates, the parts of the pitch-angle rates that do not depend on the cosine
+// (PitchSetup) and the rates at the step's own cosine, which the time-step
+// bound needs and which the first Picard iteration then reuses.
 enum FocusSlot {
-    fRateX = 0, fRateY, fMomentumRate, fKappaPerp, fDirX, fDirY, fDirZ, fMomentum, fMu, fSpeed,
-    fGamma, fBmag, fDivV, fBBGradV, fConvective, fFocusing, fSigma2, fLc
+    fRateX = 0, fRateY, fMomentumRate, fKappaPerp, fDirX, fDirY, fDirZ, fMomentum, fMu, fDivV,
+    fBBGradV, fFocusing0, fConvective, fXi, fXiGk, fPref, fPitchD, fPitchRate
 };
-static_assert(fLc + 1 <= kFocusTermCount, "focus term row layout");
+static_assert(fPitchRate + 1 == kFocusTermCount, "focus term row layout");
+
+template <typename T>
+__device__ __forceinline__ const LibFocusConsts<T>& focus_consts(const LibFocusLaunch& L) {
+    if constexpr (sizeof(T) == 4) {
+        return L.c32;
+    } else {
+        return L.c64;
+    }
+}
 
 // The first failure of a particle's step is the one reported, as the
 // reference throws at its first failed check.
@@ -927,7 +957,7 @@ __device__ __forceinline__ T positive_floor(T v, T floor_value) {
 
 template <typename T>
 struct PitchRates {
-    T focusing, D, dD, rate;
+    T D, rate;
 };
 
 // The parts of evaluate_pitch_angle_at_mu (FocusSolver.hpp:664-695) and of
@@ -940,65 +970,65 @@ struct PitchRates {
 // |mu|+h0 (equal to within two ulp).
 template <typename T>
 struct PitchSetup {
-    T speed, focusing0, convective, omega, xi, xi_gk, pref;
-    int error;  // 12, 13 or 14: the input check that fails, in the reference's order
+    T focusing0, convective, xi, xi_gk, pref, divv, bbgradv;
 };
 
+// Returns 0, or 12, 13 or 14: the input check that fails, in the reference's
+// order.  v: the sampled basis.
 template <typename T>
-__device__ PitchSetup<T> focus_pitch_setup(const LibFocusLaunch& L, const T* t) {
-    PitchSetup<T> q{};
-    q.speed = static_cast<T>(t[fSpeed]);
-    if (q.speed <= T(0)) {
-        q.error = 12;  // "pitch-angle stepping requires positive particle speed"
-        return q;
+__device__ int focus_pitch_setup(const LibFocusConsts<T>& C, const T* v, T speed, T gamma,
+                                 PitchSetup<T>& q) {
+    if (speed <= T(0)) {
+        return 12;  // "pitch-angle stepping requires positive particle speed"
     }
-    q.focusing0 = -q.speed * static_cast<T>(t[fFocusing]);
-    q.convective = T(2) * static_cast<T>(t[fConvective]) / q.speed;
-    const T safe_b = positive_floor(static_cast<T>(t[fBmag]), static_cast<T>(L.min_b));
-    const T safe_sigma2 = positive_floor(static_cast<T>(t[fSigma2]), static_cast<T>(L.min_sigma2));
-    const T safe_lc = positive_floor(static_cast<T>(t[fLc]), static_cast<T>(L.min_lc));
-    const T safe_speed = positive_floor(q.speed, static_cast<T>(L.min_speed));
+    q.focusing0 = -speed * v[22];
+    q.convective = T(2) * v[24] / speed;
+    q.divv = v[21];
+    q.bbgradv = v[23];
+    const T safe_b = positive_floor(v[18], C.min_b);
+    const T safe_sigma2 = positive_floor(v[25], C.min_sigma2);
+    const T safe_lc = positive_floor(v[26], C.min_lc);
+    const T safe_speed = positive_floor(speed, C.min_speed);
     if (safe_b <= T(0) || safe_sigma2 <= T(0) || safe_lc <= T(0) || safe_speed <= T(0)) {
-        q.error = 13;  // "pitch-angle scattering requires positive local inputs"
-        return q;
+        return 13;  // "pitch-angle scattering requires positive local inputs"
     }
-    q.omega = static_cast<T>(L.abs_charge) * safe_b /
-              (static_cast<T>(L.rest_mass) * static_cast<T>(L.speed_of_light)) /
-              static_cast<T>(t[fGamma]);
-    if (q.omega <= T(0)) {
-        q.error = 14;  // "D_mumu requires positive omega, speed, sigma2, and Lc"
-        return q;
+    const T omega = C.abs_charge * safe_b / (C.rest_mass * C.speed_of_light) / gamma;
+    if (omega <= T(0)) {
+        return 14;  // "D_mumu requires positive omega, speed, sigma2, and Lc"
     }
-    q.xi = q.omega * safe_lc / safe_speed;
-    q.xi_gk = LibMath<T>::pow(q.xi, static_cast<T>(L.gk));
-    q.pref = static_cast<T>(0.25 * 3.141592653589793238462643383279502884) * q.omega *
-             safe_sigma2 * static_cast<T>(L.qlt_norm);
-    return q;
+    q.xi = omega * safe_lc / safe_speed;
+    q.xi_gk = LibMath<T>::pow(q.xi, C.gk);
+    q.pref = static_cast<T>(0.25 * 3.141592653589793238462643383279502884) * omega *
+             safe_sigma2 * C.qlt_norm;
+    return 0;
 }
 
 // evaluate_pitch_angle_at_mu with the slab-QLT evaluate_pitch_angle_scattering
-// (LegencyModel.hpp:539-693) at one trial cosine.
+// (LegencyModel.hpp:539-693) at one trial cosine.  Which products round on
+// their own is written out: the pitch angle amplifies a last bit within a few
+// steps, and the terms and the update have to agree on the rates they share.
 template <typename T>
-__device__ PitchRates<T> focus_pitch(const LibFocusLaunch& L, const T* t,
-                                     const PitchSetup<T>& q, T trial, int* error) {
-    PitchRates<T> r{T(0), T(0), T(0), T(0)};
-    const T mu = focus_reflect(trial, static_cast<T>(L.max_mu), error);
-    if (q.error != 0) {
-        set_error(error, q.error);
+__device__ PitchRates<T> focus_pitch(const LibFocusConsts<T>& C, const PitchSetup<T>& q,
+                                     int setup_error, T trial, int* error) {
+    using M = LibMath<T>;
+    PitchRates<T> r{T(0), T(0)};
+    const T mu = focus_reflect(trial, C.max_mu, error);
+    if (setup_error != 0) {
+        set_error(error, setup_error);
         return r;
     }
-    const T mu2 = mu * mu;
-    const T one_minus_mu2 = T(1) - mu2;
-    r.focusing = T(0.5) * one_minus_mu2 *
-                 (q.focusing0 + mu * static_cast<T>(t[fDivV]) -
-                  T(3) * mu * static_cast<T>(t[fBBGradV]) - q.convective);
+    const T one_minus_mu2 = M::fused(-mu, mu, T(1));
+    const T focusing =
+        M::product(T(0.5) * one_minus_mu2,
+                   M::fused(-(T(3) * mu), q.bbgradv, M::fused(mu, q.divv, q.focusing0)) -
+                       q.convective);
     T d = T(0);
     T dd = T(0);
     if (one_minus_mu2 > T(0)) {
-        const T reg = (mu >= T(0) ? mu : -mu) + static_cast<T>(L.h0);
-        const T gk = static_cast<T>(L.gk);
-        const T reg_gk1 = LibMath<T>::pow(reg, gk - T(1));
-        const T reg_gk = reg > T(0) ? reg_gk1 * reg : LibMath<T>::pow(reg, gk);
+        const T reg = (mu >= T(0) ? mu : -mu) + C.h0;
+        const T gk = C.gk;
+        const T reg_gk1 = M::pow(reg, gk - T(1));
+        const T reg_gk = reg > T(0) ? M::product(reg_gk1, reg) : M::pow(reg, gk);
         const T den = reg_gk + q.xi_gk;
         if (den <= T(0)) {
             set_error(error, 15);  // "D_mumu denominator must be positive"
@@ -1009,12 +1039,11 @@ __device__ PitchRates<T> focus_pitch(const LibFocusLaunch& L, const T* t,
         const T sign = mu > T(0) ? T(1) : (mu < T(0) ? T(-1) : T(0));
         if (d != T(0) && sign != T(0)) {
             const T shape = sign * ((gk - T(1)) / reg - gk * reg_gk1 / den);
-            dd = d * (T(-2) * mu / one_minus_mu2 + shape);
+            dd = M::product(d, T(-2) * mu / one_minus_mu2 + shape);
         }
     }
     r.D = d;
-    r.dD = dd;
-    r.rate = r.focusing + dd;
+    r.rate = focusing + dd;
     return r;
 }
 
@@ -1026,15 +1055,15 @@ template <typename T>
 __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
     using M = LibMath<T>;
     constexpr bool kMixed = sizeof(T) == 4;
+    const LibFocusConsts<T>& C = focus_consts<T>(L);
     const LibGrid& g = L.grid;
     const SystemArrays& s = L.sys;
     double pos[2] = {s.x[i], s.y[i]};
 #pragma unroll
     for (int dim = 0; dim < 2; ++dim) {
         const LibAxis& a = g.axis[dim];
-        if (!kMixed || !(pos[dim] >= a.lower && pos[dim] < a.upper)) {
-            pos[dim] = lib_wrap(a, pos[dim]);
-        }
+        if (lib_inside(a, pos[dim])) continue;
+        pos[dim] = lib_wrap(a, pos[dim]);
         if (!lib_contains(a.lower, a.upper, pos[dim])) {
             for (int k = 0; k < kFocusTermCount; ++k) t[k] = T(0);
             return T(0);
@@ -1048,6 +1077,8 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
         double q[2];
 #pragma unroll
         for (int dim = 0; dim < 2; ++dim) {
+            q[dim] = pos[dim];
+            if (lib_inside(g.axis[dim], pos[dim])) continue;
             q[dim] = lib_wrap(g.axis[dim], pos[dim]);
             if (!lib_contains(g.axis[dim].ghost_lower, g.axis[dim].ghost_upper, q[dim])) {
                 set_error(error, 1);
@@ -1058,10 +1089,10 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
     }
     const T p_in = static_cast<T>(s.p[i]);
     const T p = p_in >= T(0) ? p_in : -p_in;
-    const T mu = focus_reflect(static_cast<T>(s.mu[i]), static_cast<T>(L.max_mu), error);
-    const T normalized = p / static_cast<T>(L.mc);
+    const T mu = focus_reflect(static_cast<T>(s.mu[i]), C.max_mu, error);
+    const T normalized = p / C.mc;
     const T gamma = M::sqrt(T(1) + normalized * normalized);
-    const T speed = p / (gamma * static_cast<T>(L.rest_mass));
+    const T speed = p / (gamma * C.rest_mass);
     const T bmag = v[18];
     if (!finite_positive(bmag)) {
         set_error(error, 9);  // "focused transport requires |B| > 0"
@@ -1090,7 +1121,7 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
     const T mu2 = mu * mu;
     const T gdf = T(0.5) * (T(1) - mu2);
     const T cdf = mu2;
-    const T prefactor = p * speed * static_cast<T>(L.speed_of_light) / static_cast<T>(L.charge);
+    const T prefactor = p * speed * C.speed_of_light / C.charge;
     T total[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1111,17 +1142,8 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
     t[fDirX] = dir[0];
     t[fDirY] = dir[1];
     t[fDirZ] = dir[2];
-    if constexpr (!kMixed) t[fMomentum] = p;
+    t[fMomentum] = p;
     t[fMu] = mu;
-    t[fSpeed] = speed;
-    t[fGamma] = gamma;
-    t[fBmag] = bmag;
-    t[fDivV] = v[21];
-    t[fFocusing] = v[22];
-    t[fBBGradV] = v[23];
-    t[fConvective] = v[24];
-    t[fSigma2] = v[25];
-    t[fLc] = v[26];
     const T one_minus_mu2 = T(1) - mu2;
     T acceleration = T(0);
     if (speed > T(0)) acceleration = mu * v[24] / speed;
@@ -1129,7 +1151,18 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
                               acceleration;
     const T momentum_rate = -p * momentum_factor;
     t[fMomentumRate] = momentum_rate;
-    const PitchRates<T> pitch = focus_pitch<T>(L, t, focus_pitch_setup<T>(L, t), mu, error);
+    PitchSetup<T> setup{};
+    const int setup_error = focus_pitch_setup<T>(C, v, speed, gamma, setup);
+    const PitchRates<T> pitch = focus_pitch<T>(C, setup, setup_error, mu, error);
+    t[fDivV] = setup.divv;
+    t[fBBGradV] = setup.bbgradv;
+    t[fFocusing0] = setup.focusing0;
+    t[fConvective] = setup.convective;
+    t[fXi] = setup.xi;
+    t[fXiGk] = setup.xi_gk;
+    t[fPref] = setup.pref;
+    t[fPitchD] = pitch.D;
+    t[fPitchRate] = pitch.rate;
 
     const T large = static_cast<T>(kLargeTimeStep);  // +inf in FP32
     T dmin = large;
@@ -1139,10 +1172,11 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
         const LibAxis& a = g.axis[dim];
         T dx;
         if (kMixed && !a.stored) {
-            dx = static_cast<T>(a.dx);
+            dx = a.dx32;
         } else {
-            const double x = kMixed ? pos[dim] : lib_wrap(a, pos[dim]);
-            if (!lib_contains(a.lower, a.upper, x)) {
+            const bool inside = kMixed || lib_inside(a, pos[dim]);
+            const double x = inside ? pos[dim] : lib_wrap(a, pos[dim]);
+            if (!inside && !lib_contains(a.lower, a.upper, x)) {
                 return large;
             }
             const double cell = static_cast<double>(lib_cell_index(a, x));
@@ -1182,8 +1216,18 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
     return a2 < b2 ? a2 : b2;
 }
 
+// Mixed: latency bound on the gather of four basis rows of 112 bytes from a
+// table larger than L2, so the step wants warps in flight and a short last
+// wave.  Blocks of 128 at 64 registers (eight an SM; 256 threads left the
+// kernel at three blocks, 24 warps, and 3.4 waves): 250 steps of 400 000
+// particles on 1024 x 2048 take 21.3 ms against 24.7, 22.5 at 48 registers.
+// With the term rows, the shared rates and the two launches a step is 0.085 ms,
+// 0.134 before.
+constexpr int kFocusMixedThreads = 128;
 template <typename T>
-__global__ void __launch_bounds__(256) focus_terms_kernel(const LibFocusLaunch L) {
+__global__ void __launch_bounds__(sizeof(T) == 4 ? kFocusMixedThreads : 256,
+                                  sizeof(T) == 4 ? 8 : 1)
+    focus_terms_kernel(const LibFocusLaunch L) {
     T local = static_cast<T>(kLargeTimeStep);
     T* terms = reinterpret_cast<T*>(L.terms);
     const bool stopped = *L.error != 0;
@@ -1192,14 +1236,20 @@ __global__ void __launch_bounds__(256) focus_terms_kernel(const LibFocusLaunch L
         if (L.sys.status[i] != 0) continue;
         if (L.apply_boundary && !lib_boundary_t<T>(L.grid, L.sys, i)) continue;
         int err = 0;
-        const T dt = focus_terms<T>(L, i, terms + i * kFocusTermCount, &err);
+        T row[kFocusTermCount];
+        const T dt = focus_terms<T>(L, i, row, &err);
         if (err != 0) {
             record_error(L.error, err, static_cast<uint32_t>(i), L.error_index);
             continue;
         }
+#pragma unroll
+        for (int k = 0; k < kFocusTermCount; ++k) {
+            if (sizeof(T) == 4 && k == fMomentum) continue;  // its base is the FP64 state
+            terms[k * L.term_stride + i] = row[k];
+        }
         local = dt < local ? dt : local;
     }
-    block_min_to_global(local, L.min_bits);
+    finish_terms(local, L);
 }
 
 // advance_*_with_packed_interpolator (FocusSolver.hpp:1580-1637) with the
@@ -1207,9 +1257,10 @@ __global__ void __launch_bounds__(256) focus_terms_kernel(const LibFocusLaunch L
 // noise increments and the pitch-angle update in FP32 and adds the
 // increments, with the FP64 drift dt * rate, to the FP64 positions.
 template <typename T>
-__global__ void __launch_bounds__(256) focus_advance_kernel(const LibFocusLaunch L) {
+__global__ void __launch_bounds__(sizeof(T) == 4 ? kFocusMixedThreads : 256)
+    focus_advance_kernel(const LibFocusLaunch L) {
     const double dt = L.dt_device != nullptr ? *L.dt_device : L.dt;
-    if (!(isfinite(dt) && dt > 0.0) || *L.error != 0) {
+    if (!(f64_finite(dt) && f64_positive(dt)) || *L.error != 0) {
         return;
     }
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
@@ -1222,7 +1273,12 @@ __global__ void __launch_bounds__(256) focus_advance_kernel(const LibFocusLaunch
             s.prev_y[i] = s.y[i];
         }
         if (i >= L.count || s.status[i] != 0) continue;
-        const T* t = reinterpret_cast<const T*>(L.terms) + i * kFocusTermCount;
+        T t[kFocusTermCount];
+#pragma unroll
+        for (int k = 0; k < kFocusTermCount; ++k) {
+            if (sizeof(T) == 4 && k == fMomentum) continue;
+            t[k] = reinterpret_cast<const T*>(L.terms)[k * L.term_stride + i];
+        }
         T inc[2] = {T(0), T(0)};
         T pitch_normal = T(0);
         const T tdt = static_cast<T>(dt);
@@ -1230,12 +1286,11 @@ __global__ void __launch_bounds__(256) focus_advance_kernel(const LibFocusLaunch
             NormalPair<T> n01, n23;
             step_normals<T>(L.key, L.frame, L.noise, L.count, i, n01, n23);
             const T gv[3] = {n01.x, n01.y, n23.x};
-            const T d[3] = {static_cast<T>(t[fDirX]), static_cast<T>(t[fDirY]),
-                            static_cast<T>(t[fDirZ])};
+            const T d[3] = {t[fDirX], t[fDirY], t[fDirZ]};
             T parallel = T(0);
 #pragma unroll
             for (int c = 0; c < 3; ++c) parallel += gv[c] * d[c];
-            const T kperp = static_cast<T>(t[fKappaPerp]);
+            const T kperp = t[fKappaPerp];
             const T scale = kperp > T(0) ? LibMath<T>::sqrt(T(2) * kperp * tdt) : T(0);
 #pragma unroll
             for (int c = 0; c < 2; ++c) inc[c] = scale * (gv[c] - parallel * d[c]);
@@ -1251,17 +1306,22 @@ __global__ void __launch_bounds__(256) focus_advance_kernel(const LibFocusLaunch
             // base is the FP64 state, as the terms pass read it
             s.x[i] += static_cast<double>(tdt * t[fRateX] + inc[0]);
             s.y[i] += static_cast<double>(tdt * t[fRateY] + inc[1]);
-            const double base = s.p[i] >= 0.0 ? s.p[i] : -s.p[i];
-            const double updated = base + static_cast<double>(tdt * t[fMomentumRate]);
-            s.p[i] = updated > 0.0 ? updated : 0.0;
+            const double updated = fabs(s.p[i]) + static_cast<double>(tdt * t[fMomentumRate]);
+            s.p[i] = f64_positive(updated) && !f64_nan(updated) ? updated : 0.0;
         }
         int err = 0;
-        const T max_mu = static_cast<T>(L.max_mu);
-        const T initial = focus_reflect(static_cast<T>(t[fMu]), max_mu, &err);
-        const PitchSetup<T> setup = focus_pitch_setup<T>(L, t);
+        const LibFocusConsts<T>& C = focus_consts<T>(L);
+        const T max_mu = C.max_mu;
+        const T initial = focus_reflect(t[fMu], max_mu, &err);
+        const PitchSetup<T> setup{t[fFocusing0], t[fConvective], t[fXi],    t[fXiGk],
+                                  t[fPref],      t[fDivV],       t[fBBGradV]};
+        // a cosine so far out that its reflections were cut short is evaluated again
+        const bool kept = t[fMu] >= -max_mu && t[fMu] <= max_mu;
         T trial = initial;
         for (int it = 0; it < 3; ++it) {
-            const PitchRates<T> pitch = focus_pitch<T>(L, t, setup, trial, &err);
+            const PitchRates<T> pitch = it == 0 && kept
+                                            ? PitchRates<T>{t[fPitchD], t[fPitchRate]}
+                                            : focus_pitch<T>(C, setup, 0, trial, &err);
             const T scale = pitch.D > T(0) ? LibMath<T>::sqrt(T(2) * pitch.D * tdt) : T(0);
             trial = initial + tdt * pitch.rate + scale * pitch_normal;
             trial = focus_reflect(trial, max_mu, &err);
@@ -2537,16 +2597,12 @@ cudaError_t lib_basis_to_f32(const double* src, int src_stride, float* dst, int 
 }
 
 cudaError_t lib_parker_step(const LibParkerLaunch& L, cudaStream_t stream) {
-    lib_reset_min_kernel<<<1, 1, 0, stream>>>(L.min_bits);
-    if (L.count > 0) {
-        if (L.mixed) {
-            lib_parker_terms_kernel<float><<<grid_for(L.count, 256), 256, 0, stream>>>(L);
-        } else {
-            lib_parker_terms_kernel<double><<<grid_for(L.count, 256), 256, 0, stream>>>(L);
-        }
+    const uint64_t count = L.count > 0 ? L.count : 1;  // the dt is noted in any case
+    if (L.mixed) {
+        lib_parker_terms_kernel<float><<<grid_for(count, 256), 256, 0, stream>>>(L);
+    } else {
+        lib_parker_terms_kernel<double><<<grid_for(count, 256), 256, 0, stream>>>(L);
     }
-    lib_finish_dt_kernel<<<1, 1, 0, stream>>>(L.min_bits, L.courant, L.dt_device_out,
-                                              L.dt_history, L.error, L.advance);
     if (L.advance) {
         LibParkerLaunch A = L;
         A.dt_device = L.dt_device_out;
@@ -2560,21 +2616,19 @@ cudaError_t lib_parker_step(const LibParkerLaunch& L, cudaStream_t stream) {
 }
 
 cudaError_t lib_focus_step(const LibFocusLaunch& L, cudaStream_t stream) {
-    lib_reset_min_kernel<<<1, 1, 0, stream>>>(L.min_bits);
-    if (L.count > 0) {
-        if (L.mixed) {
-            focus_terms_kernel<float><<<grid_for(L.count, 256), 256, 0, stream>>>(L);
-        } else {
-            focus_terms_kernel<double><<<grid_for(L.count, 256), 256, 0, stream>>>(L);
-        }
+    const uint64_t count = L.count > 0 ? L.count : 1;  // the dt is noted in any case
+    if (L.mixed) {
+        focus_terms_kernel<float><<<grid_for(count, kFocusMixedThreads), kFocusMixedThreads, 0,
+                                    stream>>>(L);
+    } else {
+        focus_terms_kernel<double><<<grid_for(count, 256), 256, 0, stream>>>(L);
     }
-    lib_finish_dt_kernel<<<1, 1, 0, stream>>>(L.min_bits, L.courant, L.dt_device_out,
-                                              L.dt_history, L.error, L.advance);
     if (L.advance) {
         LibFocusLaunch A = L;
         A.dt_device = L.dt_device_out;
         if (L.mixed) {
-            focus_advance_kernel<float><<<grid_for(L.capacity, 256), 256, 0, stream>>>(A);
+            focus_advance_kernel<float><<<grid_for(L.capacity, kFocusMixedThreads),
+                                          kFocusMixedThreads, 0, stream>>>(A);
         } else {
             focus_advance_kernel<double><<<grid_for(L.capacity, 256), 256, 0, stream>>>(A);
         }
