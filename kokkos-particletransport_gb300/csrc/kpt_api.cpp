@@ -607,13 +607,19 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
     KPT_REQUIRE(precision == KPT_PRECISION_F64 || precision == KPT_PRECISION_MIXED,
                 "kpt_field_create: unknown precision");
     const size_t cells = static_cast<size_t>(nx) * static_cast<size_t>(ny);
-    // data read by kpt_field_data_read was checked on the reading thread
-    for (size_t k = 0; !device_readable && k < 3 * cells; ++k) {
-        if (!std::isfinite(b_cells[k]) || !std::isfinite(v_cells[k])) {
-            return set_error(KPT_ERROR_FORMAT, "AthenaFieldReader: non-finite field value.");
+    // data read by kpt_field_data_read was checked on the reading thread; other
+    // cells are checked by the table kernel, and here only ahead of an earlier
+    // failure, which they come before
+    auto non_finite = [] {
+        return set_error(KPT_ERROR_FORMAT, "AthenaFieldReader: non-finite field value.");
+    };
+    auto failed = [&](int rc) {
+        for (size_t k = 0; !device_readable && k < 3 * cells; ++k) {
+            if (!std::isfinite(b_cells[k]) || !std::isfinite(v_cells[k])) return non_finite();
         }
-    }
-    if (int rc = activate(ctx)) return rc;
+        return rc;
+    };
+    if (int rc = activate(ctx)) return failed(rc);
     struct FieldDeleter {
         void operator()(kpt_field* doomed) const { kpt_field_destroy(doomed); }
     };
@@ -635,7 +641,7 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
         std::vector<double> centers;
         std::vector<int> buckets;
         if (int rc = build_axis(counts[d], edges[d], f->grid.axis[d], centers, buckets)) {
-            return rc;
+            return failed(rc);
         }
         FixedAxisHost fixed = build_fixed_axis(f->grid.axis[d], centers);
         f->fixed[d] = fixed.axis;
@@ -667,7 +673,11 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
     double* staging = nullptr;
     cudaError_t err = cudaSuccess;
     if (!device_readable) {
-        KPT_CUDA(cudaMalloc(&staging, 6 * cells * sizeof(double)));
+        // the cells and, behind them, the check's flag
+        KPT_CUDA(cudaMalloc(&staging, (6 * cells + 1) * sizeof(double)));
+        err = cudaMemsetAsync(staging + 6 * cells, 0, sizeof(double), ctx->stream);
+    }
+    if (!device_readable && err == cudaSuccess) {
         err = cudaMemcpyAsync(staging, b_cells, 3 * cells * sizeof(double),
                               cudaMemcpyHostToDevice, ctx->stream);
         if (err == cudaSuccess) {
@@ -681,9 +691,16 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
         launch.b_cells = device_readable ? b_device : staging;
         launch.v_cells = device_readable ? v_device : staging + 3 * cells;
         launch.table = f->table;
+        launch.non_finite =
+            device_readable ? nullptr : reinterpret_cast<int*>(staging + 6 * cells);
         launch.focused = table_kind == KPT_TABLE_FOCUSED21;
         launch.precision = precision;
         err = kpt::launch_build_table(launch, ctx->stream);
+    }
+    int found = 0;
+    if (err == cudaSuccess && !device_readable) {
+        err = cudaMemcpyAsync(&found, staging + 6 * cells, sizeof(int), cudaMemcpyDeviceToHost,
+                              ctx->stream);
     }
     if (err == cudaSuccess) {
         err = cudaStreamSynchronize(ctx->stream);
@@ -693,6 +710,7 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
         return set_error(KPT_ERROR_CUDA,
                          std::string("kpt_field_create: ") + cudaGetErrorString(err));
     }
+    if (found != 0) return non_finite();
     *out = f.release();
     return KPT_OK;
 }

@@ -6,6 +6,7 @@
 // table is bit-identical to the reference's host build.
 #include <cuda_runtime.h>
 
+#include "kpt_f64.cuh"
 #include "kpt_internal.h"
 
 namespace kpt {
@@ -100,6 +101,14 @@ __global__ void build_table_kernel(const TableLaunch L) {
         const double by = b(1, i, j);
         const double bz = b(2, i, j);
         const double bm = bmag(b, i, j);
+        // The reader's check of the cells, each by the thread of its own point:
+        // on the host it took 1.1 ms of a frame's 2.1 ms for 512 x 1024 cells,
+        // here it is three loads and six integer tests beside the rest.
+        if (L.non_finite != nullptr && i >= 0 && i < nx && j >= 0 && j < ny &&
+            !(f64_finite(bx) && f64_finite(by) && f64_finite(bz) && f64_finite(v(0, i, j)) &&
+              f64_finite(v(1, i, j)) && f64_finite(v(2, i, j)))) {
+            *L.non_finite = 1;
+        }
         if (!FOCUSED) {
             out[0] = v(0, i, j);
             out[1] = v(1, i, j);

@@ -146,6 +146,7 @@ struct TableLaunch {
     const double* b_cells;
     const double* v_cells;
     void* table;
+    int* non_finite;  // set when a cell holds an infinity or NaN (NULL: checked already)
     int focused;
     int precision;
 };
