@@ -1998,7 +1998,7 @@ int kpt_particles_sort(kpt_context* ctx, kpt_particles* parts, const kpt_field* 
                 "kpt_particles_sort: too many tiles");
     const uint64_t n = std::max<uint64_t>(parts->count, 1);
     KPT_CUDA(parts->order.reserve(n * sizeof(uint32_t)));
-    KPT_CUDA(parts->keys.reserve(n * sizeof(uint32_t)));
+    KPT_CUDA(parts->keys.reserve(2 * n * sizeof(uint32_t)));
     KPT_CUDA(parts->tile_counts.reserve((static_cast<size_t>(tiles_x) * tiles_y + 1) *
                                         sizeof(uint32_t)));
     kpt::SortLaunch launch{};
@@ -2010,6 +2010,7 @@ int kpt_particles_sort(kpt_context* ctx, kpt_particles* parts, const kpt_field* 
     launch.tiles_x = tiles_x;
     launch.tiles_y = tiles_y;
     launch.keys = parts->keys.as<unsigned int>();
+    launch.ranks = launch.keys + n;
     launch.counts = parts->tile_counts.as<unsigned int>();
     launch.order = parts->order.as<unsigned int>();
     KPT_CUDA(kpt::launch_sort(launch, ctx->stream));
@@ -4002,7 +4003,7 @@ int batch_prepare(kpt_batch* b) {
             const int ty = (run.lower->ny + b->sort_tile - 1) / b->sort_tile;
             const uint64_t n = std::max<uint64_t>(parts->count, 1);
             KPT_CUDA(parts->order.reserve(n * sizeof(uint32_t)));
-            KPT_CUDA(parts->keys.reserve(n * sizeof(uint32_t)));
+            KPT_CUDA(parts->keys.reserve(2 * n * sizeof(uint32_t)));
             KPT_CUDA(parts->tile_counts.reserve((static_cast<size_t>(tx) * ty + 1) *
                                                 sizeof(uint32_t)));
             parts->order_valid = true;
@@ -4052,6 +4053,7 @@ cudaError_t batch_sort_all(const kpt_batch* b, cudaStream_t stream) {
         s.tiles_x = (run.lower->nx + b->sort_tile - 1) / b->sort_tile;
         s.tiles_y = (run.lower->ny + b->sort_tile - 1) / b->sort_tile;
         s.keys = parts->keys.as<unsigned int>();
+        s.ranks = s.keys + parts->count;
         s.counts = parts->tile_counts.as<unsigned int>();
         s.order = parts->order.as<unsigned int>();
         const cudaError_t err = kpt::launch_sort(s, stream);

@@ -227,6 +227,7 @@ struct SortLaunch {
     uint64_t count;
     int tile_x, tile_y, tiles_x, tiles_y;
     unsigned int* keys;     // count
+    unsigned int* ranks;    // count: place within the tile
     unsigned int* counts;   // tiles + 1
     unsigned int* order;    // count
 };

@@ -328,19 +328,69 @@ __device__ __forceinline__ int cell_of(const Axis& a, double x) {
     return k;
 }
 
+__device__ __forceinline__ unsigned sort_key(const SortLaunch& L, uint64_t i) {
+    if (L.parts.status[i] != 0) {
+        return static_cast<unsigned>(L.tiles_x) * static_cast<unsigned>(L.tiles_y);
+    }
+    const int cx = cell_of(L.grid.axis[0], L.parts.x[i]);
+    const int cy = cell_of(L.grid.axis[1], L.parts.y[i]);
+    return static_cast<unsigned>(cy / L.tile_y) * static_cast<unsigned>(L.tiles_x) +
+           static_cast<unsigned>(cx / L.tile_x);
+}
+
+// Keys, ranks within a tile (the atomics' results, so that the scatter needs
+// none) and tile counts.  With few tiles the population meets in few words and
+// the atomics' serial chain is the kernel's time (190 000 particles in 257
+// tiles: 50 us, and again in the scatter): then a block ranks its chunk of 512
+// particles in shared memory and takes one range of each tile it holds, 8.3 us
+// (11.4 us in chunks of 2048, whose FP64 cell maps queue on too few SMs); the
+// scatter takes 3.9 us.  Clearing and reading a word for every tile costs more
+// than the direct atomics from some thousands of tiles on (126 000 particles in
+// 8192 tiles: 5.7 us direct), 80 000 in 1000 tiles take 14 us directly.
+constexpr int kSortThreads = 256;
+constexpr int kSortItems = 2;
+constexpr int kSortChunk = kSortThreads * kSortItems;
+constexpr int kSortShared = 2048;  // the most words ranked in shared memory
+
+__global__ void __launch_bounds__(kSortThreads) sort_key_shared_kernel(const SortLaunch L) {
+    __shared__ unsigned int tally[kSortShared];
+    const int words = L.tiles_x * L.tiles_y + 1;
+    const int tid = static_cast<int>(threadIdx.x);
+    for (uint64_t base = blockIdx.x * static_cast<uint64_t>(kSortChunk); base < L.count;
+         base += static_cast<uint64_t>(gridDim.x) * kSortChunk) {
+        for (int k = tid; k < words; k += kSortThreads) tally[k] = 0u;
+        __syncthreads();
+        unsigned key[kSortItems], rank[kSortItems];
+#pragma unroll
+        for (int m = 0; m < kSortItems; ++m) {
+            const uint64_t i = base + m * kSortThreads + tid;
+            if (i >= L.count) continue;
+            key[m] = sort_key(L, i);
+            rank[m] = atomicAdd(tally + key[m], 1u);
+        }
+        __syncthreads();
+        for (int k = tid; k < words; k += kSortThreads) {
+            const unsigned held = tally[k];
+            if (held != 0u) tally[k] = atomicAdd(L.counts + k, held);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < kSortItems; ++m) {
+            const uint64_t i = base + m * kSortThreads + tid;
+            if (i >= L.count) continue;
+            L.keys[i] = key[m];
+            L.ranks[i] = tally[key[m]] + rank[m];
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void sort_key_kernel(const SortLaunch L) {
-    const unsigned tiles = static_cast<unsigned>(L.tiles_x) * static_cast<unsigned>(L.tiles_y);
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < L.count;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        unsigned key = tiles;
-        if (L.parts.status[i] == 0) {
-            const int cx = cell_of(L.grid.axis[0], L.parts.x[i]);
-            const int cy = cell_of(L.grid.axis[1], L.parts.y[i]);
-            key = static_cast<unsigned>(cy / L.tile_y) * static_cast<unsigned>(L.tiles_x) +
-                  static_cast<unsigned>(cx / L.tile_x);
-        }
+        const unsigned key = sort_key(L, i);
         L.keys[i] = key;
-        atomicAdd(L.counts + key, 1u);
+        L.ranks[i] = atomicAdd(L.counts + key, 1u);
     }
 }
 
@@ -384,8 +434,7 @@ __global__ void __launch_bounds__(1024) sort_scan_kernel(unsigned int* counts, i
 __global__ void sort_scatter_kernel(const SortLaunch L) {
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < L.count;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const unsigned slot = atomicAdd(L.counts + L.keys[i], 1u);
-        L.order[slot] = static_cast<unsigned int>(i);
+        L.order[L.counts[L.keys[i]] + L.ranks[i]] = static_cast<unsigned int>(i);
     }
 }
 
@@ -398,7 +447,13 @@ cudaError_t launch_sort(const SortLaunch& L, cudaStream_t stream) {
     const int threads = 256;
     const uint64_t want = (L.count + threads - 1) / threads;
     const int blocks = static_cast<int>(want > 152u * 16u ? 152u * 16u : want);
-    sort_key_kernel<<<blocks, threads, 0, stream>>>(L);
+    if (tiles <= kSortShared) {
+        const uint64_t chunks = (L.count + kSortChunk - 1) / kSortChunk;
+        sort_key_shared_kernel<<<static_cast<int>(chunks > 152u * 16u ? 152u * 16u : chunks),
+                                 kSortThreads, 0, stream>>>(L);
+    } else {
+        sort_key_kernel<<<blocks, threads, 0, stream>>>(L);
+    }
     sort_scan_kernel<<<1, 1024, 0, stream>>>(L.counts, tiles);
     sort_scatter_kernel<<<blocks, threads, 0, stream>>>(L);
     return cudaGetLastError();
