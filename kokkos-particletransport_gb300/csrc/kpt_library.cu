@@ -1223,10 +1223,12 @@ __device__ T focus_terms(const LibFocusLaunch& L, size_t i, T* t, int* error) {
 // particles on 1024 x 2048 take 21.3 ms against 24.7, 22.5 at 48 registers.
 // With the term rows, the shared rates and the two launches a step is 0.085 ms,
 // 0.134 before.
+// FP64: two blocks of 128 registers fill the FP64 pipe (left to itself the
+// compiler took 232 registers, one block an SM, the pipe 76 % busy).
 constexpr int kFocusMixedThreads = 128;
 template <typename T>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? kFocusMixedThreads : 256,
-                                  sizeof(T) == 4 ? 8 : 1)
+                                  sizeof(T) == 4 ? 8 : 2)
     focus_terms_kernel(const LibFocusLaunch L) {
     T local = static_cast<T>(kLargeTimeStep);
     T* terms = reinterpret_cast<T*>(L.terms);
