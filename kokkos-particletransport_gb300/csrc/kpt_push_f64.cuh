@@ -8,8 +8,9 @@
 // project pow about 100.  One warp per sub-partition fills the pipe, and the
 // time of an interval is the number of FP64 warp instructions on the busiest
 // sub-partition.  The code below is therefore organised around that count,
-// with the same operations on the same operands (every result equals the
-// lane-by-lane evaluation bit for bit):
+// with the same operations on the same operands (strict arithmetic equals the
+// lane-by-lane evaluation bit for bit, contracted arithmetic but for last bits
+// of single particles, where the compiler fuses another product):
 //
 //  * Warp-collective work.  The table interpolation (17 operations per
 //    component) and the divisions, square roots and powers of a substep are
