@@ -21,6 +21,7 @@
 
 #include "kpt_internal.h"
 #include "kpt_pow.h"
+#include "kpt_rules.h"
 
 // One substep in KPT_JUDGE_PERIOD (a power of two) of every particle also
 // evaluates the plain closure to judge the learned one.
@@ -3930,9 +3931,9 @@ struct kpt_batch {
     std::vector<DeviceBuffer> records;
     std::vector<std::pair<uint64_t, uint64_t>> record_serials;
     bool use_records = false;
-    // cached graph of the last interval loop
+    // cached graph of the last interval loop and what it was captured for
     cudaGraphExec_t graph = nullptr;
-    uint32_t graph_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    std::vector<uint64_t> graph_key;
 };
 
 namespace {
@@ -4213,15 +4214,17 @@ int kpt_batch_run(kpt_batch* b, uint32_t intervals, int use_graph) {
     if (int rc = activate(ctx)) return rc;
     if (int rc = batch_prepare(b)) return rc;
     cudaStream_t st = ctx->stream;
-    const uint32_t key[8] = {intervals, static_cast<uint32_t>(b->sort_tile),
-                             static_cast<uint32_t>(b->blocks_per_sm),
-                             static_cast<uint32_t>(b->sort_every),
-                             static_cast<uint32_t>(b->runs.size()),
-                             static_cast<uint32_t>(b->threads),
-                             static_cast<uint32_t>(b->particles_per_lane),
-                             b->use_records ? 1u : 0u};
+    std::vector<kpt::BatchGraphRun> key_runs;
+    for (const kpt_batch::Run& run : b->runs) {
+        const kpt_particles* p = run.parts;
+        key_runs.push_back({p->count, p->order.ptr, p->keys.ptr, p->tile_counts.ptr});
+    }
+    std::vector<uint64_t> key = kpt::batch_graph_key(
+        {intervals, b->sort_tile, b->blocks_per_sm, b->sort_every, b->threads,
+         b->particles_per_lane, b->use_records},
+        key_runs);
     if (use_graph && st != nullptr) {
-        if (b->graph == nullptr || std::memcmp(key, b->graph_key, sizeof(key)) != 0) {
+        if (b->graph == nullptr || key != b->graph_key) {
             batch_drop_graph(b);
             cudaGraph_t graph = nullptr;
             KPT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -4235,7 +4238,7 @@ int kpt_batch_run(kpt_batch* b, uint32_t intervals, int use_graph) {
             const cudaError_t inst = cudaGraphInstantiate(&b->graph, graph, 0);
             cudaGraphDestroy(graph);
             KPT_CUDA(inst);
-            std::memcpy(b->graph_key, key, sizeof(key));
+            b->graph_key = std::move(key);
         }
         KPT_CUDA(cudaGraphLaunch(b->graph, st));
     } else {
