@@ -171,7 +171,11 @@ __device__ __forceinline__ void copies_done() {
 // The kernels of consecutive steps are launched with programmatic dependence:
 // a kernel's blocks may start while the previous kernel drains, and read or
 // write nothing an earlier kernel touches before previous_done (which returns
-// once the previous kernel, and so everything before it, has completed).
+// once the previous kernel, and so everything before it, has completed).  The
+// buffers the kernels hand on therefore change while their readers are
+// resident: they are plain pointers, read with ordinary loads after the wait.
+// (const __restrict__ would promise data that is constant for the kernel's
+// life, and allow non-coherent loads; only the training set is that.)
 __device__ __forceinline__ void previous_done() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -200,9 +204,8 @@ template <int H>
 __global__ void __launch_bounds__(kPassThreads)
     train_pass_kernel(const float* __restrict__ x, const float* __restrict__ t, int n,
                       uint64_t seed, int step, int batch, const SurrogateBox box,
-                      const float* __restrict__ params, float* __restrict__ xb,
-                      float* __restrict__ h1, float* __restrict__ h2, float* __restrict__ g1,
-                      float* __restrict__ g2, float* __restrict__ gy, float* loss, int quant) {
+                      const float* params, float* xb, float* h1, float* h2, float* g1, float* g2,
+                      float* gy, float* loss, int quant) {
     // quant != 0: the forward sees the served network's rounding (weights,
     // inputs and activations in the 16-bit type, FP16 pre-activations too;
     // biases and accumulation FP32) and the backward passes straight
@@ -425,10 +428,8 @@ constexpr size_t grad_smem_bytes() {
 }
 template <int H>
 __global__ void __launch_bounds__(kGradThreads + 32)
-    train_grad_kernel(int batch, const float* __restrict__ xb, const float* __restrict__ h1,
-                      const float* __restrict__ h2, const float* __restrict__ g1,
-                      const float* __restrict__ g2, const float* __restrict__ gy,
-                      float* __restrict__ partial) {
+    train_grad_kernel(int batch, const float* xb, const float* h1, const float* h2,
+                      const float* g1, const float* g2, const float* gy, float* partial) {
     using M = Mlp<H>;
     extern __shared__ __align__(16) float grad_smem[];
     const int tid = threadIdx.x;
@@ -547,24 +548,22 @@ __global__ void __launch_bounds__(kGradThreads + 32)
 }
 
 // The chunk partials of one parameter in chunk order.
-__device__ __forceinline__ float chunk_sum(const float* __restrict__ partial, int chunks,
-                                           int params, int k) {
+__device__ __forceinline__ float chunk_sum(const float* partial, int chunks, int params, int k) {
     float sum = 0.0f;
 #pragma unroll 16
     for (int ch = 0; ch < chunks; ++ch) sum += partial[static_cast<size_t>(ch) * params + k];
     return sum;
 }
 
-__global__ void grad_sum_kernel(const float* __restrict__ partial, int chunks, int params,
-                                float* __restrict__ grad) {
+__global__ void grad_sum_kernel(const float* partial, int chunks, int params, float* grad) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < params) grad[k] = chunk_sum(partial, chunks, params, k);
 }
 
 // Chunk sums and Adam, one thread per parameter.
-__global__ void train_update_kernel(const float* __restrict__ partial, int chunks, float* params,
-                                    float* m, float* v, int count, float lr, float beta1,
-                                    float beta2, float eps, float bias1, float bias2) {
+__global__ void train_update_kernel(const float* partial, int chunks, float* params, float* m,
+                                    float* v, int count, float lr, float beta1, float beta2,
+                                    float eps, float bias1, float bias2) {
     next_may_start();
     previous_done();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
