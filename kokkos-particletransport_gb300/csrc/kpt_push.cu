@@ -32,6 +32,7 @@
 #include "kpt_device.cuh"
 #include "kpt_internal.h"
 #include "kpt_pow.h"
+#include "kpt_tally.h"
 
 // What this translation unit emits.  0 (the default): everything but the
 // strict FP64 push and the FP64 table sampling, with FMA contraction and
@@ -1050,36 +1051,9 @@ __device__ __forceinline__ bool substep_records(StateMixed& st, const PushParams
     return have && advance_mixed<FOCUSED>(st, P, c);
 }
 
-// Counters of one block, in shared memory: they change when a particle
-// finishes, is judged or falls back, so keeping them out of the registers
-// costs nothing per substep and leaves 7 (14 with the network's) registers to
-// the warps.
-struct BlockTally {
-    unsigned steps[2], fallbacks[2];  // low and high words
-    unsigned pushed, failed, max_steps, judged;
-    unsigned max_error;  // float bits (non-negative floats order like them)
-};
-
 __device__ __forceinline__ void tally_init(BlockTally& b) {
     if (threadIdx.x == 0) b = BlockTally{};
     __syncthreads();
-}
-
-__device__ __forceinline__ void tally_add(unsigned (&word)[2], unsigned v) {
-    const unsigned old = atomicAdd(&word[0], v);
-    if (old + v < old) atomicAdd(&word[1], 1u);
-}
-
-// A particle the block loaded has reached its last substep.
-__device__ __forceinline__ void tally_finish(BlockTally& b, int steps, int status) {
-    tally_add(b.steps, static_cast<unsigned>(steps));
-    atomicAdd(&b.pushed, 1u);
-    if (status != 0) atomicAdd(&b.failed, 1u);
-    atomicMax(&b.max_steps, static_cast<unsigned>(steps));
-}
-
-__device__ __forceinline__ unsigned long long tally_word(const unsigned (&word)[2]) {
-    return (static_cast<unsigned long long>(word[1]) << 32) | word[0];
 }
 
 // The block's counters to the launch's (every thread calls it, at the end).
@@ -1093,9 +1067,9 @@ __device__ __forceinline__ void tally_flush(const BlockTally& b, PushCounters* c
     if (b.failed) atomicAdd(&counters->failed, static_cast<unsigned long long>(b.failed));
     if (b.max_steps) atomicMax(&counters->max_steps, b.max_steps);
     if (judge != nullptr) {
-        // every substep of a particle is served by the network or falls back
+        const unsigned long long evaluations = tally_evaluations(b);
         const unsigned long long fallbacks = tally_word(b.fallbacks);
-        if (steps != fallbacks) atomicAdd(judge + 0, steps - fallbacks);
+        if (evaluations) atomicAdd(judge + 0, evaluations);
         if (b.judged) atomicAdd(judge + 1, static_cast<unsigned long long>(b.judged));
         if (fallbacks) atomicAdd(judge + 2, fallbacks);
         atomicMax(judge + 3, static_cast<unsigned long long>(b.max_error));
@@ -1522,6 +1496,8 @@ __global__ void __launch_bounds__(128, H == 32 ? KPT_SURROGATE_TC32_MIN_BLOCKS
         const bool more = substep_surrogate<FP16, H, true>(st, P, have, nullptr, tally, xpose,
                                                            &net, &fail, &stop);
         if (stop) {
+            // the substep that was under way is not served
+            if (have) tally_abandon(tally, st.steps - 1);
             break;
         }
         if (have && !more) {
