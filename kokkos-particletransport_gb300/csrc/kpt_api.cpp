@@ -1110,26 +1110,6 @@ void fill_push_launch(const kpt_context* ctx, const kpt_particles* parts, const 
     launch.surrogate = nullptr;
 }
 
-// Whether a push gains from cell records (KPT_RECORDS_AUTO).  They cost about
-// 0.15 ns per table point to build.  Populations of a quarter of the points
-// and more always gain; so do smaller ones that fill the chip
-// (1.25 times the lanes of the record kernel's five blocks per SM, four times
-// with the learned closure, whose network hides more of the gathers) once the
-// interval's fewest substeps, mhd_dt / dt_max, make ten particle-steps a
-// point: 130 000 focused particles on 512 x 1024, 100 steps 2.79 -> 2.45 ms;
-// 300 000 Parker particles on 1024 x 2048, 100 steps 2.02 -> 1.86 ms, adaptive
-// 25.7 -> 20.8 ms; below, 100 000 Parker 0.90 / 0.98 ms, 13.7 / 14.7 ms;
-// learned 200 000 4.73 / 4.91 ms, 400 000 8.43 / 8.10 ms.
-bool records_pay(const kpt_context* ctx, const kpt_particles* parts, const kpt_field* lower,
-                 const kpt_settings* settings) {
-    if (parts->count * 4 >= lower->points) return true;
-    const double lanes = 640.0 * ctx->sm_count;
-    const double fill = settings->closure == KPT_CLOSURE_SURROGATE ? 4.0 : 1.25;
-    const double count = static_cast<double>(parts->count);
-    return count >= fill * lanes &&
-           count >= 10.0 * settings->dt_max_rel * static_cast<double>(lower->points);
-}
-
 // The cell records a mixed push samples (*out = nullptr: the point-major
 // tables), built on the context's stream when the table pair differs from
 // the one they hold.  Should the records not fit in device memory the push
@@ -1142,7 +1122,10 @@ int push_records(kpt_context* ctx, const kpt_particles* parts, const kpt_field* 
         lower->points >= (1ull << 32)) {
         return KPT_OK;
     }
-    if (ctx->records_mode == KPT_RECORDS_AUTO && !records_pay(ctx, parts, lower, settings)) {
+    if (ctx->records_mode == KPT_RECORDS_AUTO &&
+        !kpt::records_pay({settings->focused != 0, settings->closure == KPT_CLOSURE_SURROGATE,
+                           parts->count, lower->points, settings->dt_min_rel,
+                           settings->dt_max_rel, ctx->sm_count})) {
         return KPT_OK;
     }
     if (ctx->records_lower != lower->serial || ctx->records_upper != upper->serial ||

@@ -1,0 +1,92 @@
+"""The launch rules (kpt_rules.h) on the host, against times measured on the
+GB300 (152 SMs) at sizes, substeps and populations on both sides of each line:
+what a rule picks may not be slower than the simple choice it departs from."""
+from __future__ import annotations
+
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "kokkos-particletransport_gb300", "csrc")
+SMS = 152
+SHIM = """
+#include "kpt_rules.h"
+extern "C" int records_pay(int focused, int learned, uint64_t particles, uint64_t points,
+                           double dt_min, double dt_max, int sms) {
+    return kpt::records_pay({focused != 0, learned != 0, particles, points, dt_min, dt_max, sms});
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    path = tmp_path_factory.mktemp("rules")
+    src, so = str(path / "rules.cpp"), str(path / "rules.so")
+    with open(src, "w") as f:
+        f.write(SHIM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", CSRC, src, "-o", so],
+                   check=True)
+    lib = ctypes.CDLL(so)
+    u64, dbl, i32 = ctypes.c_uint64, ctypes.c_double, ctypes.c_int
+    lib.records_pay.argtypes = [i32, i32, u64, u64, dbl, dbl, i32]
+    return lib
+
+
+# focused, nx, ny, particles, substeps, and ms of an interval whose tables are
+# new: on the point tables, on records (plain closures, fixed steps)
+SINGLE = [
+    (0, 1024, 1024, 126814, 100, 0.785, 0.958), (0, 1024, 1024, 126814, 200, 1.484, 1.580),
+    (0, 1024, 1024, 211356, 100, 1.110, 1.221), (0, 1024, 1024, 211356, 400, 4.297, 3.710),
+    (0, 1024, 1024, 253628, 50, 0.712, 0.770), (0, 1024, 1024, 253628, 200, 2.667, 2.242),
+    (0, 1024, 2048, 126567, 200, 1.521, 1.992), (0, 1024, 2048, 126567, 400, 2.955, 3.276),
+    (0, 1024, 2048, 253134, 100, 1.372, 1.706), (0, 1024, 2048, 253134, 200, 2.679, 2.839),
+    (0, 1024, 2048, 421891, 100, 2.193, 2.332), (0, 1024, 2048, 421891, 400, 8.641, 7.137),
+    (0, 1024, 2048, 506269, 50, 1.320, 1.540), (0, 1024, 2048, 506269, 400, 10.230, 8.161),
+    (0, 2048, 4096, 252396, 400, 6.520, 7.684), (0, 2048, 4096, 504792, 200, 5.529, 7.922),
+    (0, 2048, 4096, 504792, 400, 10.483, 13.901), (0, 2048, 4096, 1009584, 100, 5.125, 7.253),
+    (0, 2048, 4096, 1009584, 400, 19.979, 22.901), (0, 2048, 4096, 1682640, 100, 8.344, 9.967),
+    (0, 2048, 4096, 2019168, 50, 5.112, 6.470), (0, 2048, 4096, 2019168, 100, 9.970, 11.107),
+    (1, 1024, 1024, 126814, 100, 1.215, 1.414), (1, 1024, 1024, 126814, 200, 2.299, 2.526),
+    (1, 1024, 1024, 211356, 100, 1.688, 1.903), (1, 1024, 1024, 211356, 200, 3.256, 3.456),
+    (1, 1024, 1024, 253628, 50, 1.077, 1.115), (1, 1024, 1024, 253628, 200, 4.064, 3.579),
+    (1, 1024, 2048, 126567, 200, 2.511, 2.921), (1, 1024, 2048, 126567, 400, 4.611, 5.136),
+    (1, 1024, 2048, 253134, 100, 2.149, 2.424), (1, 1024, 2048, 421891, 400, 12.935, 11.647),
+    (1, 1024, 2048, 506269, 50, 2.039, 2.227), (1, 1024, 2048, 506269, 400, 15.164, 13.213),
+    (1, 2048, 4096, 504792, 200, 9.489, 10.569), (1, 2048, 4096, 504792, 400, 17.366, 19.014),
+    (1, 2048, 4096, 1009584, 100, 8.217, 9.802), (1, 2048, 4096, 1009584, 200, 15.997, 17.677),
+    (1, 2048, 4096, 1682640, 100, 13.153, 14.107), (1, 2048, 4096, 2019168, 50, 8.050, 9.084),
+]
+
+
+def _records(rules, focused, nx, ny, particles, dt_min, dt_max, learned=0):
+    return rules.records_pay(focused, learned, particles, (nx + 4) * (ny + 4), dt_min, dt_max, SMS)
+
+
+@pytest.mark.parametrize("case", SINGLE, ids=lambda c: "-".join(map(str, c[:5])))
+def test_records_of_a_thin_population(rules, case):
+    focused, nx, ny, particles, substeps, points_ms, records_ms = case
+    dt = (1.0 + 1e-6) / substeps
+    picked = records_ms if _records(rules, focused, nx, ny, particles, dt, dt) else points_ms
+    assert picked <= 1.02 * points_ms
+    if records_ms <= 0.88 * points_ms:
+        assert picked == records_ms
+
+
+def test_records_of_dense_and_small_populations(rules):
+    for focused in (0, 1):
+        for dt in (0.1, 0.001):
+            assert _records(rules, focused, 256, 256, 20000, dt, dt)      # a quarter: always
+            assert not _records(rules, focused, 4096, 4096, 60000, dt, dt)  # does not fill the chip
+    # adaptive Parker, ms: 17.97 / 17.06, 15.58 / 15.02 and 11.04 / 11.82, 11.73 / 13.51
+    assert _records(rules, 0, 1024, 2048, 253134, 1e-4, 0.01)
+    assert _records(rules, 0, 1024, 1024, 211356, 1e-4, 0.01)
+    assert not _records(rules, 0, 1024, 1024, 126814, 1e-4, 0.01)
+    assert not _records(rules, 0, 1024, 2048, 126567, 1e-4, 0.01)
+    # learned closure, ms: 4.85 / 3.85, 9.66 / 7.07, 1.65 / 2.80
+    assert _records(rules, 1, 1024, 2048, 421891, 0.01, 0.01, learned=1)
+    assert _records(rules, 1, 1024, 2048, 421891, 0.005, 0.005, learned=1)
+    assert not _records(rules, 1, 2048, 4096, 504792, 0.04, 0.04, learned=1)
