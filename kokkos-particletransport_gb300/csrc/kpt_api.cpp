@@ -3921,38 +3921,22 @@ struct kpt_batch {
 
 namespace {
 
-// Whether a batch gains from cell records (KPT_RECORDS_AUTO): as a rule when
-// its particles number a quarter of its tables' points.  Where every run's
-// step is fixed the substeps are known, and a population that fills the chip
-// but leaves most points alone goes by them: an interval reads each record it
-// meets from DRAM, so a particle has to make enough substeps, and the points
-// enough particle-steps to repay the build.  Adaptive runs can only add to
-// their fewest substeps.  Sixteen runs, 4.1 M points, first interval / later
-// ones in ms, point tables against records: Parker 980 000 particles x 50
-// 3.71 / 3.05, 4.34 / 3.01; x 100 6.02 / 5.32, 5.86 / 4.45; 1.7 M x 25
-// 4.57 / 3.74, 5.90 / 4.61, x 50 5.96 / 4.98, 6.55 / 5.11; 340 000 x 200
-// 4.69 / 4.07, 4.75 / 3.38.  Focused 980 000 x 25 3.61 / 2.83, 4.61 / 3.16;
-// x 50 5.52 / 4.60, 5.36 / 3.82; 340 000 x 50 2.59 / 1.97, 3.09 / 1.74, x 200
-// 7.07 / 6.44, 6.15 / 4.68.
+// kpt::batch_records_pay for the batch's runs.
 bool batch_records_pay(const kpt_batch* b) {
-    double particles = 0.0, points = 0.0, fewest = 0.0;
-    bool fixed = true, learned = false;
+    kpt::BatchRecordsCase c{};
+    c.focused = b->focused == 1;
+    c.fixed = true;
+    c.runs = b->runs.size();
+    c.sm_count = b->ctx->sm_count;
     for (const kpt_batch::Run& run : b->runs) {
         const double count = static_cast<double>(run.parts->count);
-        particles += count;
-        points += static_cast<double>(run.lower->points);
-        fewest += count / run.settings.dt_max_rel;
-        fixed = fixed && run.settings.dt_min_rel == run.settings.dt_max_rel;
-        learned = learned || run.settings.closure == KPT_CLOSURE_SURROGATE;
+        c.particles += count;
+        c.points += static_cast<double>(run.lower->points);
+        c.steps += count / run.settings.dt_max_rel;
+        c.fixed = c.fixed && run.settings.dt_min_rel == run.settings.dt_max_rel;
+        c.learned = c.learned || run.settings.closure == KPT_CLOSURE_SURROGATE;
     }
-    const bool dense = particles * 4.0 >= points;
-    if (learned || particles < 1.25 * 640.0 * b->ctx->sm_count || particles >= points) {
-        return dense;
-    }
-    const bool focused = b->focused == 1;
-    const bool steps = fewest >= (focused ? 40.0 : 70.0) * particles &&
-                       fewest >= (focused ? 9.0 : 18.0) * points;
-    return steps || (dense && !fixed);
+    return kpt::batch_records_pay(c);
 }
 
 // Cell records for the batched push: every run's table pair gets its

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
@@ -87,6 +88,59 @@ inline bool records_pay(const RecordsCase& c) {
     const double longer = c.focused ? 1.3 + 0.025e-6 * points : 1.13 + 0.07e-6 * points;
     return steps * (0.97 * point_rounds - longer * record_rounds) >=
            (c.focused ? 0.8e-4 : 1.0e-4) * points;
+}
+
+// ---- cell records of a batch (KPT_RECORDS_AUTO)
+
+struct BatchRecordsCase {
+    bool focused, learned;
+    bool fixed;        // every run's step is fixed
+    size_t runs;
+    double particles;  // of all runs
+    double points;     // of all runs' tables
+    double steps;      // particle-steps of an interval, at least
+    int sm_count;
+};
+
+// Whether a batch gains from cell records.  They are built once for a batch's
+// tables and read by every interval; an interval reads each record it meets
+// from DRAM, so a particle has to make enough substeps and the points enough
+// particle-steps, more of them on a finer table, where a particle stays in a
+// cell for less time.  As a rule a batch takes records from a quarter as many
+// particles as points on; with fixed steps, where the substeps are known, a
+// population that fills the chip goes by both: a dense one falls back to the
+// point tables below the lower line, a thin one takes records above the higher
+// one.  Particles as many as points: always.  Adaptive runs only add to their
+// fewest substeps.  First interval / later ones in ms, point tables against
+// records (runs x table, particles, substeps):
+//   Parker   16 x  512 x  512, 2.50 M x  25   6.32 /  5.37    7.90 /  6.49
+//                              2.50 M x  50   8.20 /  7.22    8.43 /  6.80
+//                              0.99 M x 100   7.19 /  5.75    7.83 /  5.26
+//             4 x 1024 x 2048, 2.52 M x  50   8.33 /  7.86   11.27 / 10.02
+//                              2.52 M x 100  15.77 / 14.77   14.85 / 13.41
+//            48 x  256 x  256, 1.89 M x  50   6.82 /  5.73    8.18 /  5.14
+//   focused   4 x 1024 x 2048, 2.01 M x  50   9.67 /  9.22   11.76 /  9.92
+//                              2.01 M x 100  18.02 / 17.57   17.32 / 15.61
+//            16 x 1024 x 1024, 4.03 M x  50  19.37 / 18.29   22.97 / 19.23
+//            48 x  256 x  256, 1.89 M x  25   6.68 /  5.58    8.16 /  5.06
+//            16 x  512 x  512, 0.99 M x 100   9.81 /  9.16    9.23 /  7.60
+inline bool batch_records_pay(const BatchRecordsCase& c) {
+    const bool dense = c.particles * 4.0 >= c.points;
+    if (c.learned || c.particles < 1.25 * 640.0 * c.sm_count || c.particles >= c.points) {
+        return dense;
+    }
+    const double side = std::sqrt(c.points / static_cast<double>(c.runs));
+    double substeps, per_point;
+    if (c.focused) {
+        substeps = dense ? 20.0 : 40.0;
+        per_point = dense ? 0.006 * side + 8.0 : 0.0085 * side + 10.0;
+    } else {
+        substeps = dense ? 40.0 : 70.0;
+        per_point = 0.014 * side + 8.0;
+        if (!dense && per_point < 18.0) per_point = 18.0;
+    }
+    const bool pays = c.steps >= substeps * c.particles && c.steps >= per_point * c.points;
+    return pays || (dense && !c.fixed);
 }
 
 }  // namespace kpt

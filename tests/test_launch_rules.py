@@ -19,6 +19,11 @@ extern "C" int records_pay(int focused, int learned, uint64_t particles, uint64_
                            double dt_min, double dt_max, int sms) {
     return kpt::records_pay({focused != 0, learned != 0, particles, points, dt_min, dt_max, sms});
 }
+extern "C" int batch_records_pay(int focused, int fixed, int runs, double particles, double points,
+                                 double steps, int sms) {
+    return kpt::batch_records_pay({focused != 0, false, fixed != 0, (size_t)runs, particles, points,
+                                   steps, sms});
+}
 """
 
 
@@ -33,6 +38,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(so)
     u64, dbl, i32 = ctypes.c_uint64, ctypes.c_double, ctypes.c_int
     lib.records_pay.argtypes = [i32, i32, u64, u64, dbl, dbl, i32]
+    lib.batch_records_pay.argtypes = [i32, i32, i32, dbl, dbl, dbl, i32]
     return lib
 
 
@@ -90,3 +96,46 @@ def test_records_of_dense_and_small_populations(rules):
     assert _records(rules, 1, 1024, 2048, 421891, 0.01, 0.01, learned=1)
     assert _records(rules, 1, 1024, 2048, 421891, 0.005, 0.005, learned=1)
     assert not _records(rules, 1, 2048, 4096, 504792, 0.04, 0.04, learned=1)
+
+
+# focused, runs, nx, ny, particles of a run, substeps, and ms of a later
+# interval of the batch: on the point tables, on records (fixed steps)
+BATCH = [
+    (0, 4, 512, 512, 38678, 100, 1.13, 1.15), (0, 4, 512, 512, 38678, 200, 1.98, 1.83),
+    (0, 4, 512, 512, 61865, 50, 1.00, 1.08), (0, 4, 512, 512, 77000, 50, 1.15, 1.28),
+    (0, 4, 512, 512, 155000, 50, 1.99, 1.87), (0, 4, 512, 512, 155000, 200, 6.60, 4.66),
+    (0, 4, 1024, 2048, 168000, 200, 8.10, 8.49), (0, 4, 1024, 2048, 314000, 100, 7.62, 8.24),
+    (0, 4, 1024, 2048, 630000, 50, 7.86, 10.02), (0, 4, 1024, 2048, 630000, 100, 14.77, 13.41),
+    (0, 4, 1024, 2048, 1250000, 25, 11.22, 14.04), (0, 4, 1024, 2048, 1250000, 50, 15.15, 14.82),
+    (0, 16, 512, 512, 62000, 50, 3.26, 3.67), (0, 16, 512, 512, 62000, 100, 5.75, 5.26),
+    (0, 16, 512, 512, 156000, 25, 5.37, 6.49), (0, 16, 512, 512, 156000, 50, 7.22, 6.80),
+    (0, 16, 1024, 1024, 84000, 100, 8.57, 9.16), (0, 16, 1024, 1024, 252000, 50, 12.63, 16.53),
+    (0, 16, 1024, 1024, 314000, 25, 11.08, 16.91), (0, 16, 1024, 1024, 630000, 10, 19.89, 25.15),
+    (0, 48, 256, 256, 15600, 100, 4.70, 4.04), (0, 48, 256, 256, 15600, 200, 8.45, 6.57),
+    (0, 48, 256, 256, 39400, 25, 4.32, 4.47), (0, 48, 256, 256, 39400, 50, 5.73, 5.14),
+    (1, 4, 512, 512, 38678, 100, 1.70, 1.56), (1, 4, 512, 512, 77000, 25, 1.08, 1.10),
+    (1, 4, 512, 512, 77000, 50, 1.74, 1.59), (1, 4, 512, 512, 155000, 25, 1.90, 1.82),
+    (1, 4, 1024, 2048, 168000, 100, 6.41, 6.62), (1, 4, 1024, 2048, 502000, 50, 9.22, 9.92),
+    (1, 4, 1024, 2048, 502000, 100, 17.57, 15.61), (1, 4, 1024, 2048, 630000, 25, 6.99, 9.65),
+    (1, 4, 1024, 2048, 630000, 100, 21.88, 18.08), (1, 4, 1024, 2048, 1250000, 50, 22.16, 17.25),
+    (1, 16, 512, 512, 62000, 25, 3.00, 3.77), (1, 16, 512, 512, 62000, 100, 9.16, 7.60),
+    (1, 16, 512, 512, 156000, 10, 5.42, 6.44), (1, 16, 512, 512, 156000, 50, 11.44, 8.40),
+    (1, 16, 1024, 1024, 158000, 50, 11.72, 15.18), (1, 16, 1024, 1024, 252000, 50, 18.29, 19.23),
+    (1, 16, 1024, 1024, 314000, 25, 13.74, 18.86), (1, 48, 256, 256, 15600, 100, 7.45, 6.03),
+    (1, 48, 256, 256, 39400, 25, 5.58, 5.06), (1, 48, 256, 256, 39400, 50, 9.21, 6.49),
+]
+
+
+@pytest.mark.parametrize("case", BATCH, ids=lambda c: "-".join(map(str, c[:6])))
+def test_records_of_a_batch(rules, case):
+    focused, runs, nx, ny, particles, substeps, points_ms, records_ms = case
+    points = runs * (nx + 4) * (ny + 4)
+    total = runs * particles
+    on = rules.batch_records_pay(focused, 1, runs, total, points, total * substeps, SMS)
+    picked = records_ms if on else points_ms
+    # never slower than the quarter rule, and no clear gain left
+    assert picked <= 1.02 * (records_ms if 4 * total >= points else points_ms)
+    assert picked <= 1.15 * min(records_ms, points_ms)
+    # adaptive runs of a dense batch keep their records
+    assert rules.batch_records_pay(focused, 0, runs, total, points, total * substeps, SMS) or \
+        4 * total < points
