@@ -863,7 +863,7 @@ typedef struct kpt_batch kpt_batch;
 
 typedef struct kpt_batch_tuning {
     int32_t sort_tile;      /* cell-sort tile (cells), 0 = no sort */
-    int32_t blocks_per_sm;  /* resident blocks per SM, 0 = as many as fit */
+    int32_t blocks_per_sm;  /* resident blocks per SM, 0 = the library's choice */
     int32_t sort_every;     /* sort every k intervals */
     int32_t candidates;     /* schedules timed */
     float best_ms;          /* median time of the chosen schedule over the tuning intervals */
@@ -881,6 +881,10 @@ int kpt_batch_destroy(kpt_batch* batch);
 int kpt_batch_add_run(kpt_batch* batch, kpt_particles* particles, const kpt_field* lower,
                       const kpt_field* upper, const kpt_settings* settings, uint64_t seed,
                       uint32_t first_frame, int* run_index);
+/* Cell-sort tile (0 = no sort), resident blocks per SM (at most as many as
+ * fit; 0 = the library's choice: as many as fit, or on the point tables with
+ * fixed steps three blocks of 128 threads where they need few more rounds)
+ * and intervals between sorts. */
 int kpt_batch_set_schedule(kpt_batch* batch, int sort_tile, int blocks_per_sm, int sort_every);
 int kpt_batch_get_schedule(const kpt_batch* batch, int* sort_tile, int* blocks_per_sm,
                            int* sort_every);

@@ -127,7 +127,9 @@ struct BatchLaunch {
     int focused;
     unsigned long long* cursor;
     int sm_count;
-    int blocks_per_sm;       // resident blocks per SM, 0 = as many as fit
+    int blocks_per_sm;       // resident blocks per SM, 0 = chosen (batch_point_threads)
+    uint64_t particles;      // of all runs
+    int fixed_steps;         // every run's step is fixed
     int threads;             // threads per block: 64, 128 or 256
     int particles_per_lane;  // particles a lane advances side by side: 1 or 2
     int records;             // every run's PushParams carries cell records

@@ -32,6 +32,7 @@
 #include "kpt_device.cuh"
 #include "kpt_internal.h"
 #include "kpt_pow.h"
+#include "kpt_rules.h"
 #include "kpt_tally.h"
 
 // What this translation unit emits.  0 (the default): everything but the
@@ -1712,10 +1713,6 @@ constexpr int kBatchMaxRuns = 1024;
 __host__ __device__ constexpr size_t batch_offset_bytes(int runs) {
     return (static_cast<size_t>(runs + 1) * sizeof(uint64_t) + 15) / 16 * 16;
 }
-// Without records the tables' rows are shared through L1, and three blocks of
-// 128 threads reuse them better than five: 16 Parker runs, 50 steps, 3.60 ->
-// 3.31 ms.
-constexpr int kBatchPointThreads = 3 * 128;
 
 __device__ __forceinline__ int batch_run_of(const uint64_t* offsets, int runs, uint64_t slot) {
     int lo = 0;
@@ -1981,8 +1978,10 @@ cudaError_t launch_batch_shape(const BatchLaunch& B, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
     int per_sm = B.blocks_per_sm > 0 && B.blocks_per_sm < resident ? B.blocks_per_sm : resident;
-    if (B.blocks_per_sm == 0 && B.records == 0 && per_sm * THREADS > kBatchPointThreads) {
-        per_sm = kBatchPointThreads / THREADS > 0 ? kBatchPointThreads / THREADS : 1;
+    if (B.blocks_per_sm == 0 && B.records == 0) {
+        const int want = batch_point_threads(B.particles, B.fixed_steps != 0, per_sm * THREADS,
+                                             B.sm_count) / THREADS;
+        per_sm = want > 0 ? want : 1;
     }
     push_batch_kernel<FOCUSED, THREADS, PPL><<<B.sm_count * per_sm, THREADS, smem, stream>>>(B);
     return cudaGetLastError();

@@ -143,4 +143,27 @@ inline bool batch_records_pay(const BatchRecordsCase& c) {
     return pays || (dense && !c.fixed);
 }
 
+// ---- residency of a batch on the point tables
+
+// Threads per SM for a batch that samples the point tables, of the `fit` that
+// the batch's registers admit.  With fixed steps a batch runs in rounds of the
+// resident lanes.  Three blocks of 128 share the tables' rows through L1
+// better than five, whose rounds take 1.5 (few rounds) to 1.65 times as long,
+// so they win where they need few more rounds: ms at 384 / 640 threads, 50
+// steps, 980 000 Parker particles 3.31 / 3.60, 223 000 1.16 / 1.21 (focused
+// 1.59 / 1.64), 112 000 0.59 / 0.66 (0.82 / 0.90); and lose where the last of
+// the rounds is nearly empty: 190 000 1.02 / 0.96 (1.48 / 1.28), 84 000 0.54 /
+// 0.49 (0.77 / 0.64), 64 000 0.46 / 0.41 (0.62 / 0.58).  Adaptive steps have no
+// rounds and want the lanes: 192 000 Parker particles 9.40 / 8.97.
+inline int batch_point_threads(uint64_t particles, bool fixed, int fit, int sm_count) {
+    const int few = 3 * 128;
+    if (fit <= few || !fixed) return fit;
+    const auto rounds = [&](int threads) {
+        const uint64_t lanes = static_cast<uint64_t>(threads) * static_cast<uint64_t>(sm_count);
+        return static_cast<double>((particles + lanes - 1) / lanes);
+    };
+    const double longer = rounds(fit) <= 4.0 ? 1.48 : 1.65;
+    return longer * rounds(fit) < rounds(few) ? fit : few;
+}
+
 }  // namespace kpt

@@ -24,6 +24,9 @@ extern "C" int batch_records_pay(int focused, int fixed, int runs, double partic
     return kpt::batch_records_pay({focused != 0, false, fixed != 0, (size_t)runs, particles, points,
                                    steps, sms});
 }
+extern "C" int batch_point_threads(uint64_t particles, int fixed, int fit, int sms) {
+    return kpt::batch_point_threads(particles, fixed != 0, fit, sms);
+}
 """
 
 
@@ -39,6 +42,7 @@ def rules(tmp_path_factory):
     u64, dbl, i32 = ctypes.c_uint64, ctypes.c_double, ctypes.c_int
     lib.records_pay.argtypes = [i32, i32, u64, u64, dbl, dbl, i32]
     lib.batch_records_pay.argtypes = [i32, i32, i32, dbl, dbl, dbl, i32]
+    lib.batch_point_threads.argtypes = [u64, i32, i32, i32]
     return lib
 
 
@@ -139,3 +143,29 @@ def test_records_of_a_batch(rules, case):
     # adaptive runs of a dense batch keep their records
     assert rules.batch_records_pay(focused, 0, runs, total, points, total * substeps, SMS) or \
         4 * total < points
+
+
+# particles of all runs, ms of a fixed-step interval on the point tables with
+# 640 and with 384 resident threads per SM, Parker and focused
+RESIDENT = [
+    (24000, (0.61, 0.47), (0.91, 0.65)), (64000, (0.41, 0.46), (0.58, 0.62)),
+    (84000, (0.49, 0.54), (0.64, 0.77)), (112000, (0.66, 0.59), (0.90, 0.82)),
+    (120000, (0.73, 0.76), (0.99, 1.03)), (160000, (0.87, 0.91), (1.19, 1.26)),
+    (188800, (0.96, 1.01), (1.28, 1.48)), (224000, (1.21, 1.16), (1.64, 1.59)),
+    (304000, (1.46, 1.46), (1.97, 2.09)), (480000, (1.49, 1.47), (1.88, 1.87)),
+    (640000, (2.02, 1.97), (2.60, 2.55)), (980000, (3.60, 3.31), None),
+]
+
+
+@pytest.mark.parametrize("case", RESIDENT, ids=lambda c: str(c[0]))
+def test_residency_of_a_batch(rules, case):
+    particles, *times = case
+    threads = rules.batch_point_threads(particles, 1, 640, SMS)
+    assert threads in (640, 384)
+    for ms in times:
+        if ms is not None:
+            assert ms[threads == 384] <= 1.03 * min(ms)
+    # adaptive steps, 192 000 particles: 8.97 / 9.40 ms
+    assert rules.batch_point_threads(particles, 0, 640, SMS) == 640
+    # shapes that hold no more anyway
+    assert rules.batch_point_threads(particles, 1, 320, SMS) == 320
