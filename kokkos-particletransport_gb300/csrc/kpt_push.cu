@@ -1586,24 +1586,37 @@ PushParams make_push_params(const PushLaunch& L) {
 namespace kpt {
 namespace {
 
-// Ask for no more of an SM's 256 KB as shared memory than `blocks` blocks use;
-// the rest caches the gathers.  Left alone the driver set 132 KB aside for the
-// 61 KB of five blocks: 50.7 -> 49.2 ms (1 Mi Parker particles), 7.38 -> 7.22
-// ms (777 777 focused), 54.6 -> 54.0 ms (4 Mi, learned closure).  The
-// occupancy queries see the share too, so it is set before them.
-template <typename Kernel>
-cudaError_t keep_l1(Kernel kernel, int blocks, size_t block_smem) {
-    int device = 0, per_sm = 0, reserved = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess) return err;
-    err = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
-    if (err != cudaSuccess) return err;
-    err = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
-    if (err != cudaSuccess) return err;
-    const size_t block = (block_smem + static_cast<size_t>(reserved) + 1023) / 1024 * 1024;
-    const size_t percent = (100 * blocks * block + per_sm - 1) / per_sm;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                percent < 100 ? static_cast<int>(percent) : 100);
+// Launch asking for no more of an SM's 256 KB as shared memory than `blocks`
+// blocks of block_smem bytes use (0: the driver's share); the rest caches the
+// gathers.  Left alone the driver set 132 KB aside for the 61 KB of five
+// blocks: 50.7 -> 49.2 ms (1 Mi Parker particles), 7.38 -> 7.22 ms (777 777
+// focused), 54.6 -> 54.0 ms (4 Mi, learned closure).  The share goes with the
+// launch: a kernel's own attribute would be one for all threads and contexts.
+template <typename Params>
+cudaError_t launch_with_l1(void (*kernel)(const Params), int blocks, size_t block_smem, int grid,
+                           int threads, size_t smem, cudaStream_t stream, const Params& params) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(static_cast<unsigned>(grid));
+    config.blockDim = dim3(static_cast<unsigned>(threads));
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    if (blocks > 0) {
+        int device = 0, per_sm = 0, reserved = 0;
+        cudaError_t err = cudaGetDevice(&device);
+        if (err != cudaSuccess) return err;
+        err = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+        if (err != cudaSuccess) return err;
+        err = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
+        if (err != cudaSuccess) return err;
+        const size_t block = (block_smem + static_cast<size_t>(reserved) + 1023) / 1024 * 1024;
+        const size_t percent = (100 * blocks * block + per_sm - 1) / per_sm;
+        attr.val.sharedMemCarveout = percent < 100 ? static_cast<unsigned>(percent) : 100u;
+        config.attrs = &attr;
+        config.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&config, kernel, params);
 }
 
 // Persistent grid: as many resident blocks per SM as the kernel's registers
@@ -1615,20 +1628,15 @@ cudaError_t launch_push_kind(const PushParams& P, const PushLaunch& L, cudaStrea
     const size_t rows = KIND == kPushDense ? record_xpose_bytes(FOCUSED, threads / 32) : 0;
     const size_t smem = network + (P.records != nullptr ? rows : 0);
     const auto kernel = push_refill_kernel<FOCUSED, SURR, KIND>;
-    cudaError_t err = cudaSuccess;
-    if (KIND == kPushDense) {
-        err = keep_l1(kernel, push_blocks<FOCUSED, SURR, KIND>(),
-                      network + rows + sizeof(BlockTally));
-        if (err != cudaSuccess) return err;
-    }
     int resident = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
+    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
     int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm : resident;
     if (KIND == kPushFew) per_sm = kFewBlocks;  // the places lane_cap was computed for
-    kernel<<<L.sm_count * per_sm, threads, smem, stream>>>(P);
-    return cudaGetLastError();
+    const int blocks = KIND == kPushDense ? push_blocks<FOCUSED, SURR, KIND>() : 0;
+    return launch_with_l1(kernel, blocks, network + rows + sizeof(BlockTally),
+                          L.sm_count * per_sm, threads, smem, stream, P);
 }
 
 // Persistent grid of the tcgen05 push: as many blocks per SM as both the
@@ -1964,16 +1972,8 @@ template <bool FOCUSED, int THREADS, int PPL>
 cudaError_t launch_batch_shape(const BatchLaunch& B, cudaStream_t stream) {
     const size_t smem = batch_offset_bytes(B.runs) +
                         (B.records != 0 ? record_xpose_bytes(FOCUSED, THREADS / 32) : 0);
-    cudaError_t err =
-        B.records != 0
-            ? keep_l1(push_batch_kernel<FOCUSED, THREADS, PPL>,
-                      BatchMinBlocks<FOCUSED, THREADS, PPL>::value, smem)
-            : cudaFuncSetAttribute(push_batch_kernel<FOCUSED, THREADS, PPL>,
-                                   cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   cudaSharedmemCarveoutDefault);
-    if (err != cudaSuccess) return err;
     int resident = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &resident, push_batch_kernel<FOCUSED, THREADS, PPL>, THREADS, smem);
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
@@ -1983,8 +1983,9 @@ cudaError_t launch_batch_shape(const BatchLaunch& B, cudaStream_t stream) {
                                              B.sm_count) / THREADS;
         per_sm = want > 0 ? want : 1;
     }
-    push_batch_kernel<FOCUSED, THREADS, PPL><<<B.sm_count * per_sm, THREADS, smem, stream>>>(B);
-    return cudaGetLastError();
+    const int blocks = B.records != 0 ? BatchMinBlocks<FOCUSED, THREADS, PPL>::value : 0;
+    return launch_with_l1(push_batch_kernel<FOCUSED, THREADS, PPL>, blocks, smem,
+                          B.sm_count * per_sm, THREADS, smem, stream, B);
 }
 
 template <bool FOCUSED>

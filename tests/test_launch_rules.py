@@ -169,3 +169,10 @@ def test_residency_of_a_batch(rules, case):
     assert rules.batch_point_threads(particles, 0, 640, SMS) == 640
     # shapes that hold no more anyway
     assert rules.batch_point_threads(particles, 1, 320, SMS) == 320
+
+
+def test_no_launch_leaves_a_preference_on_its_kernel():
+    """A kernel's shared-memory share is a property of the process: two threads
+    whose launches want different ones would take each other's."""
+    with open(os.path.join(CSRC, "kpt_push.cu")) as f:
+        assert "cudaFuncAttributePreferredSharedMemoryCarveout" not in f.read()
