@@ -928,37 +928,6 @@ PowPlan make_pow_plan(const PushLaunch& L) {
     return plan;
 }
 
-// Blocks per SM (each one warp per sub-partition).
-//  * Every particle takes the same steps (dt_min = dt_max): the time is the
-//    number of full rounds of the population times the warps that share a
-//    sub-partition, over how well that many keep its FP64 pipe busy (0.80,
-//    0.92, 0.97, 1.0 of the best for 1 to 4 warps, measured at 400 000
-//    particles).  60 000 focused particles, 50 steps: 10.1 / 7.6 / 8.8 / 7.9
-//    ms with 1 / 2 / 3 / 4 blocks; 25 000: 5.2 / 3.4 / 4.4 / 5.5 ms.
-//  * Adaptive steps: the interval ends with its longest particles (6 840 of
-//    a mean of 1 095 substeps on the driver's uniform field), whose substeps
-//    take as long as the warps beside them allow: one block up to eight
-//    populations of its lanes, two beyond.  40 000 Parker particles: 111 /
-//    135 / 163 / 188 ms with 1 / 2 / 3 / 4 blocks, 131 072: 254 / 257 / 274 /
-//    300, 400 000: 693 / 639 / 659 / 685.
-int f64_blocks_per_sm(const PushLaunch& L, uint64_t lanes) {
-    if (L.settings.dt_min != L.settings.dt_max) {
-        return L.count <= 8 * lanes ? 1 : 2;
-    }
-    const double busy[4] = {0.80, 0.92, 0.97, 1.0};
-    int best = 1;
-    double least = 0.0;
-    for (int b = 1; b <= kF64Blocks; ++b) {
-        const uint64_t rounds = (L.count + lanes * b - 1) / (lanes * b);
-        const double cost = static_cast<double>(rounds * b) / busy[b - 1];
-        if (b == 1 || cost <= least) {
-            best = b;
-            least = cost;
-        }
-    }
-    return best;
-}
-
 template <bool FOCUSED, int SURR = 0>
 cudaError_t launch_push_f64(const PushLaunch& L, cudaStream_t stream) {
     PushParams P = make_push_params(L);
@@ -971,8 +940,8 @@ cudaError_t launch_push_f64(const PushLaunch& L, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     const uint64_t sm = static_cast<uint64_t>(L.sm_count);
     const uint64_t lanes = sm * threads;  // those of one block per SM
-    int per_sm = f64_blocks_per_sm(L, lanes);
-    if (L.blocks_per_sm > 0 && L.blocks_per_sm < per_sm) per_sm = L.blocks_per_sm;
+    const int per_sm = f64_blocks_per_sm(L.count, L.settings.dt_min == L.settings.dt_max, lanes,
+                                         kF64Blocks, L.blocks_per_sm);
     const uint64_t warps = sm * per_sm * (threads / 32);
     const uint64_t cap = (L.count + warps - 1) / warps;
     P.f64.simple = L.schedule == kScheduleSimple ? 1 : 0;

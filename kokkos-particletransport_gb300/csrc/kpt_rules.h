@@ -166,4 +166,40 @@ inline int batch_point_threads(uint64_t particles, bool fixed, int fit, int sm_c
     return longer * rounds(fit) < rounds(few) ? fit : few;
 }
 
+// ---- residency of the FP64 push
+
+// Blocks per SM (each one warp per sub-partition).
+//  * Every particle takes the same steps (dt_min = dt_max): the time is the
+//    number of full rounds of the population times the warps that share a
+//    sub-partition, over how well that many keep its FP64 pipe busy (0.80,
+//    0.92, 0.97, 1.0 of the best for 1 to 4 warps, measured at 400 000
+//    particles).  60 000 focused particles, 50 steps: 10.1 / 7.6 / 8.8 / 7.9
+//    ms with 1 / 2 / 3 / 4 blocks; 25 000: 5.2 / 3.4 / 4.4 / 5.5 ms.
+//  * Adaptive steps: the interval ends with its longest particles (6 840 of
+//    a mean of 1 095 substeps on the driver's uniform field), whose substeps
+//    take as long as the warps beside them allow: one block up to eight
+//    populations of its lanes, two beyond.  40 000 Parker particles: 111 /
+//    135 / 163 / 188 ms with 1 / 2 / 3 / 4 blocks, 131 072: 254 / 257 / 274 /
+//    300, 400 000: 693 / 639 / 659 / 685.
+// A request (blocks_per_sm of the push schedule, 0: none) is taken as it is,
+// up to the `most` that fit.
+inline int f64_blocks_per_sm(uint64_t particles, bool fixed, uint64_t lanes, int most,
+                             int requested) {
+    if (requested > 0) return requested < most ? requested : most;
+    if (!fixed) return particles <= 8 * lanes || most < 2 ? 1 : 2;
+    const double busy[4] = {0.80, 0.92, 0.97, 1.0};
+    int best = 1;
+    double least = 0.0;
+    for (int b = 1; b <= most; ++b) {
+        const uint64_t resident = lanes * static_cast<uint64_t>(b);
+        const uint64_t rounds = (particles + resident - 1) / resident;
+        const double cost = static_cast<double>(rounds) * b / busy[b < 4 ? b - 1 : 3];
+        if (b == 1 || cost <= least) {
+            best = b;
+            least = cost;
+        }
+    }
+    return best;
+}
+
 }  // namespace kpt

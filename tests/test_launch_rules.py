@@ -27,6 +27,10 @@ extern "C" int batch_records_pay(int focused, int fixed, int runs, double partic
 extern "C" int batch_point_threads(uint64_t particles, int fixed, int fit, int sms) {
     return kpt::batch_point_threads(particles, fixed != 0, fit, sms);
 }
+extern "C" int f64_blocks_per_sm(uint64_t particles, int fixed, uint64_t lanes, int most,
+                                 int requested) {
+    return kpt::f64_blocks_per_sm(particles, fixed != 0, lanes, most, requested);
+}
 """
 
 
@@ -43,6 +47,7 @@ def rules(tmp_path_factory):
     lib.records_pay.argtypes = [i32, i32, u64, u64, dbl, dbl, i32]
     lib.batch_records_pay.argtypes = [i32, i32, i32, dbl, dbl, dbl, i32]
     lib.batch_point_threads.argtypes = [u64, i32, i32, i32]
+    lib.f64_blocks_per_sm.argtypes = [u64, i32, u64, i32, i32]
     return lib
 
 
@@ -176,3 +181,22 @@ def test_no_launch_leaves_a_preference_on_its_kernel():
     whose launches want different ones would take each other's."""
     with open(os.path.join(CSRC, "kpt_push.cu")) as f:
         assert "cudaFuncAttributePreferredSharedMemoryCarveout" not in f.read()
+
+
+def test_residency_of_the_fp64_push(rules):
+    lanes = 128 * SMS
+    # the rule: adaptive one block up to eight populations of its lanes, two
+    # beyond; fixed 60 000 particles 10.1 / 7.6 / 8.8 / 7.9 ms, 25 000 5.2 / 3.4 /
+    # 4.4 / 5.5 ms with 1 / 2 / 3 / 4 blocks
+    assert rules.f64_blocks_per_sm(40000, 0, lanes, 4, 0) == 1
+    assert rules.f64_blocks_per_sm(400000, 0, lanes, 4, 0) == 2
+    assert rules.f64_blocks_per_sm(60000, 1, lanes, 4, 0) in (2, 4)
+    assert rules.f64_blocks_per_sm(25000, 1, lanes, 4, 0) == 2
+    # a request is honoured in both directions, up to what fits
+    for fixed in (0, 1):
+        for particles in (256, 40000, 400000):
+            for requested in (1, 2, 3, 4, 9):
+                assert rules.f64_blocks_per_sm(particles, fixed, lanes, 4, requested) == \
+                    min(requested, 4)
+                assert rules.f64_blocks_per_sm(particles, fixed, lanes, 2, requested) == \
+                    min(requested, 2)
