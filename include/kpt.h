@@ -247,7 +247,8 @@ int kpt_context_set_fp64_arithmetic(kpt_context* ctx, int mode);
  * points, or of fewer that fill the GPU for enough substeps to repay the
  * build; KPT_RECORDS_OFF never, KPT_RECORDS_ON for every refill-scheduled
  * mixed push.  Results are bit-identical either way.  The records are built
- * on the context's stream; a later push on another stream waits for them. */
+ * on the context's stream; a later push on another stream waits for them.  A
+ * push whose stream is being captured samples the point tables. */
 enum kpt_records_mode { KPT_RECORDS_AUTO = 0, KPT_RECORDS_OFF = 1, KPT_RECORDS_ON = 2 };
 int kpt_context_set_cell_records(kpt_context* ctx, int mode);
 

@@ -1112,8 +1112,9 @@ void fill_push_launch(const kpt_context* ctx, const kpt_particles* parts, const 
 
 // The cell records a mixed push samples (*out = nullptr: the point-major
 // tables), built on the context's stream when the table pair differs from
-// the one they hold.  Should the records not fit in device memory the push
-// samples the point tables, which gives the same values.
+// the one they hold.  Should the records not fit in device memory, or the
+// stream be captured, the push samples the point tables, which gives the same
+// values.
 int push_records(kpt_context* ctx, const kpt_particles* parts, const kpt_field* lower,
                  const kpt_field* upper, const kpt_settings* settings, const float** out) {
     *out = nullptr;
@@ -1128,6 +1129,10 @@ int push_records(kpt_context* ctx, const kpt_particles* parts, const kpt_field* 
                            settings->dt_max_rel, ctx->sm_count})) {
         return KPT_OK;
     }
+    // a captured push is replayed when the records may hold another pair
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    KPT_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return KPT_OK;
     if (ctx->records_lower != lower->serial || ctx->records_upper != upper->serial ||
         ctx->records.ptr == nullptr) {
         const bool focused = lower->kind == KPT_TABLE_FOCUSED21;
