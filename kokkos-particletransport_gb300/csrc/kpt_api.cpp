@@ -42,6 +42,7 @@ int set_error(int code, const std::string& message) {
     do {                                                                                \
         const cudaError_t kpt_err_ = (expr);                                            \
         if (kpt_err_ != cudaSuccess) {                                                  \
+            cudaGetLastError(); /* or the next launch's check would find it */          \
             return set_error(kpt_err_ == cudaErrorMemoryAllocation ? KPT_ERROR_OUT_OF_MEMORY \
                                                                    : KPT_ERROR_CUDA,    \
                              std::string(#expr) + ": " + cudaGetErrorString(kpt_err_)); \
@@ -2027,11 +2028,8 @@ int kpt_host_alloc(uint64_t bytes, void** out) {
     *out = nullptr;
     if (bytes == 0) return KPT_OK;
     const cudaError_t err = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
-    if (err != cudaSuccess) {
-        cudaGetLastError();  // the caller may go on without page-locked memory
-        *out = nullptr;
-        KPT_CUDA(err);
-    }
+    if (err != cudaSuccess) *out = nullptr;
+    KPT_CUDA(err);  // the caller may go on without page-locked memory
     return KPT_OK;
 }
 
