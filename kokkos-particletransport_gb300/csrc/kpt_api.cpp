@@ -593,35 +593,17 @@ int kpt_field_create(kpt_context* ctx, int nx, int ny, const double* x_edges,
 
 namespace {
 
-// b_device / v_device (optional): device addresses of mapped page-locked
-// cells the kernels read in place (NVLink-C2C / PCIe reads), so no staging
-// copy is made; b_cells / v_cells stay the host view used for validation.
-int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const double* y_edges,
-                 const double* b_cells, const double* v_cells, int table_kind, int precision,
-                 const double* b_device, const double* v_device, kpt_field** out) {
+int non_finite_cells() {
+    return set_error(KPT_ERROR_FORMAT, "AthenaFieldReader: non-finite field value.");
+}
+
+// field_create behind its argument checks.
+int field_build(kpt_context* ctx, int nx, int ny, const double* x_edges, const double* y_edges,
+                const double* b_cells, const double* v_cells, int table_kind, int precision,
+                const double* b_device, const double* v_device, kpt_field** out) {
     const bool device_readable = b_device != nullptr && v_device != nullptr;
-    KPT_REQUIRE(ctx != nullptr && out != nullptr, "kpt_field_create: NULL handle");
-    *out = nullptr;
-    KPT_REQUIRE(nx > 0 && ny > 0, "AthenaFieldReader: Athena binary dimensions must be positive.");
-    KPT_REQUIRE(x_edges && y_edges && b_cells && v_cells, "kpt_field_create: NULL array");
-    KPT_REQUIRE(table_kind == KPT_TABLE_PARKER16 || table_kind == KPT_TABLE_FOCUSED21,
-                "kpt_field_create: unknown table kind");
-    KPT_REQUIRE(precision == KPT_PRECISION_F64 || precision == KPT_PRECISION_MIXED,
-                "kpt_field_create: unknown precision");
     const size_t cells = static_cast<size_t>(nx) * static_cast<size_t>(ny);
-    // data read by kpt_field_data_read was checked on the reading thread; other
-    // cells are checked by the table kernel, and here only ahead of an earlier
-    // failure, which they come before
-    auto non_finite = [] {
-        return set_error(KPT_ERROR_FORMAT, "AthenaFieldReader: non-finite field value.");
-    };
-    auto failed = [&](int rc) {
-        for (size_t k = 0; !device_readable && k < 3 * cells; ++k) {
-            if (!std::isfinite(b_cells[k]) || !std::isfinite(v_cells[k])) return non_finite();
-        }
-        return rc;
-    };
-    if (int rc = activate(ctx)) return failed(rc);
+    if (int rc = activate(ctx)) return rc;
     struct FieldDeleter {
         void operator()(kpt_field* doomed) const { kpt_field_destroy(doomed); }
     };
@@ -643,7 +625,7 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
         std::vector<double> centers;
         std::vector<int> buckets;
         if (int rc = build_axis(counts[d], edges[d], f->grid.axis[d], centers, buckets)) {
-            return failed(rc);
+            return rc;
         }
         FixedAxisHost fixed = build_fixed_axis(f->grid.axis[d], centers);
         f->fixed[d] = fixed.axis;
@@ -712,9 +694,37 @@ int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const 
         return set_error(KPT_ERROR_CUDA,
                          std::string("kpt_field_create: ") + cudaGetErrorString(err));
     }
-    if (found != 0) return non_finite();
+    if (found != 0) return non_finite_cells();
     *out = f.release();
     return KPT_OK;
+}
+
+// b_device / v_device (optional): device addresses of mapped page-locked
+// cells the kernels read in place (NVLink-C2C / PCIe reads), so no staging
+// copy is made; b_cells / v_cells stay the host view used for validation.
+int field_create(kpt_context* ctx, int nx, int ny, const double* x_edges, const double* y_edges,
+                 const double* b_cells, const double* v_cells, int table_kind, int precision,
+                 const double* b_device, const double* v_device, kpt_field** out) {
+    KPT_REQUIRE(ctx != nullptr && out != nullptr, "kpt_field_create: NULL handle");
+    *out = nullptr;
+    KPT_REQUIRE(nx > 0 && ny > 0, "AthenaFieldReader: Athena binary dimensions must be positive.");
+    KPT_REQUIRE(x_edges && y_edges && b_cells && v_cells, "kpt_field_create: NULL array");
+    KPT_REQUIRE(table_kind == KPT_TABLE_PARKER16 || table_kind == KPT_TABLE_FOCUSED21,
+                "kpt_field_create: unknown table kind");
+    KPT_REQUIRE(precision == KPT_PRECISION_F64 || precision == KPT_PRECISION_MIXED,
+                "kpt_field_create: unknown precision");
+    const int rc = field_build(ctx, nx, ny, x_edges, y_edges, b_cells, v_cells, table_kind,
+                               precision, b_device, v_device, out);
+    // Data read by kpt_field_data_read was checked on the reading thread; other
+    // cells are checked by the table kernel.  A non-finite cell is reported
+    // ahead of any other failure, so a build that failed before the kernel's
+    // check looks for one here.
+    if (rc == KPT_OK || (b_device != nullptr && v_device != nullptr)) return rc;
+    const size_t values = 3 * static_cast<size_t>(nx) * static_cast<size_t>(ny);
+    for (size_t k = 0; k < values; ++k) {
+        if (!std::isfinite(b_cells[k]) || !std::isfinite(v_cells[k])) return non_finite_cells();
+    }
+    return rc;
 }
 
 }  // namespace
