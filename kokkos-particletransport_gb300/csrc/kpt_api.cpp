@@ -691,6 +691,7 @@ int field_build(kpt_context* ctx, int nx, int ny, const double* x_edges, const d
     }
     cudaFree(staging);
     if (err != cudaSuccess) {
+        cudaGetLastError();
         return set_error(KPT_ERROR_CUDA,
                          std::string("kpt_field_create: ") + cudaGetErrorString(err));
     }

@@ -40,7 +40,7 @@ def test_out_of_memory_leaves_no_error_behind(ctx, kpt, field):
 def test_bad_cell_comes_before_out_of_memory(ctx, kpt, field):
     torch = pytest.importorskip("torch")
     ctx.synchronize()
-    field.v[2, -1, -1] = np.inf
+    field.v[2, -1, -1] = float("inf")
     with _full_device(torch, 48 << 20):
         with pytest.raises(kpt.KptError, match="non-finite field value"):
             ctx.field(field, kpt.TABLE_FOCUSED21, kpt.PRECISION_F64)
