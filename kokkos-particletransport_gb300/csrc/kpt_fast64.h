@@ -14,10 +14,13 @@
  * the nearest multiple of 1/4, which the fixed-point draw gives exactly.
  *
  * Errors: at most 1.5 ulp each (2 ulp for the logarithm; sine and cosine 0.75
- * ulp of 1), tested on the host against
- * extended precision.  FP64 instructions: 3 (rcp), 5 (sqrt, rsqrt), 9 (cbrt),
- * 23 (log), 20 (sine and cosine) against 6, 9, 14, 18, 33 and 27 for CUDA's
- * functions.
+ * ulp of 1), tested against extended precision on the host and, with the
+ * hardware's seeds, on the device; measured there 0.50 (rcp, cbrt), 0.75
+ * (sqrt), 0.99 (rsqrt) and 0.87 (log).  The divisions and roots they stand for
+ * were correctly rounded, several to a quantity; the state after 40 steps is as
+ * far from its exact value with either (4.6e-16).  FP64 instructions: 3 (rcp),
+ * 5 (sqrt, rsqrt), 9 (cbrt), 23 (log), 20 (sine and cosine) against 6, 9, 14,
+ * 18, 33 and 27 for CUDA's functions.
  *
  * Operands outside [2^-100, 2^100] go through the C library's functions.
  * Host builds (the tests) seed with FP32 divisions and roots instead.
@@ -141,16 +144,21 @@ KPT_F64_FN double kpt_sqrt(double x) {
     return fma(t, e * fma(e, 0.375, 0.5), t);
 }
 
-/* x^(1/3) */
+/* x^(1/3).  x = m 2^(3k) with m in [1, 8): the seed's logarithm stays below 3,
+ * where FP32 holds it to 2^-22; of 2^100 it would keep 2^-18. */
 KPT_F64_FN double kpt_cbrt(double x) {
     if (!kpt_f64_seedable(x)) return cbrt(x);
-    const float xf = kpt_f64_seed(x);
-    const double y = kpt_f64_widen(kpt_seed_cbrt(xf));
-    const double d = fma(-(y * y), y, x); /* y y exact: y has 24 bits */
-    const double r0 = kpt_f64_widen(kpt_seed_rcp(xf));
-    const double r = fma(r0, fma(-x, r0, 1.0), r0);
+    const uint64_t bits = kpt_f64_to_bits(x);
+    const int k = ((int)(bits >> 52) - (1023 - 102)) / 3 - 34; /* floor(exponent / 3) */
+    const double m = kpt_f64_from_bits(bits - ((uint64_t)(int64_t)(3 * k) << 52));
+    const float mf = kpt_f64_seed(m);
+    const double y = kpt_f64_widen(kpt_seed_cbrt(mf));
+    const double d = fma(-(y * y), y, m); /* y y exact: y has 24 bits */
+    const double r0 = kpt_f64_widen(kpt_seed_rcp(mf));
+    const double r = fma(r0, fma(-m, r0, 1.0), r0);
     const double e = d * r;
-    return fma(y, e * fma(e, 2.0 / 9.0, 1.0 / 3.0), y);
+    const double root = fma(y, e * fma(e, 2.0 / 9.0, 1.0 / 3.0), y);
+    return kpt_f64_from_bits(kpt_f64_to_bits(root) + ((uint64_t)(int64_t)k << 52));
 }
 
 /* ln u for a normal u in (0, 1] */
