@@ -14,6 +14,7 @@ available.
 from __future__ import annotations
 
 import ctypes
+import mmap
 import os
 import threading
 import weakref
@@ -373,14 +374,13 @@ class _PinnedBlock:
 
 
 class _PinnedPool:
-    """Page-locked host memory for downloads.
+    """Page-locked host memory for downloads that ask for it (pinned=True).
 
-    A download into fresh pageable arrays spends most of its time in the
-    operating system (first touch of every page by the copy, unmapping of the
-    previous result); blocks that are kept page-locked take the copy at link
-    speed.  250 mixed library steps of 400 000 particles and their download
-    (50 MB), one pass after another: 50.9 -> 33.7 ms; 40 steps of 300 000 in
-    FP64: 18.7 -> 7.9 ms.
+    For a program that downloads again and again and drops each result: the
+    copy then runs at link speed into pages that are there already.  14 arrays
+    of 400 000 particles (40 MB): 0.27 ms, 2.1 ms into new arrays; the first
+    download of a size, and one whose predecessors are all kept, locks a new
+    block and takes 1.8 ms like a new array's.
     At most LIMIT bytes are page-locked, in use and idle together (beyond that
     a download uses ordinary memory); idle blocks are freed with the last
     Context.  Safe for several threads: a block is handed out once at a time,
@@ -411,8 +411,9 @@ class _PinnedPool:
             self._total -= size
             load_library().kpt_host_free(ptr)
 
-    def take(self, nbytes: int) -> Optional[np.ndarray]:
-        """nbytes of page-locked memory as a uint8 array, or None."""
+    def take(self, nbytes: int, select=None) -> Optional[np.ndarray]:
+        """nbytes of page-locked memory as a uint8 array, or None.  A new block
+        is locked with the device current that select() makes so."""
         if nbytes < self.SMALLEST or nbytes > self.LIMIT:
             return None
         size = (nbytes + (1 << 20) - 1) >> 20 << 20
@@ -424,6 +425,8 @@ class _PinnedPool:
             self._trim(self.LIMIT - size)
             if self._total + size > self.LIMIT:
                 return None
+            if select is not None:
+                select()
             out = ctypes.c_void_p()
             if load_library().kpt_host_alloc(size, ctypes.byref(out)) != 0:
                 return None
@@ -440,13 +443,23 @@ class _PinnedPool:
 _PINNED = _PinnedPool()
 
 
-def _host_arrays(shapes: Dict[str, tuple]) -> Dict[str, np.ndarray]:
-    """Uninitialised host arrays {name: (length, dtype)} to download into: one
-    page-locked block if the pool has room, ordinary memory otherwise."""
+def _new_array(n: int, dtype) -> np.ndarray:
+    """An uninitialised array whose pages are there before the device writes
+    them: a download into untouched pages waits for each of them (14 arrays of
+    400 000 particles: 3.5 ms, 33 ms into np.zeros, 2.1 ms touched)."""
+    a = np.empty(n, dtype=dtype)
+    a.view(np.uint8)[::mmap.PAGESIZE] = 0
+    return a
+
+
+def _host_arrays(shapes: Dict[str, tuple], ctx: Optional["Context"] = None) \
+        -> Dict[str, np.ndarray]:
+    """Uninitialised host arrays {name: (length, dtype)} to download into: new
+    ones, or with ctx views of one page-locked block if the pool has room."""
     sizes = {k: (int(n) * np.dtype(t).itemsize + 63) // 64 * 64 for k, (n, t) in shapes.items()}
-    block = _PINNED.take(sum(sizes.values()))
+    block = None if ctx is None else _PINNED.take(sum(sizes.values()), ctx.synchronize)
     if block is None:
-        return {k: np.empty(n, dtype=t) for k, (n, t) in shapes.items()}
+        return {k: _new_array(n, t) for k, (n, t) in shapes.items()}
     out, at = {}, 0
     for k, (n, t) in shapes.items():
         out[k] = block[at:at + int(n) * np.dtype(t).itemsize].view(t)
@@ -1095,12 +1108,16 @@ class ParticleSystem(_Handle):
             conv[k] = np.ascontiguousarray(data[k][:n], dtype=np.int32)
         _check(self.ctx.lib.kpt_system_upload(self.handle, n, ctypes.byref(self._arrays(conv))))
 
-    def download(self, n: Optional[int] = None) -> Dict[str, np.ndarray]:
+    def download(self, n: Optional[int] = None, pinned: bool = False) -> Dict[str, np.ndarray]:
+        """The first n slots (default: all), into new arrays; with pinned, into
+        views of one page-locked block of the process's pool, for programs that
+        drop each result before the next: the arrays then do not own their
+        memory (no resize in place), and one that is kept holds the block."""
         n = self.capacity if n is None else int(n)
         shapes = {"id": (n, np.uint64)}
         shapes.update({k: (n, np.float64) for k in SYSTEM_DOUBLE_FIELDS})
         shapes.update({k: (n, np.int32) for k in SYSTEM_INT_FIELDS})
-        out = _host_arrays(shapes)
+        out = _host_arrays(shapes, self.ctx if pinned else None)
         _check(self.ctx.lib.kpt_system_download(self.handle, n, ctypes.byref(self._arrays(out))))
         return out
 
@@ -1393,14 +1410,16 @@ class ParticleStorage:
                                                  *[_ptr(conv[n]) for n in PARTICLE_FIELDS]))
 
     def download(self, count: Optional[int] = None,
-                 out: Optional[Dict[str, np.ndarray]] = None) -> Dict[str, np.ndarray]:
-        """The first `count` particles (default: all stored), into new arrays or
-        into `out` (contiguous arrays of the field dtypes, at least count long,
-        e.g. views of pinned host memory)."""
+                 out: Optional[Dict[str, np.ndarray]] = None,
+                 pinned: bool = False) -> Dict[str, np.ndarray]:
+        """The first `count` particles (default: all stored), into new arrays
+        (pinned: page-locked ones, see ParticleSystem.download) or into `out`
+        (contiguous arrays of the field dtypes, at least count long, e.g. views
+        of pinned host memory)."""
         n = self.count if count is None else int(count)
         if out is None:
             out = _host_arrays({name: (n, np.int32 if name in ("status", "level") else np.float64)
-                                for name in PARTICLE_FIELDS})
+                                for name in PARTICLE_FIELDS}, self.ctx if pinned else None)
         for name in PARTICLE_FIELDS:
             dtype = np.int32 if name in ("status", "level") else np.float64
             a = out[name]
