@@ -750,7 +750,10 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kLibMixedThreads : 256,
             continue;
         }
 #pragma unroll
-        for (int k = 0; k < kLibTermCount; ++k) terms[k * L.term_stride + i] = row[k];
+        for (int k = 0; k < kLibTermCount; ++k) {
+            if (sizeof(T) == 4 && k == kMomentum) continue;  // its base is the FP64 state
+            terms[k * L.term_stride + i] = row[k];
+        }
         local = dt < local ? dt : local;
     }
     finish_terms(local, L);
@@ -849,6 +852,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? kLibMixedThreads : 256)
         T t[kLibTermCount];
 #pragma unroll
         for (int k = 0; k < kLibTermCount; ++k) {
+            if (sizeof(T) == 4 && k == kMomentum) continue;
             t[k] = reinterpret_cast<const T*>(L.terms)[k * L.term_stride + i];
         }
         if constexpr (sizeof(T) == 8) {
