@@ -2,7 +2,8 @@
 // (21 components), plain FP64 or mixed precision.
 //
 // The per-substep physics restates reference src/main.cpp:1131-1306 (Parker)
-// and :1384-1733 (focused) once, templated on the arithmetic type.
+// and :1384-1733 (focused) once per arithmetic: in FP32 here (physics,
+// increments, advance_mixed), in FP64 as tasks of a warp in kpt_push_f64.cuh.
 //
 // GB300 notes.  FP64 issues at a small fraction of the FP32 rate on this
 // part, so the two paths differ in how they carry particle state:
@@ -58,11 +59,8 @@ constexpr double kSqrt3 = 1.7320508075688772935;
 #define KPT_FAST_SQRT 1
 #endif
 
-template <typename T>
-struct Num;
-
-template <>
-struct Num<float> {
+// FP32 operations of the mixed path.
+struct Num {
     // x^y for x >= 0 through the hardware exp2/log2 approximations.
     static __device__ __forceinline__ float pow(float a, float b) {
         return exp2f(b * __log2f(a));
@@ -381,30 +379,30 @@ __device__ __forceinline__ void sample_coefficients(const Grid& g, const T* __re
 // ------------------------------------------------------------- physics
 // Slab quasi-linear pitch-angle scattering (LegencyModel.hpp:557-645):
 // D_mumu and dD_mumu/dmu at one (mu, Omega, v).
-template <typename T>
-__device__ __forceinline__ void qlt_scattering(T mu, T omega, T speed, const Consts<T>& s,
-                                               T& dmumu, T& dmumu_dmu) {
-    using N = Num<T>;
-    dmumu = T(0);
-    dmumu_dmu = T(0);
-    const T one_minus_mu2 = T(1) - mu * mu;
-    if (one_minus_mu2 <= T(0)) {
+__device__ __forceinline__ void qlt_scattering(float mu, float omega, float speed,
+                                               const Consts<float>& s, float& dmumu,
+                                               float& dmumu_dmu) {
+    using N = Num;
+    dmumu = 0.0f;
+    dmumu_dmu = 0.0f;
+    const float one_minus_mu2 = 1.0f - mu * mu;
+    if (one_minus_mu2 <= 0.0f) {
         return;
     }
-    const T gk = s.qlt_gk;
-    const T reg = N::abs(mu) + s.qlt_h0;
-    const T xi = N::div(omega * s.qlt_lc, speed);
-    const T reg_gk1 = N::pow(reg, gk - T(1));
-    const T denominator = N::pow(reg, gk) + N::pow(xi, gk);
-    const T prefactor = static_cast<T>(0.25 * 3.141592653589793238462643383279502884) * omega *
-                        s.qlt_sigma2 * s.qlt_norm;
+    const float gk = s.qlt_gk;
+    const float reg = N::abs(mu) + s.qlt_h0;
+    const float xi = N::div(omega * s.qlt_lc, speed);
+    const float reg_gk1 = N::pow(reg, gk - 1.0f);
+    const float denominator = N::pow(reg, gk) + N::pow(xi, gk);
+    const float prefactor = static_cast<float>(0.25 * 3.141592653589793238462643383279502884) *
+                            omega * s.qlt_sigma2 * s.qlt_norm;
     dmumu = N::div(prefactor * one_minus_mu2 * xi * reg_gk1, denominator);
-    if (dmumu == T(0) || mu == T(0)) {
+    if (dmumu == 0.0f || mu == 0.0f) {
         return;
     }
-    const T sign_mu = mu > T(0) ? T(1) : T(-1);
-    const T shape = sign_mu * (N::div(gk - T(1), reg) - N::div(gk * reg_gk1, denominator));
-    const T endpoint = N::div(T(-2) * mu, one_minus_mu2);
+    const float sign_mu = mu > 0.0f ? 1.0f : -1.0f;
+    const float shape = sign_mu * (N::div(gk - 1.0f, reg) - N::div(gk * reg_gk1, denominator));
+    const float endpoint = N::div(-2.0f * mu, one_minus_mu2);
     dmumu_dmu = dmumu * (endpoint + shape);
 }
 
@@ -414,25 +412,25 @@ struct Served {
     float kpara, duu, duu_du;
 };
 
-template <typename T>
 struct Rates {
-    T dx_dt, dy_dt, dp_dt, dmu_dt, duu;
-    T skperp, skpara_perp, ib, bx, by, bz;
-    T pitch_mu;
-    T dt;        // limiter result (valid when !fixed_dt)
+    float dx_dt, dy_dt, dp_dt, dmu_dt, duu;
+    float skperp, skpara_perp, ib, bx, by, bz;
+    float pitch_mu;
+    float dt;        // limiter result (valid when !fixed_dt)
     bool fixed_dt;
 };
 
 // Coefficients, drift, dp/dt, dmu/dt and the step-size limiters of one
 // substep (src/main.cpp:1167-1257 Parker, :1421-1630 focused).  Returns
 // false where the reference sets status 2.
-template <typename T, bool FOCUSED, bool SURR = false>
-__device__ __forceinline__ bool physics(const T* c, T p, T pitch_mu, const Consts<T>& s,
-                                        Rates<T>& r, const Served* served = nullptr) {
-    using N = Num<T>;
-    T vx, vy, bx, by, bz, b, dvx_dx, dvy_dy, dbx_dx, dbx_dy, dby_dx, dby_dy, dbz_dx, dbz_dy,
+template <bool FOCUSED, bool SURR = false>
+__device__ __forceinline__ bool physics(const float* c, float p, float pitch_mu,
+                                        const Consts<float>& s, Rates& r,
+                                        const Served* served = nullptr) {
+    using N = Num;
+    float vx, vy, bx, by, bz, b, dvx_dx, dvy_dy, dbx_dx, dbx_dy, dby_dx, dby_dy, dbz_dx, dbz_dy,
         db_dx, db_dy;
-    T dvx_dy = 0, dvy_dx = 0, dvz_dx = 0, dvz_dy = 0;
+    float dvx_dy = 0, dvy_dx = 0, dvz_dx = 0, dvz_dy = 0;
     if (FOCUSED) {
         vx = c[0]; vy = c[1]; bx = c[3]; by = c[4]; bz = c[5]; b = c[6];
         dvx_dx = c[7]; dvx_dy = c[8]; dvy_dx = c[9]; dvy_dy = c[10]; dvz_dx = c[11];
@@ -443,174 +441,177 @@ __device__ __forceinline__ bool physics(const T* c, T p, T pitch_mu, const Const
         dvy_dy = c[7]; dbx_dx = c[8]; dbx_dy = c[9]; dby_dx = c[10]; dby_dy = c[11];
         dbz_dx = c[12]; dbz_dy = c[13]; db_dx = c[14]; db_dy = c[15];
     }
-    if (!N::finite(p) || p <= T(0) || !N::finite(b) || b <= T(0)) {
+    if (!N::finite(p) || p <= 0.0f || !N::finite(b) || b <= 0.0f) {
         return false;
     }
-    const T p0 = s.p0;
-    const T gamma = s.gamma_turb;
-    const T ib = N::div(T(1), b);
-    const T ib2 = ib * ib;
-    const T ib3 = ib2 * ib;
+    const float p0 = s.p0;
+    const float gamma = s.gamma_turb;
+    const float ib = N::div(1.0f, b);
+    const float ib2 = ib * ib;
+    const float ib3 = ib2 * ib;
 
-    T kpara;
+    float kpara;
     if (SURR && served->use) {
         kpara = served->kpara;
     } else {
-        T knorm_para = T(1);
+        float knorm_para = 1.0f;
         if (s.magnetic_dependency == 1) {
-            knorm_para *= N::pow(b, gamma - T(2));
+            knorm_para *= N::pow(b, gamma - 2.0f);
         }
-        T knorm = knorm_para;
+        float knorm = knorm_para;
         if (s.momentum_dependency == 1) {
             knorm *= N::pow(N::div(p, p0), s.pindex);
         }
         kpara = s.kpara0 * knorm;
     }
-    const T kperp = kpara * s.kperp_over_kpara;
-    if (!N::finite(kpara) || kpara <= T(0) || !N::finite(kperp) || kperp < T(0)) {
+    const float kperp = kpara * s.kperp_over_kpara;
+    if (!N::finite(kpara) || kpara <= 0.0f || !N::finite(kperp) || kperp < 0.0f) {
         return false;
     }
-    const T skpara = N::sqrt(T(2) * kpara);
-    const T skperp = N::sqrt(T(2) * kperp);
-    T skpara_perp;
+    const float skpara = N::sqrt(2.0f * kpara);
+    const float skperp = N::sqrt(2.0f * kperp);
+    float skpara_perp;
     if (FOCUSED) {
-        skpara_perp = kpara > kperp ? N::sqrt(T(2) * (kpara - kperp)) : T(0);
+        skpara_perp = kpara > kperp ? N::sqrt(2.0f * (kpara - kperp)) : 0.0f;
     } else {
-        skpara_perp = N::sqrt(T(2) * (kpara - kperp));
+        skpara_perp = N::sqrt(2.0f * (kpara - kperp));
     }
-    const T kpp = FOCUSED ? -kperp : kpara - kperp;
+    const float kpp = FOCUSED ? -kperp : kpara - kperp;
 
-    T dkdx = T(0);
-    T dkdy = T(0);
+    float dkdx = 0.0f;
+    float dkdy = 0.0f;
     if (s.magnetic_dependency == 1) {
-        const T magnetic_exponent = gamma - T(2);
+        const float magnetic_exponent = gamma - 2.0f;
         dkdx = db_dx * ib * magnetic_exponent;
         dkdy = db_dy * ib * magnetic_exponent;
     }
-    const T dkxx_dx = kperp * dkdx + kpp * dkdx * bx * bx * ib2 +
-                      T(2) * kpp * bx * (dbx_dx * b - bx * db_dx) * ib3;
-    const T dkyy_dy = kperp * dkdy + kpp * dkdy * by * by * ib2 +
-                      T(2) * kpp * by * (dby_dy * b - by * db_dy) * ib3;
-    const T dkxy_dx = kpp * dkdx * bx * by * ib2 +
-                      kpp * ((dbx_dx * by + bx * dby_dx) * ib2 - T(2) * bx * by * db_dx * ib3);
-    const T dkxy_dy = kpp * dkdy * bx * by * ib2 +
-                      kpp * ((dbx_dy * by + bx * dby_dy) * ib2 - T(2) * bx * by * db_dy * ib3);
+    const float dkxx_dx = kperp * dkdx + kpp * dkdx * bx * bx * ib2 +
+                          2.0f * kpp * bx * (dbx_dx * b - bx * db_dx) * ib3;
+    const float dkyy_dy = kperp * dkdy + kpp * dkdy * by * by * ib2 +
+                          2.0f * kpp * by * (dby_dy * b - by * db_dy) * ib3;
+    const float dkxy_dx = kpp * dkdx * bx * by * ib2 +
+                          kpp * ((dbx_dx * by + bx * dby_dx) * ib2 - 2.0f * bx * by * db_dx * ib3);
+    const float dkxy_dy = kpp * dkdy * bx * by * ib2 +
+                          kpp * ((dbx_dy * by + bx * dby_dy) * ib2 - 2.0f * bx * by * db_dy * ib3);
 
-    const T d1 = s.drift_param1;
-    const T d2 = s.drift_param2;
-    const T drift_denominator =
+    const float d1 = s.drift_param1;
+    const float d2 = s.drift_param2;
+    const float drift_denominator =
         N::sqrt(square(N::div(d1 * p0, p)) + square(N::div(d2 * p0 * p0, p * p)));
 
-    T dx_dt, dy_dt, dp_dt;
-    T dmu_dt = T(0), duu = T(0);
+    float dx_dt, dy_dt, dp_dt;
+    float dmu_dt = 0.0f, duu = 0.0f;
     if (FOCUSED) {
         pitch_mu = clamp_mu(pitch_mu, s.mu_max);
-        const T mu2 = pitch_mu * pitch_mu;
-        const T muf1 = T(0.5) * (T(1) - mu2);
-        const T muf2 = T(0.5) * (T(3) * mu2 - T(1));
-        const T kx = bx * dbx_dx + by * dbx_dy;
-        const T ky = bx * dby_dx + by * dby_dy;
-        const T kz = bx * dbz_dx + by * dbz_dy;
-        const T bdot_curvb = bx * dbz_dy - by * dbz_dx + bz * (dby_dx - dbx_dy);
-        const T vdp = N::div(N::div(T(1), s.charge), drift_denominator);
-        const T vdx = vdp * (muf1 * (-bz * db_dy) * ib2 + mu2 * (by * kz - bz * ky) * ib3 +
-                             muf1 * bx * bdot_curvb * ib3);
-        const T vdy = vdp * (muf1 * (bz * db_dx) * ib2 + mu2 * (bz * kx - bx * kz) * ib3 +
-                             muf1 * by * bdot_curvb * ib3);
-        const T speed = N::div(s.particle_v0 * p, p0);
-        if (!N::finite(speed) || speed <= T(0)) {
+        const float mu2 = pitch_mu * pitch_mu;
+        const float muf1 = 0.5f * (1.0f - mu2);
+        const float muf2 = 0.5f * (3.0f * mu2 - 1.0f);
+        const float kx = bx * dbx_dx + by * dbx_dy;
+        const float ky = bx * dby_dx + by * dby_dy;
+        const float kz = bx * dbz_dx + by * dbz_dy;
+        const float bdot_curvb = bx * dbz_dy - by * dbz_dx + bz * (dby_dx - dbx_dy);
+        const float vdp = N::div(N::div(1.0f, s.charge), drift_denominator);
+        const float vdx = vdp * (muf1 * (-bz * db_dy) * ib2 + mu2 * (by * kz - bz * ky) * ib3 +
+                                 muf1 * bx * bdot_curvb * ib3);
+        const float vdy = vdp * (muf1 * (bz * db_dx) * ib2 + mu2 * (bz * kx - bx * kz) * ib3 +
+                                 muf1 * by * bdot_curvb * ib3);
+        const float speed = N::div(s.particle_v0 * p, p0);
+        if (!N::finite(speed) || speed <= 0.0f) {
             return false;
         }
-        const T v_parallel_over_b = speed * pitch_mu * ib;
+        const float v_parallel_over_b = speed * pitch_mu * ib;
         dx_dt = vx + vdx + v_parallel_over_b * bx + dkxx_dx + dkxy_dy;
         dy_dt = vy + vdy + v_parallel_over_b * by + dkxy_dx + dkyy_dy;
 
-        const T divv = dvx_dx + dvy_dy;
-        const T bb_gradv = (bx * (bx * dvx_dx + by * dvx_dy) + by * (bx * dvy_dx + by * dvy_dy) +
-                            bz * (bx * dvz_dx + by * dvz_dy)) *
-                           ib2;
-        const T bv_gradv = (bx * (vx * dvx_dx + vy * dvx_dy) + by * (vx * dvy_dx + vy * dvy_dy) +
-                            bz * (vx * dvz_dx + vy * dvz_dy)) *
-                           ib;
-        const T acc_rate = -(muf1 * divv + muf2 * bb_gradv + N::div(pitch_mu * bv_gradv, speed));
+        const float divv = dvx_dx + dvy_dy;
+        const float bb_gradv =
+            (bx * (bx * dvx_dx + by * dvx_dy) + by * (bx * dvy_dx + by * dvy_dy) +
+             bz * (bx * dvz_dx + by * dvz_dy)) *
+            ib2;
+        const float bv_gradv =
+            (bx * (vx * dvx_dx + vy * dvx_dy) + by * (vx * dvy_dx + vy * dvy_dy) +
+             bz * (vx * dvz_dx + vy * dvz_dy)) *
+            ib;
+        const float acc_rate =
+            -(muf1 * divv + muf2 * bb_gradv + N::div(pitch_mu * bv_gradv, speed));
         dp_dt = p * acc_rate;
 
-        const T div_bnorm = -(bx * db_dx + by * db_dy) * ib2;
-        dmu_dt = speed * div_bnorm + pitch_mu * divv - T(3) * pitch_mu * bb_gradv -
-                 N::div(T(2) * bv_gradv, speed);
-        dmu_dt *= T(0.5) * (T(1) - mu2);
-        T duu_du = T(0);
+        const float div_bnorm = -(bx * db_dx + by * db_dy) * ib2;
+        dmu_dt = speed * div_bnorm + pitch_mu * divv - 3.0f * pitch_mu * bb_gradv -
+                 N::div(2.0f * bv_gradv, speed);
+        dmu_dt *= 0.5f * (1.0f - mu2);
+        float duu_du = 0.0f;
         if (SURR && served->use) {
             duu = served->duu;
             duu_du = served->duu_du;
         } else if (s.closure != 0) {
             // slab QLT closure (extension): Omega = Omega_0 |B| / gamma
-            const T omega = N::div(s.qlt_omega0 * b, N::sqrt(T(1) + p * p));
-            qlt_scattering<T>(pitch_mu, omega, speed, s, duu, duu_du);
+            const float omega = N::div(s.qlt_omega0 * b, N::sqrt(1.0f + p * p));
+            qlt_scattering(pitch_mu, omega, speed, s, duu, duu_du);
         } else {
             // the driver's reduced closure (src/main.cpp:1551-1589)
-            const T abs_mu = N::abs(pitch_mu);
-            const T dtmp = N::pow(abs_mu, gamma - T(1)) + s.h0;
-            const T duu0 = s.duu0;
-            duu = duu0 * (T(1) - mu2) * dtmp;
-            if (pitch_mu > T(0)) {
-                duu_du = duu0 * (T(-2) * pitch_mu * dtmp +
-                                 (T(1) - mu2) * N::pow(abs_mu, gamma - T(2)));
-            } else if (pitch_mu < T(0)) {
-                duu_du = duu0 * (T(-2) * pitch_mu * dtmp -
-                                 (T(1) - mu2) * N::pow(abs_mu, gamma - T(2)));
+            const float abs_mu = N::abs(pitch_mu);
+            const float dtmp = N::pow(abs_mu, gamma - 1.0f) + s.h0;
+            const float duu0 = s.duu0;
+            duu = duu0 * (1.0f - mu2) * dtmp;
+            if (pitch_mu > 0.0f) {
+                duu_du = duu0 * (-2.0f * pitch_mu * dtmp +
+                                 (1.0f - mu2) * N::pow(abs_mu, gamma - 2.0f));
+            } else if (pitch_mu < 0.0f) {
+                duu_du = duu0 * (-2.0f * pitch_mu * dtmp -
+                                 (1.0f - mu2) * N::pow(abs_mu, gamma - 2.0f));
             }
-            T duu_norm = T(1);
+            float duu_norm = 1.0f;
             if (s.magnetic_dependency == 1) {
-                duu_norm *= N::pow(b, T(2) - gamma);
+                duu_norm *= N::pow(b, 2.0f - gamma);
             }
             if (s.momentum_dependency == 1) {
-                duu_norm *= N::pow(N::div(p, p0), gamma - T(1));
+                duu_norm *= N::pow(N::div(p, p0), gamma - 1.0f);
             }
             duu *= duu_norm;
             duu_du *= duu_norm;
         }
         dmu_dt += duu_du;
-        if (!N::finite(dmu_dt) || !N::finite(duu) || duu < T(0)) {
+        if (!N::finite(dmu_dt) || !N::finite(duu) || duu < 0.0f) {
             return false;
         }
     } else {
-        const T vdp = N::div(N::div(T(1), T(3) * s.charge), drift_denominator);
-        const T vdx = vdp * (dbz_dy * ib2 - T(2) * bz * db_dy * ib3);
-        const T vdy = vdp * (-dbz_dx * ib2 + T(2) * bz * db_dx * ib3);
+        const float vdp = N::div(N::div(1.0f, 3.0f * s.charge), drift_denominator);
+        const float vdx = vdp * (dbz_dy * ib2 - 2.0f * bz * db_dy * ib3);
+        const float vdy = vdp * (-dbz_dx * ib2 + 2.0f * bz * db_dx * ib3);
         dx_dt = vx + vdx + dkxx_dx + dkxy_dy;
         dy_dt = vy + vdy + dkxy_dx + dkyy_dy;
-        const T divv = dvx_dx + dvy_dy;
-        dp_dt = N::div(-p * divv, T(3));
+        const float divv = dvx_dx + dvy_dy;
+        dp_dt = N::div(-p * divv, 3.0f);
     }
 
     // Step-size limiters (src/main.cpp:1243-1257, :1596-1650).
-    const T dxs = s.dx;
-    const T dys = s.dy;
+    const float dxs = s.dx;
+    const float dys = s.dy;
     r.fixed_dt = false;
-    r.dt = T(0);
+    r.dt = 0.0f;
     if (FOCUSED) {
-        const T diffusion_scale = skperp > T(0) ? skperp : skpara;
-        if (dx_dt != T(0) && dy_dt != T(0) && dp_dt != T(0) && dmu_dt != T(0) &&
-            diffusion_scale > T(0)) {
-            T dt = min_positive(square(N::div(T(0.5) * dxs, diffusion_scale)),
-                                square(N::div(T(0.5) * dys, diffusion_scale)));
+        const float diffusion_scale = skperp > 0.0f ? skperp : skpara;
+        if (dx_dt != 0.0f && dy_dt != 0.0f && dp_dt != 0.0f && dmu_dt != 0.0f &&
+            diffusion_scale > 0.0f) {
+            float dt = min_positive(square(N::div(0.5f * dxs, diffusion_scale)),
+                                    square(N::div(0.5f * dys, diffusion_scale)));
             dt = min_positive(dt, square(N::div(diffusion_scale, dx_dt)));
             dt = min_positive(dt, square(N::div(diffusion_scale, dy_dt)));
-            dt = min_positive(dt, N::div(T(0.1) * p, N::abs(dp_dt)));
-            dt = min_positive(dt, N::div(T(0.1), N::abs(dmu_dt)));
-            dt = min_positive(dt, N::div(T(2) * duu, square(dmu_dt)));
+            dt = min_positive(dt, N::div(0.1f * p, N::abs(dp_dt)));
+            dt = min_positive(dt, N::div(0.1f, N::abs(dmu_dt)));
+            dt = min_positive(dt, N::div(2.0f * duu, square(dmu_dt)));
             r.dt = dt;
         } else {
             r.fixed_dt = true;
         }
-    } else if (dx_dt != T(0) && dy_dt != T(0) && dp_dt != T(0)) {
-        const T advection_scale = skperp > T(0) ? skperp : skpara;
-        T dt = min_positive(square(N::div(T(0.5) * dxs, skpara)),
-                            square(N::div(T(0.5) * dys, skpara)));
+    } else if (dx_dt != 0.0f && dy_dt != 0.0f && dp_dt != 0.0f) {
+        const float advection_scale = skperp > 0.0f ? skperp : skpara;
+        float dt = min_positive(square(N::div(0.5f * dxs, skpara)),
+                                square(N::div(0.5f * dys, skpara)));
         dt = min_positive(dt, square(N::div(advection_scale, dx_dt)));
         dt = min_positive(dt, square(N::div(advection_scale, dy_dt)));
-        dt = min_positive(dt, N::div(T(0.1) * p, N::abs(dp_dt)));
+        dt = min_positive(dt, N::div(0.1f * p, N::abs(dp_dt)));
         r.dt = dt;
     } else {
         r.fixed_dt = true;
@@ -639,36 +640,36 @@ struct Draws {
 
 // Displacements and the new pitch cosine from the four draws of a substep
 // (src/main.cpp:1280-1291 Parker, :1660-1702 focused).
-template <typename T, bool FOCUSED>
-__device__ __forceinline__ void increments(const Rates<T>& r, T dt, const Draws& d,
-                                           const Consts<T>& s, T& delta_x, T& delta_y,
-                                           T& new_mu) {
-    using N = Num<T>;
-    const T sdt = N::sqrt(dt);
+template <bool FOCUSED>
+__device__ __forceinline__ void increments(const Rates& r, float dt, const Draws& d,
+                                           const Consts<float>& s, float& delta_x, float& delta_y,
+                                           float& new_mu) {
+    using N = Num;
+    const float sdt = N::sqrt(dt);
     if (FOCUSED) {
-        const T ran1 = N::noise(d.first);
-        const T ran2 = N::noise(d.second);
-        const T pitch_random = N::noise(d.third);
-        const T bxn = r.bx * r.ib;
-        const T byn = r.by * r.ib;
-        const T bzn = r.bz * r.ib;
-        const T bxy_norm = N::sqrt(bxn * bxn + byn * byn);
-        T stochastic_x = T(0);
-        T stochastic_y = T(0);
-        if (bxy_norm > T(0)) {
-            const T ibxy_norm = N::div(T(1), bxy_norm);
+        const float ran1 = N::noise(d.first);
+        const float ran2 = N::noise(d.second);
+        const float pitch_random = N::noise(d.third);
+        const float bxn = r.bx * r.ib;
+        const float byn = r.by * r.ib;
+        const float bzn = r.bz * r.ib;
+        const float bxy_norm = N::sqrt(bxn * bxn + byn * byn);
+        float stochastic_x = 0.0f;
+        float stochastic_y = 0.0f;
+        if (bxy_norm > 0.0f) {
+            const float ibxy_norm = N::div(1.0f, bxy_norm);
             // (-by, +bx) on ran2 as written in src/main.cpp:1682-1687.
             stochastic_x = r.skperp * ibxy_norm * sdt * (-bxn * bzn * ran1 - r.by * ran2);
             stochastic_y = r.skperp * ibxy_norm * sdt * (-byn * bzn * ran1 + r.bx * ran2);
         }
         delta_x = r.dx_dt * dt + stochastic_x;
         delta_y = r.dy_dt * dt + stochastic_y;
-        new_mu = clamp_mu(r.pitch_mu + r.dmu_dt * dt + pitch_random * N::sqrt(T(2) * r.duu) * sdt,
+        new_mu = clamp_mu(r.pitch_mu + r.dmu_dt * dt + pitch_random * N::sqrt(2.0f * r.duu) * sdt,
                           s.mu_max);
     } else {
-        const T ran1 = N::noise(d.first);
-        const T ran2 = N::noise(d.second);
-        const T ran3 = N::noise(d.third);
+        const float ran1 = N::noise(d.first);
+        const float ran2 = N::noise(d.second);
+        const float ran3 = N::noise(d.third);
         delta_x = r.dx_dt * dt + ran1 * r.skperp * sdt + ran3 * r.skpara_perp * sdt * r.bx * r.ib;
         delta_y = r.dy_dt * dt + ran2 * r.skperp * sdt + ran3 * r.skpara_perp * sdt * r.by * r.ib;
         new_mu = r.pitch_mu;
@@ -995,8 +996,8 @@ __device__ __forceinline__ bool advance_mixed(StateMixed& st, const PushParams& 
                                               const Served* served = nullptr) {
     const DeviceSettings& s = P.s;
     const FixedGrid& F = P.fixed;
-    Rates<float> r;
-    if (!physics<float, FOCUSED, SURR>(c, st.p_hi, st.mu, P.kf, r, served)) {
+    Rates r;
+    if (!physics<FOCUSED, SURR>(c, st.p_hi, st.mu, P.kf, r, served)) {
         st.status = 2;
         return false;
     }
@@ -1015,7 +1016,7 @@ __device__ __forceinline__ bool advance_mixed(StateMixed& st, const PushParams& 
         return false;
     }
     float dx, dy, mu;
-    increments<float, FOCUSED>(r, dtf, draw_mixed<FOCUSED>(st, P), P.kf, dx, dy, mu);
+    increments<FOCUSED>(r, dtf, draw_mixed<FOCUSED>(st, P), P.kf, dx, dy, mu);
     const float dp = r.dp_dt * dtf;
     if (!isfinite(dx) || !isfinite(dy) || !isfinite(dp)) {
         st.status = 2;
@@ -1111,13 +1112,13 @@ __device__ __forceinline__ Served serve_closure(const PushParams& P, bool use, f
     if (blend || judge || !use) {
         const Consts<float>& k = P.kf;
         const float speed = __fdividef(k.particle_v0 * p, k.p0);
-        const float omega = __fdividef(k.qlt_omega0 * b, Num<float>::sqrt(1.0f + p * p));
+        const float omega = __fdividef(k.qlt_omega0 * b, Num::sqrt(1.0f + p * p));
         float duu, duu_du;
-        qlt_scattering<float>(mu, omega, speed, k, duu, duu_du);
+        qlt_scattering(mu, omega, speed, k, duu, duu_du);
         // kappa_parallel in the order the physics forms it
         float knorm = 1.0f;
-        if (k.magnetic_dependency == 1) knorm *= Num<float>::pow(b, k.gamma_turb - 2.0f);
-        if (k.momentum_dependency == 1) knorm *= Num<float>::pow(__fdividef(p, k.p0), k.pindex);
+        if (k.magnetic_dependency == 1) knorm *= Num::pow(b, k.gamma_turb - 2.0f);
+        if (k.momentum_dependency == 1) knorm *= Num::pow(__fdividef(p, k.p0), k.pindex);
         const float kpara = k.kpara0 * knorm;
         if (judge) {
             const float e_d = fabsf(served.duu - duu) / duu;
