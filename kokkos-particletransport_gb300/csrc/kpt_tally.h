@@ -19,7 +19,7 @@ static inline void atomicMax(unsigned* word, unsigned v) { *word = *word < v ? v
 namespace kpt {
 
 struct BlockTally {
-    unsigned steps[2], fallbacks[2], abandoned[2];  // low and high words
+    unsigned steps[2], fallbacks[2];  // low and high words
     unsigned pushed, failed, max_steps, judged;
     unsigned max_error;  // float bits (non-negative floats order like them)
 };
@@ -41,17 +41,17 @@ KPT_TALLY_FN void tally_finish(BlockTally& b, int steps, int status) {
     atomicMax(&b.max_steps, static_cast<unsigned>(steps));
 }
 
-// A particle the block loaded and gives up: its substeps are no result, but
-// `served` of them had their closure served, and count for the judge.
+// A particle the block loaded and gives up: `served` of its substeps had their
+// closure served, and are counted, as their fallbacks have been.
 KPT_TALLY_FN void tally_abandon(BlockTally& b, int served) {
-    tally_add(b.abandoned, static_cast<unsigned>(served));
+    tally_add(b.steps, static_cast<unsigned>(served));
     atomicAdd(&b.pushed, 1u);
 }
 
 // Substeps whose closure the network served: every substep of a particle is
 // served by the network or falls back.
 KPT_TALLY_FN unsigned long long tally_evaluations(const BlockTally& b) {
-    return tally_word(b.steps) + tally_word(b.abandoned) - tally_word(b.fallbacks);
+    return tally_word(b.steps) - tally_word(b.fallbacks);
 }
 
 }  // namespace kpt

@@ -30,8 +30,8 @@ int main() {
             tally_abandon(b, particle);
         } else {
             tally_finish(b, particle, particle == 7 ? 2 : 0);
-            steps += particle;
         }
+        steps += particle;
         CHECK(tally_evaluations(b) == served);
     }
     CHECK(tally_word(b.steps) == steps && tally_word(b.fallbacks) == fallbacks);
@@ -40,7 +40,7 @@ int main() {
     BlockTally none{};
     for (int k = 0; k < 5; ++k) tally_add(none.fallbacks, 1u);
     tally_abandon(none, 5);
-    CHECK(tally_evaluations(none) == 0 && tally_word(none.steps) == 0);
+    CHECK(tally_evaluations(none) == 0 && none.pushed == 1 && none.max_steps == 0);
     // the low words carry
     BlockTally big{};
     for (int k = 0; k < 3; ++k) tally_finish(big, 0x7fffffff, 0);
