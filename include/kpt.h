@@ -222,9 +222,10 @@ int kpt_context_fp64_fma_rate(kpt_context* ctx, double* tflops);
  * build on the shim use the same one, so powers round alike on both sides. */
 int kpt_math_pow(kpt_context* ctx, uint64_t n, const double* x, const double* y, double* out);
 /* Push scheduling: KPT_SCHEDULE_REFILL (persistent warps that refill lanes
- * from a work cursor; blocks_per_sm x SM count blocks of 128 threads, 0 =
- * as many as are resident) or KPT_SCHEDULE_SIMPLE (one particle per
- * thread).  Results do not depend on the choice. */
+ * from a work cursor; blocks_per_sm x SM count blocks of 128 threads, at most
+ * as many as are resident, 0 = the library's choice for the population) or
+ * KPT_SCHEDULE_SIMPLE (one particle per thread).  Results do not depend on the
+ * choice. */
 int kpt_context_set_push_schedule(kpt_context* ctx, int schedule, int blocks_per_sm);
 /* Arithmetic of the plain FP64 push (precision KPT_PRECISION_F64):
  * KPT_FP64_STRICT (default) rounds every operation as the reference's code

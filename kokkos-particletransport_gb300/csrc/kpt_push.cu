@@ -1630,7 +1630,8 @@ cudaError_t launch_push_kind(const PushParams& P, const PushLaunch& L, cudaStrea
     const size_t smem = network + (P.records != nullptr ? rows : 0);
     const auto kernel = push_refill_kernel<FOCUSED, SURR, KIND>;
     int resident = 0;
-    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
+    const cudaError_t err =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
     int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm : resident;
@@ -1974,7 +1975,7 @@ cudaError_t launch_batch_shape(const BatchLaunch& B, cudaStream_t stream) {
     const size_t smem = batch_offset_bytes(B.runs) +
                         (B.records != 0 ? record_xpose_bytes(FOCUSED, THREADS / 32) : 0);
     int resident = 0;
-    cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+    const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &resident, push_batch_kernel<FOCUSED, THREADS, PPL>, THREADS, smem);
     if (err != cudaSuccess) return err;
     resident = resident < 1 ? 1 : resident;
