@@ -60,9 +60,11 @@ struct RecordsCase {
 //    - learned: from ten particle-steps a point on (counted with the fewest
 //      substeps an interval can take).  421 891 particles on 1024 x 2048, 100
 //      steps 4.85 -> 3.85 ms; 1 009 584 on 2048 x 4096, 100 steps 10.25 / 10.20.
-//    - adaptive steps: likewise, and twice as many or two lanes' worth of
-//      particles.  253 134 Parker on 1024 x 2048 17.97 -> 17.06 ms, 126 814 on
-//      1024 x 1024 11.04 / 11.82.
+//    - adaptive steps: likewise, for two particles a lane and more (with fewer
+//      the longest particles' chains are the time, and they are shorter on
+//      the point tables).  253 134 Parker on 1024 x 2048 17.97 -> 17.06 ms, 361
+//      922 on 1500 x 1500 51.3 -> 42.8; 126 814 on 1024 x 1024 11.04 / 11.82,
+//      133 013 on 700 x 800 5.31 / 6.06, 124 655 on 512 x 1024 2.83 / 3.30.
 //    - fixed steps run in rounds of the resident lanes: of three blocks per SM
 //      on the point tables, of five, each 1.2 to 1.7 (Parker), 1.3 to 1.5
 //      (focused) times as long with the table's size, on records.  What the
@@ -79,9 +81,8 @@ inline bool records_pay(const RecordsCase& c) {
     const double points = static_cast<double>(c.points);
     if (particles < (c.learned ? 4.0 : 1.25) * lanes) return false;
     const double steps = 1.0 / c.dt_max_rel;  // the fewest
-    if (c.learned) return particles * steps >= 10.0 * points;
-    if (c.dt_min_rel != c.dt_max_rel) {
-        return particles * steps >= (particles >= 2.0 * lanes ? 10.0 : 20.0) * points;
+    if (c.learned || c.dt_min_rel != c.dt_max_rel) {
+        return particles * steps >= 10.0 * points && (c.learned || particles >= 2.0 * lanes);
     }
     const double point_rounds = std::ceil(particles / (384.0 * c.sm_count));
     const double record_rounds = std::ceil(particles / lanes);

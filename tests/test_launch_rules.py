@@ -65,6 +65,13 @@ SINGLE = [
     (0, 2048, 4096, 504792, 400, 10.483, 13.901), (0, 2048, 4096, 1009584, 100, 5.125, 7.253),
     (0, 2048, 4096, 1009584, 400, 19.979, 22.901), (0, 2048, 4096, 1682640, 100, 8.344, 9.967),
     (0, 2048, 4096, 2019168, 50, 5.112, 6.470), (0, 2048, 4096, 2019168, 100, 9.970, 11.107),
+    (0, 512, 1024, 124655, 50, 0.409, 0.437), (0, 512, 1024, 124655, 200, 1.458, 1.211),
+    (0, 1500, 1500, 226201, 400, 4.692, 5.077), (0, 1500, 1500, 361922, 400, 7.483, 6.580),
+    (0, 256, 4096, 170560, 100, 0.916, 0.973), (0, 256, 4096, 170560, 400, 3.543, 2.822),
+    (1, 512, 1024, 124655, 50, 0.608, 0.647), (1, 512, 1024, 132081, 400, 4.516, 3.724),
+    (1, 700, 800, 140937, 100, 1.195, 1.199), (1, 700, 800, 140937, 400, 4.698, 3.942),
+    (1, 1500, 1500, 226201, 400, 7.120, 7.884), (1, 1500, 1500, 531573, 400, 16.307, 14.097),
+    (1, 256, 4096, 213200, 100, 1.697, 1.884), (1, 256, 4096, 265434, 400, 8.209, 6.202),
     (1, 1024, 1024, 126814, 100, 1.215, 1.414), (1, 1024, 1024, 126814, 200, 2.299, 2.526),
     (1, 1024, 1024, 211356, 100, 1.688, 1.903), (1, 1024, 1024, 211356, 200, 3.256, 3.456),
     (1, 1024, 1024, 253628, 50, 1.077, 1.115), (1, 1024, 1024, 253628, 200, 4.064, 3.579),
@@ -96,11 +103,16 @@ def test_records_of_dense_and_small_populations(rules):
         for dt in (0.1, 0.001):
             assert _records(rules, focused, 256, 256, 20000, dt, dt)      # a quarter: always
             assert not _records(rules, focused, 4096, 4096, 60000, dt, dt)  # does not fill the chip
-    # adaptive Parker, ms: 17.97 / 17.06, 15.58 / 15.02 and 11.04 / 11.82, 11.73 / 13.51
-    assert _records(rules, 0, 1024, 2048, 253134, 1e-4, 0.01)
-    assert _records(rules, 0, 1024, 1024, 211356, 1e-4, 0.01)
-    assert not _records(rules, 0, 1024, 1024, 126814, 1e-4, 0.01)
-    assert not _records(rules, 0, 1024, 2048, 126567, 1e-4, 0.01)
+    # adaptive Parker, ms on the point tables / on records
+    for nx, ny, particles, points_ms, records_ms in (
+            (1024, 2048, 253134, 17.97, 17.06), (1024, 1024, 211356, 15.58, 15.02),
+            (1500, 1500, 361922, 51.3, 42.8), (256, 4096, 250510, 71.3, 63.8),
+            (256, 4096, 170560, 58.8, 58.3), (1024, 1024, 126814, 11.04, 11.82),
+            (1024, 2048, 126567, 11.73, 13.51), (512, 1024, 124655, 2.83, 3.30),
+            (512, 1024, 132081, 3.02, 3.44), (700, 800, 133013, 5.31, 6.06),
+            (700, 800, 140937, 5.60, 6.26)):
+        on = _records(rules, 0, nx, ny, particles, 1e-4, 0.01)
+        assert (records_ms if on else points_ms) <= 1.02 * min(points_ms, records_ms)
     # learned closure, ms: 4.85 / 3.85, 9.66 / 7.07, 1.65 / 2.80
     assert _records(rules, 1, 1024, 2048, 421891, 0.01, 0.01, learned=1)
     assert _records(rules, 1, 1024, 2048, 421891, 0.005, 0.005, learned=1)
