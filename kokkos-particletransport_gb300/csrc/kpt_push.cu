@@ -1636,7 +1636,7 @@ cudaError_t launch_push_kind(const PushParams& P, const PushLaunch& L, cudaStrea
     resident = resident < 1 ? 1 : resident;
     int per_sm = L.blocks_per_sm > 0 && L.blocks_per_sm < resident ? L.blocks_per_sm : resident;
     if (KIND == kPushFew) per_sm = kFewBlocks;  // the places lane_cap was computed for
-    const int blocks = KIND == kPushDense ? push_blocks<FOCUSED, SURR, KIND>() : 0;
+    const int blocks = P.records != nullptr ? push_blocks<FOCUSED, SURR, KIND>() : 0;
     return launch_with_l1(kernel, blocks, network + rows + sizeof(BlockTally),
                           L.sm_count * per_sm, threads, smem, stream, P);
 }
