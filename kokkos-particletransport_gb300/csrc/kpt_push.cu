@@ -1284,9 +1284,10 @@ __device__ __forceinline__ bool live(const StateMixed& st, const PushParams& P) 
 //
 // Three builds, one register budget and one schedule of the loads each:
 //  * kPushDense: large populations, on cell records (warp-collective), or on
-//    the point-major tables when a launch asks for more than three blocks per
-//    SM.  (Without that choice in the loop the record path compiles to a
-//    schedule that is 4 % slower: 51.1 against 49.0 ms, 1 Mi Parker.)
+//    the point-major tables when a launch takes more than three blocks per SM
+//    (on request, or where fixed steps fill them better: point_blocks).
+//    (Without that choice in the loop the record path compiles to a schedule
+//    that is 4 % slower: 51.1 against 49.0 ms, 1 Mi Parker.)
 //  * kPushPoints: the point-major tables, each lane on its own, for
 //    populations too thin for records: loads in flight count for more than
 //    warps.  5 / 4 / 3 / 2 blocks per SM: 12.4 / 11.3 / 9.9 / 10.0 ms (50 000
@@ -1699,16 +1700,28 @@ cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
         push_simple_kernel<FOCUSED><<<blocks, threads, 0, stream>>>(P);
         return cudaGetLastError();
     }
-    if (P.records != nullptr || L.blocks_per_sm > kPointsBlocks) {
-        return launch_push_kind<FOCUSED, SURR, kPushDense>(P, L, stream);
-    }
     const uint64_t few = static_cast<uint64_t>(L.sm_count) * kFewBlocks * threads;
-    if (L.count <= few && L.blocks_per_sm == 0) {
+    if (P.records == nullptr && L.count <= few && L.blocks_per_sm == 0) {
         const uint64_t warps = few / 32;
         P.lane_cap = static_cast<unsigned>((L.count + warps - 1) / warps);
         return launch_push_kind<FOCUSED, SURR, kPushFew>(P, L, stream);
     }
-    return launch_push_kind<FOCUSED, SURR, kPushPoints>(P, L, stream);
+    PushLaunch M = L;
+    if (P.records == nullptr && L.blocks_per_sm == 0 && SURR == 0) {
+        int device = 0, l2 = 0;
+        cudaError_t err = cudaGetDevice(&device);
+        if (err != cudaSuccess) return err;
+        err = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
+        if (err != cudaSuccess) return err;
+        const double points = static_cast<double>(L.grid.ex) * (L.grid.axis[1].n + 4);
+        const double frames = L.settings.time_interpolation != 0 ? 2.0 : 1.0;
+        M.blocks_per_sm = point_blocks(L.count, L.settings.dt_min == L.settings.dt_max,
+                                       frames * points * (FOCUSED ? 96.0 : 64.0), l2, L.sm_count);
+    }
+    if (P.records != nullptr || M.blocks_per_sm > kPointsBlocks) {
+        return launch_push_kind<FOCUSED, SURR, kPushDense>(P, M, stream);
+    }
+    return launch_push_kind<FOCUSED, SURR, kPushPoints>(P, M, stream);
 }
 
 #if KPT_PUSH_PART == 0

@@ -144,6 +144,40 @@ inline bool batch_records_pay(const BatchRecordsCase& c) {
     return pays || (dense && !c.fixed);
 }
 
+// ---- residency of a push on the point tables
+
+// Blocks of 128 threads per SM for a population above the build for few, plain
+// closures: the build for points holds up to three, the record build (on the
+// point tables) five.  Adaptive steps: three.  Fixed steps run in rounds of the
+// resident lanes, each about as long as it is wide, so what counts is how full
+// the last one is; tables far larger than the L2 cache punish more than three
+// blocks, whose gathers evict each other.  100 steps, ms with 2 / 3 / 4 / 5
+// blocks: Parker on 512 x 1024 75 000 0.43 / 0.51 / 0.41 / 0.50, 95 000 0.62 /
+// 0.60 / 0.63 / 0.49, 110 000 0.62 / 0.62 / 0.70 / 0.74, 190 000 1.00 / 1.05 /
+// 1.05 / 0.95; on 1024 x 2048 75 000 0.55 / 0.58 / 0.59 / 0.67, 95 000 0.73 /
+// 0.62 / 0.80 / 0.92; focused QLT on 1024 x 2048 62 000 0.86 / 1.07 / 0.83 /
+// 0.89, 110 000 1.22 / 1.07 / 1.47 / 1.83.
+inline int point_blocks(uint64_t particles, bool fixed, double table_bytes, double l2_bytes,
+                        int sm_count) {
+    const int usual = 3;
+    const uint64_t lanes = 128 * static_cast<uint64_t>(sm_count);  // of a block per SM
+    if (!fixed || particles > 8 * usual * lanes) return usual;
+    const bool fits = table_bytes <= 1.7 * l2_bytes;
+    const double near[4] = {2.08, 3.0, 3.9, 4.75}, far[2] = {2.5, 3.0};
+    int best = usual;
+    double least = 0.0;
+    for (int b = 2; b <= (fits ? 5 : 3); ++b) {
+        const uint64_t resident = lanes * static_cast<uint64_t>(b);
+        const uint64_t rounds = (particles + resident - 1) / resident;
+        const double cost = static_cast<double>(rounds) * (fits ? near[b - 2] : far[b - 2]);
+        if (b == 2 || cost < least) {
+            best = b;
+            least = cost;
+        }
+    }
+    return best;
+}
+
 // ---- residency of a batch on the point tables
 
 // Threads per SM for a batch that samples the point tables, of the `fit` that

@@ -27,6 +27,10 @@ extern "C" int batch_records_pay(int focused, int fixed, int runs, double partic
 extern "C" int batch_point_threads(uint64_t particles, int fixed, int fit, int sms) {
     return kpt::batch_point_threads(particles, fixed != 0, fit, sms);
 }
+extern "C" int point_blocks(uint64_t particles, int fixed, double table_bytes, double l2_bytes,
+                            int sms) {
+    return kpt::point_blocks(particles, fixed != 0, table_bytes, l2_bytes, sms);
+}
 extern "C" int f64_blocks_per_sm(uint64_t particles, int fixed, uint64_t lanes, int most,
                                  int requested) {
     return kpt::f64_blocks_per_sm(particles, fixed != 0, lanes, most, requested);
@@ -47,6 +51,7 @@ def rules(tmp_path_factory):
     lib.records_pay.argtypes = [i32, i32, u64, u64, dbl, dbl, i32]
     lib.batch_records_pay.argtypes = [i32, i32, i32, dbl, dbl, dbl, i32]
     lib.batch_point_threads.argtypes = [u64, i32, i32, i32]
+    lib.point_blocks.argtypes = [u64, i32, dbl, dbl, i32]
     lib.f64_blocks_per_sm.argtypes = [u64, i32, u64, i32, i32]
     return lib
 
@@ -186,6 +191,49 @@ def test_residency_of_a_batch(rules, case):
     assert rules.batch_point_threads(particles, 0, 640, SMS) == 640
     # shapes that hold no more anyway
     assert rules.batch_point_threads(particles, 1, 320, SMS) == 320
+
+
+# focused (slab QLT), nx, ny, particles, and ms of 100 fixed steps on the point
+# tables at 2, 3, 4 and 5 blocks per SM, and at five blocks of an earlier build
+# that knew no other residency
+POINTS = [
+    (0, 512, 1024, 62000, 0.42, 0.47, 0.41, 0.50, 0.51), (0, 512, 1024, 75000, 0.43, 0.53, 0.41, 0.49, 0.51),
+    (0, 512, 1024, 95000, 0.62, 0.60, 0.63, 0.49, 0.50), (0, 512, 1024, 110000, 0.62, 0.61, 0.70, 0.74, 0.68),
+    (0, 512, 1024, 125000, 0.80, 0.76, 0.76, 0.82, 0.72), (0, 512, 1024, 150000, 0.81, 0.83, 0.79, 0.87, 0.82),
+    (0, 512, 1024, 190000, 1.00, 1.05, 1.05, 0.95, 0.96), (0, 512, 1024, 230000, 1.19, 1.18, 1.16, 1.27, 1.18),
+    (0, 512, 1024, 300000, 1.55, 1.58, 1.52, 1.57, 1.54), (0, 724, 1448, 62000, 0.47, 0.49, 0.42, 0.51, 0.53),
+    (0, 724, 1448, 95000, 0.66, 0.58, 0.67, 0.51, 0.53), (0, 724, 1448, 110000, 0.67, 0.63, 0.69, 0.75, 0.73),
+    (0, 724, 1448, 125000, 0.84, 0.78, 0.75, 0.80, 0.77), (0, 724, 1448, 190000, 1.07, 1.07, 1.07, 0.98, 1.00),
+    (0, 724, 1448, 230000, 1.27, 1.20, 1.18, 1.29, 1.23), (0, 1024, 2048, 62000, 0.54, 0.57, 0.50, 0.55, 0.56),
+    (0, 1024, 2048, 75000, 0.55, 0.58, 0.59, 0.67, 0.69), (0, 1024, 2048, 95000, 0.72, 0.62, 0.80, 0.92, 0.95),
+    (0, 1024, 2048, 110000, 0.73, 0.64, 0.81, 1.23, 1.27), (0, 1024, 2048, 125000, 0.90, 0.80, 0.84, 1.19, 1.23),
+    (0, 1024, 2048, 150000, 0.92, 0.85, 0.86, 1.09, 1.10), (0, 1024, 2048, 190000, 1.11, 1.09, 1.12, 1.02, 1.06),
+    (0, 1024, 2048, 230000, 1.30, 1.22, 1.20, 1.38, 1.31), (0, 1024, 2048, 300000, 1.70, 1.63, 1.58, 1.72, 1.70),
+    (1, 512, 1024, 62000, 0.64, 0.71, 0.64, 0.78, 0.79), (1, 512, 1024, 75000, 0.66, 0.74, 0.64, 0.78, 0.79),
+    (1, 512, 1024, 95000, 0.94, 0.87, 0.97, 0.78, 0.79), (1, 512, 1024, 110000, 0.95, 0.91, 1.06, 1.11, 1.13),
+    (1, 512, 1024, 125000, 1.23, 1.16, 1.20, 1.16, 1.17), (1, 512, 1024, 150000, 1.25, 1.24, 1.22, 1.32, 1.29),
+    (1, 512, 1024, 190000, 1.56, 1.60, 1.71, 1.54, 1.53), (1, 512, 1024, 230000, 1.87, 1.77, 1.81, 2.08, 2.16),
+    (1, 512, 1024, 300000, 2.45, 2.42, 2.38, 2.73, 2.81), (1, 724, 1448, 62000, 0.77, 0.82, 0.70, 0.79, 0.82),
+    (1, 724, 1448, 95000, 1.03, 0.94, 1.10, 0.92, 0.92), (1, 724, 1448, 110000, 1.03, 0.94, 1.15, 1.24, 1.30),
+    (1, 724, 1448, 125000, 1.25, 1.20, 1.22, 1.29, 1.28), (1, 724, 1448, 190000, 1.56, 1.63, 1.65, 1.54, 1.57),
+    (1, 724, 1448, 230000, 1.88, 1.81, 1.86, 1.98, 2.00), (1, 1024, 2048, 62000, 0.85, 1.10, 0.83, 0.89, 0.91),
+    (1, 1024, 2048, 75000, 0.88, 1.08, 1.00, 1.07, 1.02), (1, 1024, 2048, 95000, 1.19, 1.06, 1.47, 1.31, 1.29),
+    (1, 1024, 2048, 110000, 1.22, 1.07, 1.47, 1.83, 1.92), (1, 1024, 2048, 125000, 1.47, 1.33, 1.45, 1.81, 1.89),
+    (1, 1024, 2048, 150000, 1.50, 1.43, 1.50, 1.82, 1.83), (1, 1024, 2048, 190000, 1.82, 1.72, 1.87, 1.90, 1.91),
+    (1, 1024, 2048, 230000, 2.10, 1.88, 1.98, 2.26, 2.27), (1, 1024, 2048, 300000, 2.56, 2.53, 2.53, 2.71, 2.81),
+]
+
+
+@pytest.mark.parametrize("case", POINTS, ids=lambda c: "-".join(map(str, c[:4])))
+def test_residency_on_the_point_tables(rules, case):
+    focused, nx, ny, particles, *times, earlier = case
+    table = 2 * (nx + 4) * (ny + 4) * (96 if focused else 64)
+    picked = rules.point_blocks(particles, 1, table, 132644864, SMS)
+    assert 2 <= picked <= 5
+    ms = times[picked - 2]
+    assert ms <= 1.09 * min(times) and ms <= 1.06 * times[1] and ms <= 1.06 * earlier
+    assert rules.point_blocks(particles, 0, table, 132644864, SMS) == 3  # adaptive steps
+    assert rules.point_blocks(100 * particles, 1, table, 132644864, SMS) == 3
 
 
 def test_no_launch_leaves_a_preference_on_its_kernel():
