@@ -205,11 +205,12 @@ inline int batch_point_threads(uint64_t particles, bool fixed, int fit, int sm_c
 
 // Blocks per SM (each one warp per sub-partition).
 //  * Every particle takes the same steps (dt_min = dt_max): the time is the
-//    number of full rounds of the population times the warps that share a
+//    number of rounds of the population times the warps that share a
 //    sub-partition, over how well that many keep its FP64 pipe busy (0.80,
 //    0.92, 0.97, 1.0 of the best for 1 to 4 warps, measured at 400 000
-//    particles).  60 000 focused particles, 50 steps: 10.1 / 7.6 / 8.8 / 7.9
-//    ms with 1 / 2 / 3 / 4 blocks; 25 000: 5.2 / 3.4 / 4.4 / 5.5 ms.
+//    particles).  A last round of a few has only the warps that they fill.
+//    60 000 focused particles, 50 steps: 10.1 / 7.6 / 8.8 / 7.9 ms with 1 / 2 /
+//    3 / 4 blocks; 25 000: 5.2 / 3.4 / 4.4 / 5.5 ms.
 //  * Adaptive steps: the interval ends with its longest particles (6 840 of
 //    a mean of 1 095 substeps on the driver's uniform field), whose substeps
 //    take as long as the warps beside them allow: one block up to eight
@@ -225,10 +226,13 @@ inline int f64_blocks_per_sm(uint64_t particles, bool fixed, uint64_t lanes, int
     const double busy[4] = {0.80, 0.92, 0.97, 1.0};
     int best = 1;
     double least = 0.0;
+    const auto round = [&](int warps) { return warps / busy[warps < 4 ? warps - 1 : 3]; };
     for (int b = 1; b <= most; ++b) {
         const uint64_t resident = lanes * static_cast<uint64_t>(b);
-        const uint64_t rounds = (particles + resident - 1) / resident;
-        const double cost = static_cast<double>(rounds) * b / busy[b < 4 ? b - 1 : 3];
+        const uint64_t full = particles / resident, rest = particles - full * resident;
+        // a population of less than one round is spread over all warps
+        double cost = static_cast<double>(full > 0 ? full : 1) * round(b);
+        if (full > 0 && rest > 0) cost += round(static_cast<int>((rest + lanes - 1) / lanes));
         if (b == 1 || cost <= least) {
             best = b;
             least = cost;

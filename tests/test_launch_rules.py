@@ -252,6 +252,12 @@ def test_residency_of_the_fp64_push(rules):
     assert rules.f64_blocks_per_sm(400000, 0, lanes, 4, 0) == 2
     assert rules.f64_blocks_per_sm(60000, 1, lanes, 4, 0) in (2, 4)
     assert rules.f64_blocks_per_sm(25000, 1, lanes, 4, 0) == 2
+    # a last round of a few costs a round of their own warps, not of all: focused
+    # slab QLT, contracted, 40 steps, two blocks fit, ms with 1 / 2 blocks
+    for particles, one, two in ((41000, 5.48, 4.70), (50000, 5.55, 4.84), (58000, 5.61, 5.05),
+                                (80000, 8.97, 7.72)):
+        picked = rules.f64_blocks_per_sm(particles, 1, lanes, 2, 0)
+        assert (one, two)[picked - 1] <= min(one, two)
     # a request is honoured in both directions, up to what fits
     for fixed in (0, 1):
         for particles in (256, 40000, 400000):
