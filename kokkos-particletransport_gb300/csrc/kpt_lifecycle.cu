@@ -346,11 +346,17 @@ __device__ __forceinline__ unsigned sort_key(const SortLaunch& L, uint64_t i) {
 // (11.4 us in chunks of 2048, whose FP64 cell maps queue on too few SMs); the
 // scatter takes 3.9 us.  Clearing and reading a word for every tile costs more
 // than the direct atomics from some thousands of tiles on (126 000 particles in
-// 8192 tiles: 5.7 us direct), 80 000 in 1000 tiles take 14 us directly.
+// 8192 tiles: 5.7 us direct), 80 000 in 1000 tiles take 14 us directly.  Where
+// particles meet seldom, the block's passes over the words are what is left: a
+// whole sort of 6 000 in 129 words takes 15.6 us direct and 16.8 ranked, of 10 000
+// in 513 15.9 / 17.6, of 20 000 in 1025 19.7 / 21.8; but of 10 000 in 129 17.0 /
+// 16.4, of 20 000 in 513 19.3 / 17.6, of 200 000 in 1025 46 / 26.
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 2;
 constexpr int kSortChunk = kSortThreads * kSortItems;
 constexpr int kSortShared = 2048;  // the most words ranked in shared memory
+constexpr uint64_t kSortFew = 8192;  // the least particles for it, and per word
+constexpr uint64_t kSortPerWord = 32;
 
 __global__ void __launch_bounds__(kSortThreads) sort_key_shared_kernel(const SortLaunch L) {
     __shared__ unsigned int tally[kSortShared];
@@ -447,7 +453,8 @@ cudaError_t launch_sort(const SortLaunch& L, cudaStream_t stream) {
     const int threads = 256;
     const uint64_t want = (L.count + threads - 1) / threads;
     const int blocks = static_cast<int>(want > 152u * 16u ? 152u * 16u : want);
-    if (tiles <= kSortShared) {
+    if (tiles <= kSortShared && L.count >= kSortFew &&
+        L.count >= kSortPerWord * static_cast<uint64_t>(tiles)) {
         const uint64_t chunks = (L.count + kSortChunk - 1) / kSortChunk;
         sort_key_shared_kernel<<<static_cast<int>(chunks > 152u * 16u ? 152u * 16u : chunks),
                                  kSortThreads, 0, stream>>>(L);
