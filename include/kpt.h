@@ -885,7 +885,7 @@ int kpt_batch_add_run(kpt_batch* batch, kpt_particles* particles, const kpt_fiel
                       uint32_t first_frame, int* run_index);
 /* Cell-sort tile (0 = no sort), resident blocks per SM (at most as many as
  * fit; 0 = the library's choice: as many as fit, or on the point tables with
- * fixed steps three blocks of 128 threads where they need few more rounds)
+ * fixed steps as few blocks of 128 threads as its rounds want)
  * and intervals between sorts. */
 int kpt_batch_set_schedule(kpt_batch* batch, int sort_tile, int blocks_per_sm, int sort_every);
 int kpt_batch_get_schedule(const kpt_batch* batch, int* sort_tile, int* blocks_per_sm,

@@ -4364,25 +4364,26 @@ int kpt_batch_autotune(kpt_batch* b, uint32_t intervals, kpt_batch_tuning* out) 
     // Stage 2: block shape, particles per lane and residency with that sort.
     // Residency candidates are resident threads per SM (all that fit, or the
     // threads of 3 or 2 blocks of 128), as blocks of the shape.  Stage 1 has
-    // timed the default shape at the library's own choice: all, or 3 blocks;
-    // the other one is left.
+    // timed the default shape at the library's own choice; all that fit take
+    // that candidate's place where it was another.
     const int sort_tile = best.tile, sort_every = best.every;
     const int shapes[3] = {64, 128, 256};
     const int lanes[2] = {1, 2};
-    const int few = 384;
-    const int resident_threads[3] = {0, few, 256};
-    const kpt::BatchLaunch chosen = batch_launch(b);
-    const bool chose_few =
-        chosen.records == 0 && kpt::batch_point_threads(chosen.particles, chosen.fixed_steps != 0,
-                                                        640, chosen.sm_count) == few;
-    const int all = chose_few ? 32 : 0;  // more than fit
+    const int resident_threads[3] = {0, 384, 256};
+    const kpt::BatchLaunch launched = batch_launch(b);
+    const int chosen =
+        launched.records != 0 ? 640
+                              : kpt::batch_point_threads(launched.particles,
+                                                         launched.fixed_steps != 0, 640,
+                                                         launched.sm_count);
+    const int all = chosen < 640 ? 32 : 0;  // 32: more than fit
     for (int threads : shapes) {
         for (int ppl : lanes) {
             for (int rt : resident_threads) {
                 int bps = rt == 0 ? all : std::max(1, rt / threads);
                 if (threads == 128 && ppl == 1) {
                     if (rt == 0) continue;  // timed in stage 1, or below
-                    if (rt == few && chose_few) bps = all;
+                    if (rt == chosen) bps = all;
                 }
                 if (int rc = consider(Choice{sort_tile, sort_every, bps, threads, ppl, 0.0f,
                                              0.0f})) {

@@ -189,7 +189,10 @@ inline int point_blocks(uint64_t particles, bool fixed, double table_bytes, doub
 // 1.59 / 1.64), 112 000 0.59 / 0.66 (0.82 / 0.90); and lose where the last of
 // the rounds is nearly empty: 190 000 1.02 / 0.96 (1.48 / 1.28), 84 000 0.54 /
 // 0.49 (0.77 / 0.64), 64 000 0.46 / 0.41 (0.62 / 0.58).  Adaptive steps have no
-// rounds and want the lanes: 192 000 Parker particles 9.40 / 8.97.
+// rounds and want the lanes: 192 000 Parker particles 9.40 / 8.97.  A population
+// that one or two blocks hold takes no more: its warps then spread evenly, and
+// share an L1 with fewer.  1 / 2 / 3 / 5 blocks, focused: 8 000 particles 0.20 /
+// 0.25 / 0.33 / 0.27, 32 000 0.34 / 0.29 / 0.34 / 0.46.
 inline int batch_point_threads(uint64_t particles, bool fixed, int fit, int sm_count) {
     const int few = 3 * 128;
     if (fit <= few || !fixed) return fit;
@@ -197,6 +200,9 @@ inline int batch_point_threads(uint64_t particles, bool fixed, int fit, int sm_c
         const uint64_t lanes = static_cast<uint64_t>(threads) * static_cast<uint64_t>(sm_count);
         return static_cast<double>((particles + lanes - 1) / lanes);
     };
+    for (int threads = 128; threads < few; threads += 128) {
+        if (rounds(threads) <= 1.0) return threads;
+    }
     const double longer = rounds(fit) <= 4.0 ? 1.48 : 1.65;
     return longer * rounds(fit) < rounds(few) ? fit : few;
 }

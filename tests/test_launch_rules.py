@@ -170,7 +170,7 @@ def test_records_of_a_batch(rules, case):
 # particles of all runs, ms of a fixed-step interval on the point tables with
 # 640 and with 384 resident threads per SM, Parker and focused
 RESIDENT = [
-    (24000, (0.61, 0.47), (0.91, 0.65)), (64000, (0.41, 0.46), (0.58, 0.62)),
+    (64000, (0.41, 0.46), (0.58, 0.62)),
     (84000, (0.49, 0.54), (0.64, 0.77)), (112000, (0.66, 0.59), (0.90, 0.82)),
     (120000, (0.73, 0.76), (0.99, 1.03)), (160000, (0.87, 0.91), (1.19, 1.26)),
     (188800, (0.96, 1.01), (1.28, 1.48)), (224000, (1.21, 1.16), (1.64, 1.59)),
@@ -266,3 +266,14 @@ def test_residency_of_the_fp64_push(rules):
                     min(requested, 4)
                 assert rules.f64_blocks_per_sm(particles, fixed, lanes, 2, requested) == \
                     min(requested, 2)
+
+
+# the same with one, two, three and five blocks of 128 threads
+@pytest.mark.parametrize("particles,parker,focused", [
+    (8000, (0.15, 0.18, 0.22, 0.21), (0.20, 0.25, 0.33, 0.27)),
+    (16000, (0.17, 0.19, 0.23, 0.26), (0.21, 0.26, 0.33, 0.41)),
+    (24000, (0.46, 0.36, 0.44, 0.58), (0.60, 0.48, 0.62, 0.85)),
+    (32000, (0.27, 0.22, 0.24, 0.32), (0.34, 0.29, 0.34, 0.46))])
+def test_residency_of_a_small_batch(rules, particles, parker, focused):
+    picked = {128: 0, 256: 1, 384: 2, 640: 3}[rules.batch_point_threads(particles, 1, 640, SMS)]
+    assert parker[picked] == min(parker) and focused[picked] == min(focused)
