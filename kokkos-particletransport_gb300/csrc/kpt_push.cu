@@ -1292,7 +1292,9 @@ __device__ __forceinline__ bool live(const StateMixed& st, const PushParams& P) 
 //    populations too thin for records: loads in flight count for more than
 //    warps.  5 / 4 / 3 / 2 blocks per SM: 12.4 / 11.3 / 9.9 / 10.0 ms (50 000
 //    Parker particles, adaptive), 2.40 / 2.40 / 2.16 / 2.35 ms (100 000
-//    focused, 2 x 100 steps).
+//    focused, 2 x 100 steps).  Not with the learned closure, whose network
+//    takes the registers: 300 000 particles on 512 x 1024, 50 steps 1.79 ms in
+//    this build, 1.64 in the first.
 //  * kPushFew: the point-major tables for populations that fit in eight warps
 //    per SM.  Nothing hides a substep's latency there, so it is what counts:
 //    up to 255 registers let all loads of a substep be in flight at once, and
@@ -1336,7 +1338,7 @@ __host__ __device__ constexpr int surr_hidden(int surr) { return surr <= 2 ? 64 
 template <bool FOCUSED, int SURR, int KIND>
 constexpr int push_blocks() {
     return KIND == kPushFew ? kFewBlocks
-           : KIND == kPushPoints && SURR == 0 ? kPointsBlocks
+           : KIND == kPushPoints ? kPointsBlocks
            : SURR >= 3      ? KPT_SURROGATE32_MIN_BLOCKS
            : SURR           ? KPT_SURROGATE_MIN_BLOCKS
                             : MinBlocks<FOCUSED>::value;
@@ -1718,10 +1720,12 @@ cudaError_t launch_push(const PushLaunch& L, cudaStream_t stream) {
         M.blocks_per_sm = point_blocks(L.count, L.settings.dt_min == L.settings.dt_max,
                                        frames * points * (FOCUSED ? 96.0 : 64.0), l2, L.sm_count);
     }
-    if (P.records != nullptr || M.blocks_per_sm > kPointsBlocks) {
-        return launch_push_kind<FOCUSED, SURR, kPushDense>(P, M, stream);
+    if constexpr (SURR == 0) {
+        if (P.records == nullptr && M.blocks_per_sm <= kPointsBlocks) {
+            return launch_push_kind<FOCUSED, SURR, kPushPoints>(P, M, stream);
+        }
     }
-    return launch_push_kind<FOCUSED, SURR, kPushPoints>(P, M, stream);
+    return launch_push_kind<FOCUSED, SURR, kPushDense>(P, M, stream);
 }
 
 #if KPT_PUSH_PART == 0
