@@ -57,10 +57,11 @@ struct RecordsCase {
 //  * Fewer, if they fill the chip (1.25 times the 640 lanes of the record
 //    kernel's five blocks per SM, four times with the learned closure, whose
 //    network hides more of the gathers):
-//    - learned: from ten particle-steps a point on (counted with the fewest
-//      substeps an interval can take).  421 891 particles on 1024 x 2048, 100
-//      steps 4.85 -> 3.85 ms; 1 009 584 on 2048 x 4096, 100 steps 10.25 / 10.20.
-//    - adaptive steps: likewise, for two particles a lane and more (with fewer
+//    - learned: from 16 particle-steps a point on (counted with the fewest
+//      substeps an interval can take).  Width 64, point tables / records:
+//      421 891 particles on 1024 x 2048, 100 steps 4.11 / 3.97 ms, 400 steps
+//      15.8 / 13.9; 506 269, 50 steps (12 a point) 2.48 / 2.57.
+//    - adaptive steps: from ten, for two particles a lane and more (with fewer
 //      the longest particles' chains are the time, and they are shorter on
 //      the point tables).  253 134 Parker on 1024 x 2048 17.97 -> 17.06 ms, 361
 //      922 on 1500 x 1500 51.3 -> 42.8; 126 814 on 1024 x 1024 11.04 / 11.82,
@@ -81,8 +82,9 @@ inline bool records_pay(const RecordsCase& c) {
     const double points = static_cast<double>(c.points);
     if (particles < (c.learned ? 4.0 : 1.25) * lanes) return false;
     const double steps = 1.0 / c.dt_max_rel;  // the fewest
-    if (c.learned || c.dt_min_rel != c.dt_max_rel) {
-        return particles * steps >= 10.0 * points && (c.learned || particles >= 2.0 * lanes);
+    if (c.learned) return particles * steps >= 16.0 * points;
+    if (c.dt_min_rel != c.dt_max_rel) {
+        return particles * steps >= 10.0 * points && particles >= 2.0 * lanes;
     }
     const double point_rounds = std::ceil(particles / (384.0 * c.sm_count));
     const double record_rounds = std::ceil(particles / lanes);

@@ -118,10 +118,15 @@ def test_records_of_dense_and_small_populations(rules):
             (700, 800, 140937, 5.60, 6.26)):
         on = _records(rules, 0, nx, ny, particles, 1e-4, 0.01)
         assert (records_ms if on else points_ms) <= 1.02 * min(points_ms, records_ms)
-    # learned closure, ms: 4.85 / 3.85, 9.66 / 7.07, 1.65 / 2.80
-    assert _records(rules, 1, 1024, 2048, 421891, 0.01, 0.01, learned=1)
-    assert _records(rules, 1, 1024, 2048, 421891, 0.005, 0.005, learned=1)
-    assert not _records(rules, 1, 2048, 4096, 504792, 0.04, 0.04, learned=1)
+    # learned closure, ms on the point tables / on records
+    for nx, ny, particles, substeps, points_ms, records_ms in (
+            (1024, 2048, 421891, 50, 2.129, 2.262), (1024, 2048, 421891, 100, 4.114, 3.967),
+            (1024, 2048, 421891, 400, 15.83, 13.84), (1024, 2048, 450000, 50, 2.57, 2.75),
+            (1024, 2048, 506269, 50, 2.475, 2.565), (1024, 2048, 506269, 100, 4.807, 4.563),
+            (1024, 2048, 506269, 400, 18.53, 16.10), (2048, 4096, 504792, 25, 1.65, 2.80)):
+        dt = (1.0 + 1e-6) / substeps
+        on = _records(rules, 1, nx, ny, particles, dt, dt, learned=1)
+        assert (records_ms if on else points_ms) == min(points_ms, records_ms)
 
 
 # focused, runs, nx, ny, particles of a run, substeps, and ms of a later
